@@ -157,6 +157,9 @@ int Engine::launch_front(Staged &S) {
       (rc = dalloc(d_dkey, dd * 8)) || (rc = dalloc(d_dhead, (dd + 1) * 4)) || (rc = dalloc(d_dsel, dd * 4)) ||
       (rc = dalloc(d_segcnt, S.nseg * 8)) || (rc = dalloc(d_qlisted, std::max<size_t>(S.nq_live, 1) * 8)))
     return rc;
+  uint32_t bloom_words = 64;
+  while (bloom_words < m) bloom_words *= 2;
+  if ((rc = dalloc(d_bloom, (size_t)bloom_words * 4))) return rc;
   S.work_limit = S.match ? work_limit : 0;
   if (S.work_limit && (rc = dalloc(d_segwork, S.nseg * 8))) return rc;
   if (S.match && (rc = dalloc(d_seeds, S.seed_cap * 16))) return rc;
@@ -191,6 +194,8 @@ int Engine::launch_front(Staged &S) {
   hd.nq_live = S.nq_live;
   hd.seed_cap = S.seed_cap;
   hd.nseg = (unsigned long long)S.nq_live * n;
+  hd.bloom_mask = bloom_words - 1;
+  hd.pad = 0;
 
   // uploads (plain copies from the slot's pinned staging)
   CK(cudaEventRecord(H.ev0, stream));
@@ -209,10 +214,10 @@ int Engine::launch_front(Staged &S) {
   unsigned int *d_err = (unsigned int *)d_misc.ptr;
   unsigned long long *segwork = S.work_limit ? (unsigned long long *)d_segwork.ptr : nullptr;
   ClearArgs ca{dh, (uint32_t *)d_vtp.ptr, (unsigned long long *)d_segcnt.ptr, segwork,
-               (unsigned long long *)d_qlisted.ptr, (Sched *)d_sched.ptr, (uint32_t *)d_misc.ptr};
+               (unsigned long long *)d_qlisted.ptr, (Sched *)d_sched.ptr, (uint32_t *)d_misc.ptr, (uint32_t *)d_bloom.ptr};
   EdgeStateArgs es{g, dh, (const uint4 *)d_upd.ptr, (const unsigned long long *)d_bkey.ptr,
                    (const uint32_t *)d_bidx.ptr, (uint32_t *)d_binfo.ptr, (uint8_t *)d_gflag.ptr,
-                   (uint32_t *)d_vtp.ptr};
+                   (uint32_t *)d_vtp.ptr, (uint32_t *)d_bloom.ptr};
   AdjUpdateArgs au{g, dh, (const unsigned long long *)d_dkey.ptr, (const uint32_t *)d_dhead.ptr,
                    (const unsigned long long *)d_bkey.ptr, (const uint8_t *)d_gflag.ptr, (uint32_t *)d_dsel.ptr,
                    d_err, (unsigned long long *)((char *)d_misc.ptr + 8),
@@ -223,7 +228,8 @@ int Engine::launch_front(Staged &S) {
   MatchArgs ma;
   std::memset(&ma, 0, sizeof(ma));
   ma.g = g;
-  ma.bt = DevBatchEdges{(const unsigned long long *)d_bkey.ptr, (const uint32_t *)d_binfo.ptr, 0};
+  ma.bt = DevBatchEdges{(const unsigned long long *)d_bkey.ptr, (const uint32_t *)d_binfo.ptr,
+                        (const uint32_t *)d_bloom.ptr, 0, 0};
   ma.hdr = dh;
   ma.vtp = (const uint32_t *)d_vtp.ptr;
   ma.qd = (const QDev *)d_qd.ptr;
@@ -467,7 +473,8 @@ int Engine::finish_device(Staged &S) {
       ++stats.kernel_launches;
       std::memset(&ma, 0, sizeof(ma));
       ma.g = g;
-      ma.bt = DevBatchEdges{(const unsigned long long *)d_bkey.ptr, (const uint32_t *)d_binfo.ptr, 0};
+      ma.bt = DevBatchEdges{(const unsigned long long *)d_bkey.ptr, (const uint32_t *)d_binfo.ptr,
+                        (const uint32_t *)d_bloom.ptr, 0, 0};
       ma.hdr = dh;
       ma.vtp = (const uint32_t *)d_vtp.ptr;
       ma.qd = (const QDev *)d_qd.ptr;

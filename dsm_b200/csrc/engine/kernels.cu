@@ -68,6 +68,9 @@ __global__ void k_edge_state(EdgeStateArgs A) {
   if (any_change) {
     atomicOr(&A.g.lab[a], kTouchBit);
     atomicOr(&A.g.lab[b], kTouchBit);
+    uint32_t word;
+    const uint32_t bits = bloom_bits(a, b, A.hdr->bloom_mask, word);
+    atomicOr(&A.bloom[word], bits);
   }
   }
 }
@@ -281,6 +284,7 @@ __global__ void k_batch_clear(ClearArgs A) {
   uint32_t *sc = reinterpret_cast<uint32_t *>(A.sc);
   for (size_t i = t; i < sizeof(Sched) / 4; i += stride) sc[i] = 0;
   for (size_t i = t; i < 64; i += stride) A.misc[i] = 0;
+  for (size_t i = t; i <= h.bloom_mask; i += stride) A.bloom[i] = 0;
 }
 
 // ---------------------------------------------------------------------------

@@ -17,6 +17,8 @@ struct BatchHdr {
   uint32_t nq_live;             // queries matched
   unsigned long long seed_cap;  // seed table capacity
   unsigned long long nseg;      // nq_live * n counters
+  uint32_t bloom_mask;          // words of the changed-edge filter, less one (DevBatchEdges)
+  uint32_t pad;
 };
 
 // Clears what a batch must start from: view times (kNoView), per-(query,
@@ -30,6 +32,7 @@ struct ClearArgs {
   unsigned long long *qlisted;
   Sched *sc;
   uint32_t *misc;  // 64 words
+  uint32_t *bloom;
 };
 void launch_batch_clear(const ClearArgs &a, int blocks, cudaStream_t s);
 
@@ -44,6 +47,7 @@ struct EdgeStateArgs {
   uint32_t *binfo;                // [m] idx | op << 30 | init << 31
   uint8_t *gflag;                 // [m] 1: union insert, 2: final delete
   uint32_t *vtp;                  // [n] view time (updates applied) or kNoView
+  uint32_t *bloom;                // filter over the keys the batch changes (cleared before)
 };
 void launch_edge_state(const EdgeStateArgs &a, int blocks, cudaStream_t s);
 

@@ -42,10 +42,9 @@ constexpr unsigned long long kSeqDone = 1ull << 63;
 
 // One candidate of a packed last level: where its pivot range starts in the
 // concatenation (excl), its id, its own range of the last level's label
-// (run offset in 16-byte units, [a, b)), flags (bit 0: its own range is the
-// pivot; bit 1: it is an endpoint of an update of the batch).
+// (run offset in 16-byte units, [a, b)), own (1: its own range is the pivot).
 struct alignas(16) PackEnt {
-  uint32_t excl, cw, off, a, b, flags, pad0, pad1;
+  uint32_t excl, cw, off, a, b, own, pad0, pad1;
 };
 
 // Staged probe range of a packed last level (per warp, shared memory): the
@@ -325,9 +324,9 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   uint32_t hb = 0;  // chunks since the last heartbeat
 
   // The packed last level over the candidates m of level L = nq - 2 (lane k:
-  // candidate cw, its label word clw).  False: more than pack_max entries (or
+  // candidate cw).  False: more than pack_max entries (or
   // one range longer than that), nothing done.
-  auto pack_last = [&](uint32_t L, uint32_t m, uint32_t cw, uint32_t clw) -> bool {
+  auto pack_last = [&](uint32_t L, uint32_t m, uint32_t cw) -> bool {
     const uint32_t LL = L + 1;
     const uint32_t bnn = __shfl_sync(kFull, q_bn, LL);
     const uint32_t wn = __shfl_sync(kFull, q_lab, LL);
@@ -367,7 +366,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
     if (dep) alg += 8ull * __popc(m);
     // candidate k's entry, read by the lanes whose entries fall in its range
     __syncwarp();  // the previous pass's lanes may still read the table
-    spk[lane] = PackEnt{incl - len, cw, o_off, o_a, o_b, (own ? 1u : 0u) | ((clw >> 31) << 1), 0u, 0u};
+    spk[lane] = PackEnt{incl - len, cw, o_off, o_a, o_b, own ? 1u : 0u, 0u, 0u};
     uint32_t sinfo = stg->info;
     __syncwarp();
     if (sinfo == kStageUnset) {  // first pass of this context: stage the longest fixed range
@@ -391,6 +390,9 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
     const uint32_t same = __ballot_sync(kFull, lane < L && q_lab == wn);
     const bool sameP = cur_want == wn;
     const uint32_t qvn = __shfl_sync(kFull, q_vert, LL);
+    // backward neighbours whose edges may not be live (the candidates' own
+    // marks are not read: the filter answers for them)
+    const uint32_t touched = bnn & (__ballot_sync(kFull, my_touch) | (1u << L));
     for (uint32_t base = 0; base < total; base += 32) {
       const uint32_t t = base + lane;
       bool ok = t < total;
@@ -402,16 +404,13 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
         if (v <= t) k += s;
       }
       const PackEnt pe = spk[k];
-      const uint32_t kx = pe.excl, kc = pe.cw, ko = pe.off, ka = pe.a, kb = pe.b, kf = pe.flags;
-      const bool kown = kf & 1u;
+      const uint32_t kx = pe.excl, kc = pe.cw, ko = pe.off, ka = pe.a, kb = pe.b;
+      const bool kown = pe.own;
       const uint64_t start = kown ? (uint64_t)ko * 4 + ka : (uint64_t)f_off * 4 + f_a;
       const uint32_t e = ok ? P.g.arena[start + (t - kx)] : 0u;
       const uint32_t w = e & kIdMask;
-      uint32_t lw = 0;
-      if (wn >= 31) {  // slot 31 holds every label >= 31
-        lw = ok ? P.g.lab[w] : 0u;
-        ok = ok && ((lw & kLabelMask) == wn);
-      }
+      if (wn >= 31)  // slot 31 holds every label >= 31
+        ok = ok && ((P.g.lab[w] & kLabelMask) == wn);
       for (uint32_t sm = same; sm; sm &= sm - 1) {
         const uint32_t fjv = __shfl_sync(kFull, my_f, __ffs(sm) - 1);
         ok = ok && (w != fjv);
@@ -457,17 +456,11 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
           ++probes;
         }
       }
-      if (wn < 31) lw = ok ? P.g.lab[w] : 0u;  // touch bit of the survivors
-      if (__any_sync(kFull, ok && (lw >> 31))) {
-        for (uint32_t bits = bnn; bits; bits &= bits - 1) {
-          const uint32_t j = __ffs(bits) - 1;
-          uint32_t fjv = __shfl_sync(kFull, my_f, j), tj = __shfl_sync(kFull, my_touch, j);
-          if (j == L) {
-            fjv = kc;
-            tj = (kf >> 1) & 1u;
-          }
-          if (ok && (lw >> 31) && tj) ok = edge_live(bt, fjv, w, tp);
-        }
+      for (uint32_t bits = touched; bits; bits &= bits - 1) {
+        const uint32_t j = __ffs(bits) - 1;
+        uint32_t fjv = __shfl_sync(kFull, my_f, j);
+        if (j == L) fjv = kc;
+        if (ok && may_change(bt, fjv, w)) ok = edge_live(bt, fjv, w, tp);
       }
       const uint32_t m2 = __ballot_sync(kFull, ok);
       work += __popc(m2);
@@ -541,16 +534,8 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
       const uint32_t e = ok ? run[i] : 0;  // entry (label-major) or id
       const uint32_t w = kLM ? (e & kIdMask) : e;
       const uint32_t want = cur_want;
-      uint32_t lw = 0;
-      if constexpr (kLM) {
-        if (want >= 31) {  // slot 31 holds every label >= 31
-          lw = ok ? P.g.lab[w] : 0;
-          ok = ok && ((lw & kLabelMask) == want);
-        }
-      } else {
-        lw = ok ? P.g.lab[w] : 0;
-        ok = ok && ((lw & kLabelMask) == want);
-      }
+      // plain runs hold every label; slot 31 holds every label >= 31
+      if (!kLM || want >= 31) ok = ok && ((P.g.lab[w] & kLabelMask) == want);
       // injectivity: only earlier positions with the same label can hold w
       for (uint32_t same = __ballot_sync(kFull, lane < L && q_lab == want); same; same &= same - 1) {
         const uint32_t fj = __shfl_sync(kFull, my_f, __ffs(same) - 1);
@@ -606,17 +591,11 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
           }
         }
       }
-      if constexpr (kLM) {
-        if (want < 31) lw = ok ? P.g.lab[w] : 0;  // touch bit of the survivors
-      }
-      if (__any_sync(kFull, ok && (lw >> 31))) {
-        uint32_t bits = bnL;
-        while (bits) {
-          uint32_t j = __ffs(bits) - 1;
-          bits &= bits - 1;
-          uint32_t fj = __shfl_sync(kFull, my_f, j), tj = __shfl_sync(kFull, my_touch, j);
-          if (ok && (lw >> 31) && tj) ok = edge_live(bt, fj, w, tp);
-        }
+      // liveness: only edges of a touched vertex can have changed, and of
+      // those the filter turns away all that the batch does not change
+      for (uint32_t bits = bnL & __ballot_sync(kFull, my_touch); bits; bits &= bits - 1) {
+        const uint32_t fj = __shfl_sync(kFull, my_f, __ffs(bits) - 1);
+        if (ok && may_change(bt, fj, w)) ok = edge_live(bt, fj, w, tp);
       }
       const uint32_t m = __ballot_sync(kFull, ok);
       work += __popc(m);
@@ -628,7 +607,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
       if (L == nq - 1) {
         emit(m, w, L, 0xFFFFFFFFu, 0);
       } else if (kLM && pack_max && L + 2 == nq && m) {
-        if (!pack_last(L, m, w, lw)) cur_mask = m;
+        if (!pack_last(L, m, w)) cur_mask = m;
       } else if (P.bfs_stop == L + 1 && m) {
         if (!write_rows(L, m, w)) cur_mask = m;
       } else {
@@ -812,7 +791,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_match(MatchArgs P) {
   // the word can change while the kernel runs)
   if (__shfl_sync(kFull, lane == 0 ? ld_volatile(P.sc->error) : 0u, 0)) return;
   const uint32_t nupd = P.hdr->n;
-  const DevBatchEdges bt{P.bt.bkey, P.bt.binfo, P.hdr->m};
+  const DevBatchEdges bt{P.bt.bkey, P.bt.binfo, P.bt.bloom, P.hdr->m, P.hdr->bloom_mask};
   bool seeds_done = false;
   while (true) {
     uint32_t kind = 0;
