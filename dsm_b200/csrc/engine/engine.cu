@@ -130,7 +130,7 @@ std::vector<DevBuf *> Engine::all_dev_bufs() {
                              &d_pair_off, &d_pair_ent, &d_upd, &d_bkey, &d_bidx, &d_binfo, &d_gflag,
                              &d_vtp, &d_dkey, &d_dhead, &d_dsel, &d_seeds, &d_sched, &d_jobs,
                              &d_job_seq, &d_out_seg, &d_out_tup, &d_segcnt, &d_misc, &d_hdr, &d_qlisted, &d_segwork,
-                             &d_rinfo, &d_rmark, &d_rlist, &d_rprev, &d_rows, &d_bloom};
+                             &d_rinfo, &d_rmark, &d_rlist, &d_rprev, &d_rows, &d_bloom, &d_fdev};
   for (auto &q : slots) v.push_back(&q.bitmap);
   for (auto &q : slots) v.push_back(&q.filter_scratch);
   for (auto &q : slots) v.push_back(&q.filter_plan);
@@ -690,6 +690,35 @@ int Engine::prepare_filter(uint32_t id) {
         d.prior[d.nprior++] = (uint32_t)j;
       }
   }
+  // label slots on which each encoding bit can be set, op by op, and from
+  // them the slots of the receivers an op can change
+  std::vector<uint32_t> on(p.enc_positions + 4, 0);
+  const auto slot_bit = [&](uint32_t u) { return 1u << label_slot(p.labels[u]); };
+  for (size_t k = 0; k < p.ops.size(); ++k) {
+    const FilterOp &o = p.ops[k];
+    DevFilterOp &d = ops[k];
+    d.core_slot = label_slot(p.labels[o.core_u]);
+    uint32_t visit = 0;
+    auto leaf = [&](uint32_t pos, uint32_t slots) {
+      visit |= slots;
+      on[pos] |= slots;
+    };
+    if (o.kind == FilterOp::kEncode) {
+      for (uint32_t j = 0; j < o.nleaf; ++j) leaf(o.pos + 1 + j, slot_bit(o.leaf_u[j]));
+    } else if (o.kind == FilterOp::kMerge) {
+      leaf(o.pos + 1, on[o.left_core_pos]);
+      if (o.right_core_pos != o.right_pos) leaf(o.pos + 2, on[o.right_core_pos]);
+    } else {
+      for (uint32_t j = 0; j < o.nleaf; ++j) {
+        uint32_t all = 0xFFFFFFFFu;
+        for (uint32_t t = 0; t < o.leaf_src_count[j]; ++t) all &= on[o.leaf_src[j][t]];
+        if (o.comb_type == 1) visit |= on[o.pos + 1 + j];  // bits there are withdrawn
+        else leaf(o.pos + 1 + j, all);
+      }
+    }
+    if (o.kind != FilterOp::kCombine || o.comb_type == 0) on[o.pos] |= slot_bit(o.core_u);
+    d.leaf_slots = visit;
+  }
   desc.hops = std::min<uint32_t>(hops, kRegionMaxHops + 1);
   s.filter_hops = desc.hops;
   const size_t plan_bytes = sizeof(QFilterDesc) + ops.size() * sizeof(DevFilterOp);
@@ -710,10 +739,11 @@ int Engine::prepare_filter(uint32_t id) {
   return DSM_OK;
 }
 
-int Engine::launch_filter(uint32_t id, int mode, int force_full) {
-  Slot &s = slots[id];
+FilterDevice Engine::filter_device(uint32_t id) const {
+  const Slot &s = slots[id];
   FilterDevice f;
-  f.desc = (const QFilterDesc *)s.filter_plan.ptr;
+  std::memset(&f, 0, sizeof(f));
+  f.desc = (QFilterDesc *)s.filter_plan.ptr;
   f.ops = (const DevFilterOp *)((const char *)s.filter_plan.ptr + sizeof(QFilterDesc));
   f.nops = s.filter_nops;
   f.vcand = (uint32_t *)s.filter_scratch.ptr;
@@ -722,8 +752,33 @@ int Engine::launch_filter(uint32_t id, int mode, int force_full) {
   f.words = std::max<uint32_t>(s.plan.enc_words, 1);
   f.col_len = (nv + 31) / 32;
   f.bitmap = (uint32_t *)s.bitmap.ptr;
-  launch_query_filter(dev_graph(), f, mode, num_sms, stream, region_dev(), force_full || !filter_incremental);
-  stats.kernel_launches += 2 + (mode >= 2 ? 3 * f.nops : 0);
+  return f;
+}
+
+// The device array of the filters that the next launch runs; uploaded when
+// it differs from the last one (the upload waits: the array is pageable).
+int Engine::set_filters(const std::vector<uint32_t> &ids) {
+  std::vector<FilterDevice> f;
+  f.reserve(ids.size());
+  for (uint32_t id : ids) f.push_back(filter_device(id));
+  if (f.size() == fdev_host.size() &&
+      (f.empty() || std::memcmp(f.data(), fdev_host.data(), f.size() * sizeof(FilterDevice)) == 0))
+    return DSM_OK;
+  fdev_host.clear();
+  if (int rc = dalloc(d_fdev, std::max<size_t>(f.size(), 1) * sizeof(FilterDevice))) return rc;
+  CK(cudaMemcpyAsync(d_fdev.ptr, f.data(), f.size() * sizeof(FilterDevice), cudaMemcpyHostToDevice, stream));
+  CK(cudaStreamSynchronize(stream));
+  fdev_host = std::move(f);
+  ++query_gen;
+  return DSM_OK;
+}
+
+int Engine::run_filters(int mode, int force_full) {
+  uint32_t max_ops = 0;
+  for (const FilterDevice &f : fdev_host) max_ops = std::max(max_ops, f.nops);
+  stats.kernel_launches +=
+      launch_query_filters(dev_graph(), (const FilterDevice *)d_fdev.ptr, (uint32_t)fdev_host.size(), max_ops, mode,
+                           num_sms, stream, region_dev(), force_full || !filter_incremental);
   return DSM_OK;
 }
 
@@ -755,6 +810,8 @@ int Engine::prepare_filters() {
   if (changed)
     if (int rc = upload_qd()) return rc;
   if (changed) CK(cudaStreamSynchronize(stream));  // qd_host is pageable
+  if (filter_mode > 0)
+    if (int rc = set_filters(live_ids)) return rc;
   return DSM_OK;
 }
 
@@ -771,8 +828,7 @@ int Engine::launch_filters() {
     launch_region_build(dev_graph(), region_dev(), hdr_n, (const uint4 *)d_upd.ptr, hops, num_sms, stream);
     stats.kernel_launches += 3 + 2 * hops;
   }
-  for (uint32_t id : live_ids)
-    if (int rc = launch_filter(id, filter_mode, 0)) return rc;
+  if (int rc = run_filters(filter_mode, 0)) return rc;
   if (region) {
     launch_region_save(region_dev(), hdr_n, (const uint4 *)d_upd.ptr, stream);
     ++stats.kernel_launches;
@@ -803,7 +859,8 @@ int Engine::query_filter(uint32_t qid, uint32_t *bitmaps, uint32_t *v_cand_us) {
   if (qid >= slots.size() || !slots[qid].live) return fail(DSM_ERR_NOT_FOUND, "no such query");
   CK(cudaSetDevice(device));
   if (int rc = prepare_filter(qid)) return rc;
-  if (int rc = launch_filter(qid, 2, 1)) return rc;
+  if (int rc = set_filters({qid})) return rc;
+  if (int rc = run_filters(2, 1)) return rc;
   CK(cudaGetLastError());
   const Slot &s = slots[qid];
   if (bitmaps)

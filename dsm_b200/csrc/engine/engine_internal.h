@@ -214,7 +214,8 @@ struct Engine {
 
   // batch scratch
   DevBuf d_upd, d_bkey, d_bidx, d_binfo, d_gflag, d_vtp, d_dkey, d_dhead, d_dsel, d_seeds, d_sched, d_jobs,
-      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_bloom;
+      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_bloom, d_fdev;
+  std::vector<FilterDevice> fdev_host;  // what d_fdev holds
   HostBuf h_sched;    // Sched + the error words, read after the matcher
   HostBuf h_qlisted;  // per-query listing counters, read after the matcher
   HostOut hout[2];
@@ -260,7 +261,9 @@ struct Engine {
   void elapsed(cudaEvent_t a, cudaEvent_t b, float *ms);
   bool capturing = false;
   int prepare_filter(uint32_t id);
-  int launch_filter(uint32_t id, int mode, int force_full);
+  FilterDevice filter_device(uint32_t id) const;
+  int set_filters(const std::vector<uint32_t> &ids);
+  int run_filters(int mode, int force_full);
   int launch_match_seq(const MatchArgs &ma, int blocks, uint32_t levels);
   RegionDevice region_dev();
   int region_init();

@@ -31,6 +31,8 @@
 // read bits of earlier layers that nothing rewrites later).  A region that
 // outgrows its list, a state not computed in the previous batch, or a graph
 // changed outside a filtered batch make the run recompute every vertex.
+#include <algorithm>
+
 #include "filter.cuh"
 
 namespace dsm {
@@ -40,11 +42,13 @@ namespace {
 __device__ __forceinline__ bool ebit(const uint32_t *enc, uint32_t words, uint32_t v, uint32_t pos) {
   return (enc[(size_t)v * words + (pos >> 5)] >> (pos & 31)) & 1u;
 }
+// Inside an op a bit only ever goes one way, so one that is there already (a
+// hub hears from thousands of candidates) needs no atomic.
 __device__ __forceinline__ void eset(uint32_t *enc, uint32_t words, uint32_t v, uint32_t pos) {
-  atomicOr(&enc[(size_t)v * words + (pos >> 5)], 1u << (pos & 31));
+  if (!ebit(enc, words, v, pos)) atomicOr(&enc[(size_t)v * words + (pos >> 5)], 1u << (pos & 31));
 }
 __device__ __forceinline__ void eclr(uint32_t *enc, uint32_t words, uint32_t v, uint32_t pos) {
-  atomicAnd(&enc[(size_t)v * words + (pos >> 5)], ~(1u << (pos & 31)));
+  if (ebit(enc, words, v, pos)) atomicAnd(&enc[(size_t)v * words + (pos >> 5)], ~(1u << (pos & 31)));
 }
 
 // Whether this run of the query recomputes every vertex.
@@ -74,65 +78,73 @@ __device__ __forceinline__ bool in_region(const RegionDevice &rg, uint32_t epoch
   return (m >> 6) == epoch && (m & 63) <= hops;
 }
 
-// LDF + NLF, one warp per data vertex (filter.cu:394-613): label equal,
-// degree >= the query vertex's degree in the full query, and for every
-// label l below the query's largest label + 1 at least as many neighbours
-// of label l as the query vertex has.  Clears the vertex's encodings.  The
-// first kernel of a run: decides whether the run is full.
-__global__ void k_ldf_nlf(DevGraph g, QFilterDesc *D, uint32_t *vcand, uint32_t *valid, uint32_t *enc,
-                          uint32_t words, RegionDevice rg, int force_full) {
-  __shared__ uint32_t cnt[8][32];
-  const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+// LDF + NLF (filter.cu:394-613): label equal, degree >= the query vertex's
+// degree in the full query, and for every label l below the query's largest
+// label + 1 at least as many neighbours of label l as the query vertex has.
+// Clears the vertex's encodings.  The first kernel of a run: decides whether
+// the run is full.
+//
+// Bound by the slot offsets' bytes.  A label-major run already holds a
+// vertex's neighbours counted by label: lane l of the warp takes the
+// difference of two slot offsets (one coalesced row of at most 132 bytes)
+// where the run itself was read and every neighbour's label gathered before.
+// Only slot 31, which labels above 31 share, is read when the query uses label
+// 31.  A warp takes 32 vertices, so that labels, degrees and results move as
+// 128-byte rows and vertices without a query label cost nothing more.
+// 2^20 vertices, 2^24 edges, one query: 325 -> 41 us.
+__global__ void k_ldf_nlf(DevGraph g, const FilterDevice *F, RegionDevice rg, int force_full) {
+  const FilterDevice f = F[blockIdx.y];
+  QFilterDesc *D = f.desc;
+  const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t nl = D->nlabels;
+  const uint32_t nl = D->nlabels, words = f.words;
   const bool full = decide_full(D, rg, force_full);
   if (blockIdx.x == 0 && threadIdx.x == 0) D->full_now = full ? 1u : 0u;
   const uint32_t count = full ? g.nv : rg.info->bound[D->hops];
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += warps) {
-    const uint32_t v = full ? i : rg.list[i];
-    const uint32_t lv = g.lab[v] & kLabelMask;
-    const uint2 av = g.adj[v];
-    uint32_t um = lv < nl ? D->label_us[lv] : 0u;  // query vertices with this label
-    uint32_t keep = 0;
-    for (uint32_t b = um; b; b &= b - 1) {
-      uint32_t u = __ffs(b) - 1;
-      if (D->qdeg[u] <= av.y) keep |= 1u << u;
-    }
-    uint32_t res = 0;
-    if (keep) {
-      cnt[wib][lane] = 0;
-      __syncwarp();
-      // the run starts on a 16-byte boundary: four entries per lane per load
-      const uint32_t *run = adj_list(g, av);
-      const uint4 *run4 = reinterpret_cast<const uint4 *>(run);
-      const uint32_t n4 = av.y >> 2;
-      for (uint32_t k = lane; k < n4; k += 32) {
-        const uint4 q = run4[k];
-        const uint32_t e[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const uint32_t l = g.lab[e[t] & kIdMask] & kLabelMask;
-          if (l < nl) atomicAdd(&cnt[wib][l], 1u);
-        }
+  for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; base < count; base += warps * 32) {
+    const uint32_t i = base + lane;
+    const uint32_t v = i < count ? (full ? i : rg.list[i]) : 0u;
+    uint32_t keep = 0, res = 0;
+    if (i < count) {
+      const uint32_t lv = g.lab[v] & kLabelMask, dv = g.adj[v].y;
+      for (uint32_t b = lv < nl ? D->label_us[lv] : 0u; b; b &= b - 1) {  // query vertices with this label
+        const uint32_t u = __ffs(b) - 1;
+        if (D->qdeg[u] <= dv) keep |= 1u << u;
       }
-      for (uint32_t k = 4 * n4 + lane; k < av.y; k += 32) {
-        const uint32_t l = g.lab[run[k] & kIdMask] & kLabelMask;
-        if (l < nl) atomicAdd(&cnt[wib][l], 1u);
-      }
-      __syncwarp();
-      const uint32_t mine = cnt[wib][lane];
-      for (uint32_t b = keep; b; b &= b - 1) {
-        uint32_t u = __ffs(b) - 1;
-        bool pass = lane >= nl || mine >= D->nlc[u][lane];
-        if (__all_sync(kFull, pass)) res |= 1u << u;
-      }
-      __syncwarp();
     }
-    if (lane == 0) {
-      vcand[v] = res;
-      valid[v] = res;
+    for (uint32_t m = __ballot_sync(kFull, keep != 0); m; m &= m - 1) {
+      const uint32_t k = __ffs(m) - 1;
+      const uint32_t vk = __shfl_sync(kFull, v, k), kk = __shfl_sync(kFull, keep, k);
+      const uint32_t *t = g.loff + (size_t)vk * (g.nlt + 1);
+      const uint32_t a = lane <= g.nlt ? t[lane] : 0u;
+      uint32_t b = __shfl_down_sync(kFull, a, 1);
+      if (lane == 31 && g.nlt == 32) b = t[32];
+      uint32_t mine = lane < g.nlt ? b - a : 0u;
+      if (nl == 32 && g.nlt == 32) {  // slot 31 holds every label >= 31: count label 31 itself
+        const uint32_t lo = __shfl_sync(kFull, a, 31), hi = __shfl_sync(kFull, b, 31);
+        const uint32_t *run = adj_list(g, g.adj[vk]);
+        uint32_t c = 0;
+        for (uint32_t j = lo + lane; j < hi; j += 32) c += (g.lab[run[j] & kIdMask] & kLabelMask) == 31;
+        c = __reduce_add_sync(kFull, c);
+        if (lane == 31) mine = c;
+      }
+      uint32_t rk = 0;
+      for (uint32_t b2 = kk; b2; b2 &= b2 - 1) {
+        const uint32_t u = __ffs(b2) - 1;
+        if (__all_sync(kFull, lane >= nl || mine >= D->nlc[u][lane])) rk |= 1u << u;
+      }
+      if (lane == k) res = rk;
     }
-    for (uint32_t w = lane; w < words; w += 32) enc[(size_t)v * words + w] = 0;
+    if (i < count) {
+      f.vcand[v] = res;
+      f.valid[v] = res;
+    }
+    if (full) {
+      const size_t e0 = (size_t)base * words, e1 = (size_t)min(base + 32, count) * words;
+      for (size_t e = e0 + lane; e < e1; e += 32) f.enc[e] = 0;
+    } else if (i < count) {
+      for (uint32_t w = 0; w < words; ++w) f.enc[(size_t)v * words + w] = 0;
+    }
   }
 }
 
@@ -181,26 +193,76 @@ __device__ __forceinline__ void leaf_rule(const DevFilterOp &op, uint32_t n, con
   }
 }
 
-// Full runs: one op over every current candidate of its core vertex; a warp
-// takes 32 vertices, then walks the candidates among them one by one with
-// its lanes over the candidate's neighbours.
-__global__ void k_filter_op(DevGraph g, const QFilterDesc *D, const DevFilterOp *ops, uint32_t k,
-                            const uint32_t *vcand, uint32_t *valid, uint32_t *enc, uint32_t words) {
-  if (!D->full_now) return;
-  const DevFilterOp &op = ops[k];
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t cu = op.core_u;
-  for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; base < g.nv; base += warps * 32) {
-    const uint32_t v = base + lane;
-    const bool isc = v < g.nv && ((valid[v] >> cu) & 1u);
-    for (uint32_t m = __ballot_sync(kFull, isc); m; m &= m - 1) {
-      const uint32_t c = base + __ffs(m) - 1;
-      if (lane == 0) core_rule(op, c, valid, enc, words);
-      // its neighbours
-      const uint2 ac = g.adj[c];
-      const uint32_t *run = adj_list(g, ac);
-      for (uint32_t i = lane; i < ac.y; i += 32) leaf_rule(op, run[i] & kIdMask, vcand, enc, words);
+// The ranges of a block's 256 vertices (thread t: len entries from arena word
+// `first`) laid end to end: s_incl is the inclusive scan of the lengths, entry
+// e of the total lies at arena word s_start[o] + e for its owner o.
+struct BlockRanges {
+  unsigned long long start[256];
+  uint32_t incl[256];
+  uint32_t warp[8];
+};
+__device__ __forceinline__ uint32_t lay_ranges(BlockRanges &R, unsigned long long first, uint32_t len) {
+  const uint32_t t = threadIdx.x, lane = t & 31;
+  uint32_t incl = len;
+#pragma unroll
+  for (uint32_t d = 1; d < 32; d <<= 1) {
+    const uint32_t x = __shfl_up_sync(kFull, incl, d);
+    if (lane >= d) incl += x;
+  }
+  if (lane == 31) R.warp[t >> 5] = incl;
+  __syncthreads();
+  for (uint32_t w = 0; w < (t >> 5); ++w) incl += R.warp[w];
+  R.incl[t] = incl;
+  R.start[t] = first - (incl - len);
+  __syncthreads();
+  return R.incl[255];
+}
+__device__ __forceinline__ unsigned long long range_entry(const BlockRanges &R, uint32_t e) {
+  uint32_t o = 0;  // the first owner with incl > e
+#pragma unroll
+  for (uint32_t d = 128; d; d >>= 1)
+    if (R.incl[o + d - 1] <= e) o += d;
+  return R.start[o] + e;
+}
+
+// Full runs: one op over every current candidate of its core vertex.
+//
+// Bound by the gathers and marks of the receivers.  Only neighbours of the
+// labels the leaf rule can change are visited (leaf_slots: one contiguous
+// range each of the label-major run).  A block takes 256 vertices, one a
+// thread, lays the candidates' ranges of one label end to end (a block scan of
+// their lengths) and gives each thread one entry in turn, its owner found by
+// eight steps through the scan: a hub's range is then shared by the block,
+// where one warp walked the hub's whole run before and the launch waited for
+// it.  2^20 vertices, 2^24 edges (R-MAT), one op: 635 -> 46 us.
+__global__ void __launch_bounds__(256) k_filter_op(DevGraph g, const FilterDevice *F, uint32_t k) {
+  const FilterDevice f = F[blockIdx.y];
+  if (k >= f.nops || !f.desc->full_now) return;
+  __shared__ BlockRanges R;
+  const DevFilterOp &op = f.ops[k];
+  const uint32_t t = threadIdx.x, cu = op.core_u, words = f.words;
+  for (uint32_t base = blockIdx.x * 256; base < g.nv; base += gridDim.x * 256) {
+    const uint32_t v = base + t;
+    const bool isc = v < g.nv && ((f.valid[v] >> cu) & 1u);
+    if (!__syncthreads_or(isc)) continue;
+    uint32_t off = 0;
+    if (isc) {
+      core_rule(op, v, f.valid, f.enc, words);
+      off = g.adj[v].x;
+    }
+    for (uint32_t sm = op.leaf_slots; sm; sm &= sm - 1) {
+      const uint32_t sl = __ffs(sm) - 1;
+      if (sl >= g.nlt) break;  // no vertex has a label of this slot or a later one
+      uint32_t a = 0, len = 0;
+      if (isc) {
+        const uint32_t *lo = g.loff + (size_t)v * (g.nlt + 1) + sl;
+        a = lo[0];
+        len = lo[1] - a;
+      }
+      const uint32_t total = lay_ranges(R, (unsigned long long)off * 4 + a, len);
+      for (uint32_t e = t; e < total; e += 256)
+        leaf_rule(op, g.arena[range_entry(R, e)] & kIdMask, f.vcand, f.enc, words);
+      __syncthreads();
     }
   }
 }
@@ -223,45 +285,48 @@ __device__ __forceinline__ bool replayed_valid(const DevFilterOp *ops, const Dev
 }
 
 // Region runs, op k, first half: every receiver of the region pulls its
-// leaf bits (a warp per receiver scans its neighbours for a valid core
-// candidate at the op's start).
-__global__ void k_filter_pull(DevGraph g, const QFilterDesc *D, const DevFilterOp *ops, uint32_t k,
-                              const uint32_t *vcand, const uint32_t *valid, uint32_t *enc, uint32_t words,
-                              RegionDevice rg) {
-  if (D->full_now) return;
-  const DevFilterOp &op = ops[k];
+// leaf bits (a warp per receiver scans its neighbours of the core's label for
+// a valid core candidate at the op's start).
+__global__ void k_filter_pull(DevGraph g, const FilterDevice *F, uint32_t k, RegionDevice rg) {
+  const FilterDevice f = F[blockIdx.y];
+  const QFilterDesc *D = f.desc;
+  if (k >= f.nops || D->full_now) return;
+  const DevFilterOp &op = f.ops[k];
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t epoch = rg.info->epoch, hops = D->hops;
+  const uint32_t epoch = rg.info->epoch, hops = D->hops, words = f.words;
   const uint32_t count = rg.info->bound[hops];
-  const uint32_t cu = op.core_u;
+  const uint32_t cu = op.core_u, sl = op.core_slot;
+  if (sl >= g.nlt) return;  // no candidates
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += warps) {
     const uint32_t n = rg.list[i];
-    const uint2 an = g.adj[n];
-    const uint32_t *run = adj_list(g, an);
+    const uint32_t *run = adj_list(g, g.adj[n]);
+    const uint32_t *lo = g.loff + (size_t)n * (g.nlt + 1) + sl;
+    const uint32_t end = lo[1];
     bool has = false;
-    for (uint32_t b = 0; b < an.y && !has; b += 32) {
+    for (uint32_t b = lo[0]; b < end && !has; b += 32) {
       bool cv = false;
-      if (b + lane < an.y) {
+      if (b + lane < end) {
         const uint32_t c = run[b + lane] & kIdMask;
-        cv = in_region(rg, epoch, hops, c) ? ((valid[c] >> cu) & 1u) != 0
-                                           : replayed_valid(ops, op, c, vcand, enc, words);
+        cv = in_region(rg, epoch, hops, c) ? ((f.valid[c] >> cu) & 1u) != 0
+                                           : replayed_valid(f.ops, op, c, f.vcand, f.enc, words);
       }
       has = __any_sync(kFull, cv);
     }
-    if (has && lane == 0) leaf_rule(op, n, vcand, enc, words);
+    if (has && lane == 0) leaf_rule(op, n, f.vcand, f.enc, words);
   }
 }
 
 // Region runs, op k, second half: the core rule for the region's candidates.
-__global__ void k_filter_core(const QFilterDesc *D, const DevFilterOp *ops, uint32_t k, uint32_t *valid,
-                              uint32_t *enc, uint32_t words, RegionDevice rg) {
-  if (D->full_now) return;
-  const DevFilterOp &op = ops[k];
+__global__ void k_filter_core(const FilterDevice *F, uint32_t k, RegionDevice rg) {
+  const FilterDevice f = F[blockIdx.y];
+  const QFilterDesc *D = f.desc;
+  if (k >= f.nops || D->full_now) return;
+  const DevFilterOp &op = f.ops[k];
   const uint32_t count = rg.info->bound[D->hops];
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
     const uint32_t c = rg.list[i];
-    if ((valid[c] >> op.core_u) & 1u) core_rule(op, c, valid, enc, words);
+    if ((f.valid[c] >> op.core_u) & 1u) core_rule(op, c, f.valid, f.enc, f.words);
   }
 }
 
@@ -269,20 +334,21 @@ __global__ void k_filter_core(const QFilterDesc *D, const DevFilterOp *ops, uint
 // position (or, with LDF+NLF only, from vcand).  Full runs: a warp per word;
 // region runs: a warp per region vertex, rewriting its whole word.  The
 // last kernel of a run: records the epoch the state belongs to.
-__global__ void k_filter_compact(uint32_t nv, QFilterDesc *D, const uint32_t *vcand, const uint32_t *enc,
-                                 uint32_t words, uint32_t col_len, uint32_t *bitmap, int ldf_only, RegionDevice rg) {
+__global__ void k_filter_compact(uint32_t nv, const FilterDevice *F, int ldf_only, RegionDevice rg) {
+  const FilterDevice f = F[blockIdx.y];
+  QFilterDesc *D = f.desc;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   const Scope sc = scope_of(D, rg, nv);
-  const uint32_t count = sc.full ? col_len : sc.count;
+  const uint32_t count = sc.full ? f.col_len : sc.count;
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += warps) {
     const uint32_t w = sc.full ? i : (sc.list[i] >> 5);
     const uint32_t v = w * 32 + lane;
     for (uint32_t u = 0; u < D->nq; ++u) {
       bool b = false;
-      if (v < nv) b = ldf_only ? ((vcand[v] >> u) & 1u) : ebit(enc, words, v, D->pos_of_u[u]);
+      if (v < nv) b = ldf_only ? ((f.vcand[v] >> u) & 1u) : ebit(f.enc, f.words, v, D->pos_of_u[u]);
       uint32_t m = __ballot_sync(kFull, b);
-      if (lane == 0) bitmap[(size_t)u * col_len + w] = m;
+      if (lane == 0) f.bitmap[(size_t)u * f.col_len + w] = m;
     }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) D->fepoch = rg.info ? rg.info->epoch : 0xFFFFFFFFu;
@@ -324,28 +390,23 @@ __global__ void k_region_seed(DevGraph g, RegionDevice rg, const uint32_t *hdr_n
 
 __global__ void k_region_close(RegionInfo *I, uint32_t hop) { I->bound[hop] = min(I->total, I->cap); }
 
-// Hop `hop`: every neighbour of the vertices first reached at hop - 1.
-__global__ void k_region_expand(DevGraph g, RegionDevice rg, uint32_t hop) {
+// Hop `hop`: every neighbour of the vertices first reached at hop - 1.  A
+// block shares the runs of 256 of them (a warp per run left the launch waiting
+// for the warps that had drawn the hubs).
+__global__ void __launch_bounds__(256) k_region_expand(DevGraph g, RegionDevice rg, uint32_t hop) {
+  __shared__ BlockRanges R;
   const RegionInfo &I = *rg.info;
   if (I.ov_round < 64) return;  // the list is full: queries that far out run in full
   const uint32_t lo = hop >= 2 ? I.bound[hop - 2] : 0u, hi = I.bound[hop - 1];
-  const uint32_t lane = threadIdx.x & 31, epoch = I.epoch;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < hi; i += warps) {
-    const uint32_t v = rg.list[i];
-    const uint2 av = g.adj[v];
-    const uint32_t *run = adj_list(g, av);
-    const uint4 *run4 = reinterpret_cast<const uint4 *>(run);  // 16-byte aligned run
-    const uint32_t n4 = av.y >> 2;
-    for (uint32_t k = lane; k < n4; k += 32) {
-      const uint4 q = run4[k];
-      claim(rg, epoch, q.x & kIdMask, hop);
-      claim(rg, epoch, q.y & kIdMask, hop);
-      claim(rg, epoch, q.z & kIdMask, hop);
-      claim(rg, epoch, q.w & kIdMask, hop);
+  const uint32_t t = threadIdx.x, epoch = I.epoch;
+  for (uint32_t base = lo + blockIdx.x * 256; base < hi; base += gridDim.x * 256) {
+    const uint2 av = base + t < hi ? g.adj[rg.list[base + t]] : make_uint2(0, 0);
+    const uint32_t total = lay_ranges(R, (unsigned long long)av.x * 4, av.y);
+    for (uint32_t e = t; e < total; e += 256) {
+      claim(rg, epoch, g.arena[range_entry(R, e)] & kIdMask, hop);
+      if ((e >> 8) % 8 == 7 && *(volatile const uint32_t *)&rg.info->ov_round < 64) break;
     }
-    for (uint32_t k = 4 * n4 + lane; k < av.y; k += 32) claim(rg, epoch, run[k] & kIdMask, hop);
-    if (*(volatile const uint32_t *)&rg.info->ov_round < 64) return;
+    if (__syncthreads_or(*(volatile const uint32_t *)&rg.info->ov_round < 64)) return;
   }
 }
 
@@ -366,20 +427,32 @@ __global__ void k_region_save(RegionDevice rg, const uint32_t *hdr_n, const uint
 
 }  // namespace
 
-void launch_query_filter(const DevGraph &g, const FilterDevice &f, int mode, int num_sms, cudaStream_t s,
-                         const RegionDevice &rg, int force_full) {
-  const int blocks = num_sms * 8;
-  QFilterDesc *D = const_cast<QFilterDesc *>(f.desc);
-  k_ldf_nlf<<<blocks, 256, 0, s>>>(g, D, f.vcand, f.valid, f.enc, f.words, rg, force_full);
-  if (mode >= 2)
-    for (uint32_t k = 0; k < f.nops; ++k) {
-      k_filter_op<<<blocks, 256, 0, s>>>(g, D, f.ops, k, f.vcand, f.valid, f.enc, f.words);
-      if (rg.info) {
-        k_filter_pull<<<blocks, 256, 0, s>>>(g, D, f.ops, k, f.vcand, f.valid, f.enc, f.words, rg);
-        k_filter_core<<<blocks, 256, 0, s>>>(D, f.ops, k, f.valid, f.enc, f.words, rg);
+int launch_query_filters(const DevGraph &g, const FilterDevice *f, uint32_t nf, uint32_t max_ops, int mode,
+                         int num_sms, cudaStream_t s, const RegionDevice &rg, int force_full) {
+  if (nf == 0) return 0;
+  // queries share the launch: about 16 blocks per SM over all of them, and
+  // never fewer than an SM's worth of one query's
+  const unsigned per = std::max<unsigned>(num_sms * 16u / nf, num_sms);
+  int launched = 0;
+  for (uint32_t q0 = 0; q0 < nf; q0 += 65535u) {  // the grid's limit in y
+    const uint32_t nq = std::min(nf - q0, 65535u);
+    const FilterDevice *fq = f + q0;
+    const dim3 grid(per, nq), light(std::min<unsigned>(per, num_sms * 2u), nq);
+    k_ldf_nlf<<<grid, 256, 0, s>>>(g, fq, rg, force_full);
+    ++launched;
+    for (uint32_t k = 0; mode >= 2 && k < max_ops; ++k) {
+      k_filter_op<<<grid, 256, 0, s>>>(g, fq, k);
+      ++launched;
+      if (rg.info && !force_full) {
+        k_filter_pull<<<grid, 256, 0, s>>>(g, fq, k, rg);
+        k_filter_core<<<light, 256, 0, s>>>(fq, k, rg);
+        launched += 2;
       }
     }
-  k_filter_compact<<<blocks, 256, 0, s>>>(g.nv, D, f.vcand, f.enc, f.words, f.col_len, f.bitmap, mode < 2, rg);
+    k_filter_compact<<<grid, 256, 0, s>>>(g.nv, fq, mode < 2, rg);
+    ++launched;
+  }
+  return launched;
 }
 
 void launch_region_build(const DevGraph &g, const RegionDevice &rg, const uint32_t *hdr_n, const uint4 *upd,

@@ -39,6 +39,9 @@ struct DevFilterOp {
   // (merges and combines), for the incremental filter's validity replay
   uint32_t nprior;
   uint32_t prior[15];
+  // label slots: of the receivers the leaf rule can change (a bit is only ever
+  // set on vertices of its members' labels), and of the core vertex
+  uint32_t leaf_slots, core_slot;
 };
 
 // Incremental region (one per engine, shared by the queries of a batch).
@@ -72,18 +75,20 @@ struct RegionDevice {
 };
 
 struct FilterDevice {
-  const QFilterDesc *desc;
+  QFilterDesc *desc;
   const DevFilterOp *ops;
-  uint32_t nops;
   uint32_t *vcand, *valid, *enc, *bitmap;
-  uint32_t words, col_len;
+  uint32_t nops, words, col_len, pad;
 };
 
-// mode 1: LDF+NLF only; mode 2: cluster encoding.  Writes f.bitmap.  With a
-// region (rg.info != nullptr) and force_full == 0, only the vertices of the
-// query's region are recomputed, unless the region overflowed.
-void launch_query_filter(const DevGraph &g, const FilterDevice &f, int mode, int num_sms, cudaStream_t s,
-                         const RegionDevice &rg, int force_full);
+// Runs the filters of nf queries (device array f): one launch per step for
+// all of them, as the steps of different queries are independent.
+// mode 1: LDF+NLF only; mode 2: cluster encoding (max_ops: the longest plan).
+// Writes each bitmap.  With a region (rg.info != nullptr) and force_full == 0,
+// only the vertices of a query's region are recomputed, unless the region
+// overflowed.  Returns the number of kernels launched.
+int launch_query_filters(const DevGraph &g, const FilterDevice *f, uint32_t nf, uint32_t max_ops, int mode,
+                         int num_sms, cudaStream_t s, const RegionDevice &rg, int force_full);
 
 // Region of a batch: hops 0..hops from the endpoints of the batch's updates
 // (upd, hdr->n) and of the previous batch's (rg.prev); then the batch's own

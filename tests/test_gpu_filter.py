@@ -182,3 +182,26 @@ def test_incremental_filter_ldf_only_and_graph_changes():
         assert fulls < 8 * len(qs)
         for e, _ in (inc, full):
             e.close()
+
+
+@pytest.mark.parametrize("nv", [31, 32, 33, 255, 256, 257, 700])
+@pytest.mark.parametrize("labels_to", [3, 31, 32, 40])
+def test_filter_at_the_edges_of_its_tiles(nv, labels_to):
+    """Vertex counts around the tiles of 32 and 256, labels up to and beyond
+    the slot they share (31), one hub that neighbours every vertex, vertices
+    without neighbours: masks and bitmaps equal the oracle's."""
+    rng = np.random.default_rng(nv * 100 + labels_to)
+    # labels from the top of the range down, so that slot 31 is crowded where there is one
+    labels = (labels_to - 1 - rng.integers(0, min(labels_to, 10), nv)).astype(np.uint32)
+    edges = {(0, v) for v in range(1, nv - 2)}
+    while len(edges) < 3 * nv:
+        a, b = sorted(int(x) for x in rng.integers(0, nv - 2, 2))
+        if a != b:
+            edges.add((a, b))
+    qs = []
+    for k in range(4):
+        nq = 4 + k
+        tree = {(int(rng.integers(0, v)), v) for v in range(1, nq)} | {(0, nq - 1)}
+        ql = np.minimum(labels[rng.integers(0, nv, nq)], 31)
+        qs.append(d.Query.from_edges(ql, sorted(tree)))
+    _filter_case(nv, labels, np.array(sorted(edges), np.uint32), qs)
