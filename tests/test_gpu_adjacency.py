@@ -1,0 +1,57 @@
+"""The in-place merge and removal of adjacency runs (kernels.cu) at the sizes
+where they change hands: runs around a warp's and a block's tile (128, 1024
+entries) and around the length from which a block takes a run (2048), changes
+at the front, the back and everywhere, in place and past the run's capacity,
+and a run emptied and filled again.  Graph and counts (which read the slot
+offsets) must equal the oracle's."""
+import numpy as np
+import pytest
+
+import dsm_b200 as d
+from tests.helpers import oracle_stream
+
+pytestmark = pytest.mark.gpu
+
+
+def _updates(op, vs):
+    u = np.zeros((len(vs), 4), np.uint32)
+    u[:, 0] = op
+    u[:, 2] = vs
+    return u
+
+
+@pytest.mark.parametrize("nlab", [1, 5])
+@pytest.mark.parametrize("deg", [0, 1, 3, 4, 127, 128, 129, 1023, 1025, 2046, 2047, 2048, 2049, 4097, 9001])
+def test_hub_run_grows_and_shrinks(deg, nlab):
+    rng = np.random.default_rng(deg * 10 + nlab)
+    nv = deg + 600
+    labels = rng.integers(0, nlab, nv).astype(np.uint32)
+    others = rng.permutation(np.arange(1, nv))
+    edges = [(0, int(v)) for v in others[:deg]]
+    edges += [(int(a), int(b)) for a, b in rng.integers(1, nv, (300, 2)) if a != b]
+    q = d.Query.from_edges([labels[0], 0, nlab - 1], [(0, 1), (1, 2)])
+    e = d.Engine(0)
+    e.set_option(d.OPT_LIST, 0)
+    e.load_graph_edges(nv, labels, np.array(edges, np.uint32).reshape(-1, 2))
+    qid = e.register(q)
+    st = oracle_stream(nv, labels, np.array(edges, np.uint32).reshape(-1, 2), q)
+    there, absent = np.sort(others[:deg]), np.sort(others[deg:])
+    steps = [
+        _updates(1, absent[:1]),  # one at the front of its label's range
+        _updates(1, absent[-2:]),
+        _updates(1, absent[1:80:3]),
+        _updates(0, there[:1]),
+        _updates(0, there[-3:]),
+        _updates(1, absent),  # past the capacity: the run moves
+        np.concatenate([_updates(0, absent[5:200]), _updates(1, there[:1])]),
+        _updates(0, np.arange(1, nv)),  # empties it
+        _updates(1, others[:deg + 1]),
+    ]
+    for k, b in enumerate(steps):
+        r = e.run_batch(b)
+        s, c, _ = st.apply(b, listed=False)
+        assert np.array_equal(r.signs, s), k
+        assert np.array_equal(r.counts[r.query_index(qid)], c), k
+        for x, y in zip(e.export_graph(), st.export()):
+            assert np.array_equal(x, y), k
+    e.close()
