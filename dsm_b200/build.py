@@ -28,6 +28,7 @@ LIB_SOURCES = [
     "engine/kernels.cu",
     "engine/match.cu",
     "engine/filter.cu",
+    "engine/list.cu",
     "engine/engine.cu",
     "engine/batch.cu",
     "engine/serve.cu",

@@ -11,9 +11,10 @@
 //                  the batch's sizes from a device header)
 //   finish_device  waits for the matcher; regrows the result table and
 //                  reruns on overflow; segment B = deletions and marks; the
+//                  listed tuples to their segments, sorted (list.cu); the
 //                  downloads into the slot's pinned buffers
-//   assemble       waits for the downloads; per-(query, update) counts and
-//                  canonically sorted tuples
+//   assemble       waits for the downloads; per-(query, update) counts,
+//                  offsets and tuples
 //
 // An arena that cannot hold the batch's relocated runs is detected on the
 // device before anything is written: the insert, the matcher and the deletes
@@ -172,6 +173,9 @@ int Engine::launch_front(Staged &S) {
   if (list_mode && S.match) {
     const size_t cap = std::max<uint64_t>(result_cap, 1024);
     if ((rc = dalloc(d_out_seg, cap * 4)) || (rc = dalloc(d_out_tup, cap * S.W * 4))) return rc;
+    // without room for these the table itself crosses to the host
+    S.placed = !dalloc(d_segoff, (S.nseg + 1) * 8) && !dalloc(d_segcur, S.nseg * 4) &&
+               !dalloc(d_segchunk, (S.nseg + 1) * 4) && !dalloc(d_listsum, 3 * kListBlocks * 8);
   }
   // what allocates, synchronises or copies pageable memory runs before the
   // segments, so that each segment can be captured into a CUDA graph
@@ -186,6 +190,8 @@ int Engine::launch_front(Staged &S) {
   if (!H.ev0) {
     CK(cudaEventCreate(&H.ev0));
     CK(cudaEventCreate(&H.ev_end));
+    CK(cudaEventCreate(&H.ev_sort));
+    CK(cudaEventCreate(&H.ev_sorted));
   }
   BatchHdr &hd = *(BatchHdr *)H.hdr.ptr;
   hd.n = n;
@@ -267,6 +273,7 @@ int Engine::launch_front(Staged &S) {
       CK(cudaMemcpyAsync(h_qlisted.ptr, d_qlisted.ptr, (size_t)S.nq_live * 8, cudaMemcpyDeviceToHost, stream));
     return DSM_OK;
   };
+  const ListArgs la = list_args(S);
   if (S.match && filter_mode > 0) filter_timed = true;  // a replayed graph records the filter events too
   if (graphed) {
     // everything the captured nodes bake in: pointers, settings, grids
@@ -286,6 +293,8 @@ int Engine::launch_front(Staged &S) {
     key_append(key, d_rows.ptr);
     key_append(key, d_rows.bytes);
     key_append(key, stall_test);
+    key_append(key, la);
+    key_append(key, S.placed);
     key_append(key, h_sched.ptr);
     key_append(key, h_qlisted.ptr);
     rc = run_segment(0, key, [&]() -> int {
@@ -294,6 +303,10 @@ int Engine::launch_front(Staged &S) {
         if (int r = rec(ev_pool[2])) return r;
         if (int r = launch_match_seq(ma, blocks, bfs_levels)) return r;
         if (int r = rec(ev_pool[3])) return r;
+        if (S.placed) {
+          launch_list_scan(la, stream);
+          stats.kernel_launches += 2;
+        }
       }
       return read_back();
     });
@@ -354,6 +367,10 @@ int Engine::match_eager(Staged &S, MatchArgs &ma, SeedArgs &sa, int blocks) {
     if (int r = rec(ev_pool[2])) return r;
     if (int r = launch_match_seq(ma, blocks, bfs_levels)) return r;
     if (int r = rec(ev_pool[3])) return r;
+    if (S.placed) {
+      launch_list_scan(list_args(S), stream);
+      stats.kernel_launches += 2;
+    }
     CK(cudaMemcpyAsync(h_sched.ptr, d_sched.ptr, sizeof(Sched), cudaMemcpyDeviceToHost, stream));
     CK(cudaMemcpyAsync((char *)h_sched.ptr + sizeof(Sched), d_misc.ptr, 64, cudaMemcpyDeviceToHost, stream));
     if (S.nq_live)
@@ -391,9 +408,64 @@ int Engine::match_eager(Staged &S, MatchArgs &ma, SeedArgs &sa, int blocks) {
   total.out_count.v = out;
   if (int r = rec(ev_pool[3])) return r;
   std::memcpy(hs, &total, sizeof(Sched));
+  if (S.placed) {
+    launch_list_scan(list_args(S), stream);
+    stats.kernel_launches += 2;
+  }
   CK(cudaMemcpyAsync((char *)h_sched.ptr + sizeof(Sched), d_misc.ptr, 64, cudaMemcpyDeviceToHost, stream));
   if (S.nq_live)
     CK(cudaMemcpyAsync(h_qlisted.ptr, d_qlisted.ptr, (size_t)S.nq_live * 8, cudaMemcpyDeviceToHost, stream));
+  return DSM_OK;
+}
+
+ListArgs Engine::list_args(const Staged &S) {
+  ListArgs a;
+  std::memset(&a, 0, sizeof(a));
+  if (!S.placed) return a;
+  a.hdr = (const BatchHdr *)d_hdr.ptr;
+  a.segcnt = (const unsigned long long *)d_segcnt.ptr;
+  a.qlisted = (const unsigned long long *)d_qlisted.ptr;
+  a.qlimit = S.qlimit;
+  a.widths = (const uint32_t *)d_widths.ptr;
+  a.off = (unsigned long long *)d_segoff.ptr;
+  a.cursor = (uint32_t *)d_segcur.ptr;
+  a.chunk = (uint32_t *)d_segchunk.ptr;
+  a.partial = (unsigned long long *)d_listsum.ptr;
+  a.totals = (unsigned long long *)((char *)d_misc.ptr + 32);
+  return a;
+}
+
+// The batch's listed tuples, placed and (DSM_OPT_SORT) sorted: behind the
+// table's rows while the table has room for them, else in d_list.  The rows
+// are scratch for the sort once they are placed.  Without room for d_list they
+// cross to the host, which places and sorts them.
+int Engine::place_results(Staged &S) {
+  S.placed = S.placed && S.listed && S.match_rc == DSM_OK;
+  if (!S.placed) return DSM_OK;
+  const unsigned long long *totals =
+      (const unsigned long long *)((const char *)h_sched.ptr + sizeof(Sched)) + 4;
+  S.words = totals[0];
+  if (!S.words) return DSM_OK;
+  uint32_t *table = (uint32_t *)d_out_tup.ptr;
+  const size_t used = S.cnt * (size_t)S.W;
+  if (used + S.words <= d_out_tup.bytes / 4) {
+    S.out = table + used;
+  } else if (dalloc(d_list, S.words * 4) == DSM_OK) {
+    S.out = (uint32_t *)d_list.ptr;
+  } else {
+    S.placed = false;
+    S.words = 0;
+    return DSM_OK;
+  }
+  const ListArgs a = list_args(S);
+  launch_list_place(a, (const uint32_t *)d_out_seg.ptr, table, S.W, S.cnt, S.out, num_sms, stream);
+  ++stats.kernel_launches;
+  if (S.sort) {
+    CK(cudaEventRecord(hout[S.slot].ev_sort, stream));
+    stats.kernel_launches += launch_list_sort(a, S.W, (size_t)S.nq_live * S.n, totals[1], totals[2],
+                                              S.out, table, num_sms, stream);
+    CK(cudaEventRecord(hout[S.slot].ev_sorted, stream));
+  }
   return DSM_OK;
 }
 
@@ -514,7 +586,12 @@ int Engine::finish_device(Staged &S) {
         if (int r = rec(ev_pool[2])) return r;
         if (int r = launch_match_seq(ma, mblocks, bfs_levels)) return r;
         if (int r = rec(ev_pool[3])) return r;
+        if (S.placed) {
+          launch_list_scan(list_args(S), stream);
+          stats.kernel_launches += 2;
+        }
         CK(cudaMemcpyAsync(h_sched.ptr, d_sched.ptr, sizeof(Sched), cudaMemcpyDeviceToHost, stream));
+        CK(cudaMemcpyAsync((char *)h_sched.ptr + sizeof(Sched), d_misc.ptr, 64, cudaMemcpyDeviceToHost, stream));
         if (S.nq_live)
           CK(cudaMemcpyAsync(h_qlisted.ptr, d_qlisted.ptr, (size_t)S.nq_live * 8, cudaMemcpyDeviceToHost,
                              stream));
@@ -537,9 +614,12 @@ int Engine::finish_device(Staged &S) {
   S.cnt = (S.listed && S.match_rc == DSM_OK) ? (size_t)std::min<unsigned long long>(
                                                    S.sc.out_count.v, d_out_seg.bytes / 4)
                                              : 0;
-  if (S.cnt) {
+  if (int rc = place_results(S)) return rc;
+  if (S.cnt && !S.placed) {
     if (int rc = halloc(H.out_seg, S.cnt * 4)) return rc;
     if (int rc = halloc(H.out_tup, S.cnt * S.W * 4)) return rc;
+  } else if (S.words) {
+    if (int rc = halloc(H.out_tup, S.words * 4)) return rc;
   }
   const bool graphed = use_graph && !S.plain;
   auto seg_b = [&]() -> int {
@@ -557,7 +637,10 @@ int Engine::finish_device(Staged &S) {
     return rc;
   }
   const size_t nn = std::max<uint32_t>(S.n, 1);
-  if (S.cnt) {
+  if (S.placed) {
+    if (S.words)
+      CK(cudaMemcpyAsync(H.out_tup.ptr, S.out, S.words * 4, cudaMemcpyDeviceToHost, stream));
+  } else if (S.cnt) {
     CK(cudaMemcpyAsync(H.out_seg.ptr, d_out_seg.ptr, S.cnt * 4, cudaMemcpyDeviceToHost, stream));
     CK(cudaMemcpyAsync(H.out_tup.ptr, d_out_tup.ptr, S.cnt * S.W * 4, cudaMemcpyDeviceToHost, stream));
   }
@@ -632,8 +715,17 @@ int Engine::assemble(Staged &S, BatchResult &R) {
       R.offsets[s + 1] = R.offsets[s] + (lst ? R.counts[s] * R.widths[ql] : 0);
     }
   R.listed = S.listed;
-  R.tuples.clear();
-  if (S.listed) {
+  R.tuples.resize(0);
+  if (S.placed) {
+    if (S.words != R.offsets.back()) return fail(DSM_ERR_CUDA, "listed words differ from the counts");
+    R.tuples.resize(S.words);
+    const uint32_t *from = (const uint32_t *)H.out_tup.ptr;
+    uint32_t *to = R.tuples.data();
+    parallel_for(S.words, 1u << 19, [&](size_t lo, size_t hi) { std::memcpy(to + lo, from + lo, (hi - lo) * 4); });
+    float ms = 0;
+    if (S.sort && S.words) elapsed(H.ev_sort, H.ev_sorted, &ms);
+    R.sort_ms = ms;
+  } else if (S.listed) {
     R.tuples.resize(R.offsets.back());
     const uint32_t *hs = (const uint32_t *)H.out_seg.ptr, *ht = (const uint32_t *)H.out_tup.ptr;
     const size_t nseg = (size_t)nql * n;

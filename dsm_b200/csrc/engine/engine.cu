@@ -119,6 +119,8 @@ Engine::~Engine() {
       if (b->ptr) cudaFreeHost(b->ptr);
     if (H.ev0) cudaEventDestroy(H.ev0);
     if (H.ev_end) cudaEventDestroy(H.ev_end);
+    if (H.ev_sort) cudaEventDestroy(H.ev_sort);
+    if (H.ev_sorted) cudaEventDestroy(H.ev_sorted);
   }
   for (auto &ev : ev_pool)
     if (ev) cudaEventDestroy(ev);
@@ -130,7 +132,8 @@ std::vector<DevBuf *> Engine::all_dev_bufs() {
                              &d_pair_off, &d_pair_ent, &d_upd, &d_bkey, &d_bidx, &d_binfo, &d_gflag,
                              &d_vtp, &d_dkey, &d_dhead, &d_dsel, &d_seeds, &d_sched, &d_jobs,
                              &d_job_seq, &d_out_seg, &d_out_tup, &d_segcnt, &d_misc, &d_hdr, &d_qlisted, &d_segwork,
-                             &d_rinfo, &d_rmark, &d_rlist, &d_rprev, &d_rows, &d_bloom, &d_fdev};
+                             &d_rinfo, &d_rmark, &d_rlist, &d_rprev, &d_rows, &d_bloom, &d_fdev,
+                             &d_widths, &d_segoff, &d_segcur, &d_segchunk, &d_listsum, &d_list};
   for (auto &q : slots) v.push_back(&q.bitmap);
   for (auto &q : slots) v.push_back(&q.filter_scratch);
   for (auto &q : slots) v.push_back(&q.filter_plan);
@@ -366,10 +369,14 @@ size_t Engine::query_bytes_allocated() const {
 // once every other query retired.
 int Engine::admit(QueryPlan &plan, uint32_t *qid, bool *fits_later, int64_t want_id) {
   const size_t foot = query_footprint(plan);
-  const size_t base = bytes_in_use - std::min(bytes_in_use, query_bytes_allocated());
+  size_t base = bytes_in_use - std::min(bytes_in_use, query_bytes_allocated());
   size_t charged = 0;
   for (const Slot &q : slots)
     if (q.live) charged += q.foot;
+  if (base + charged + foot > budget && d_list.ptr) {  // scratch a listing batch can do without
+    dfree(d_list);
+    base = bytes_in_use - std::min(bytes_in_use, query_bytes_allocated());
+  }
   if (fits_later) *fits_later = base + foot <= budget;
   if (base + charged + foot > budget)
     return fail(DSM_ERR_OOM, "query admission: footprint " + std::to_string(foot) + " bytes exceeds the budget");
@@ -486,6 +493,11 @@ int Engine::sync_queries() {
   if ((rc = dalloc(d_qd, qd.size() * sizeof(QDev))) || (rc = dalloc(d_orders, orders.size() * sizeof(OrderRec))) ||
       (rc = dalloc(d_pair_off, pair_off.size() * 4)) || (rc = dalloc(d_pair_ent, pair_ent.size() * 4)))
     return rc;
+  std::vector<uint32_t> widths;
+  for (uint32_t id : live_ids) widths.push_back(slots[id].plan.nq);
+  if (widths.empty()) widths.push_back(1);
+  if ((rc = dalloc(d_widths, widths.size() * 4))) return rc;
+  CK(cudaMemcpyAsync(d_widths.ptr, widths.data(), widths.size() * 4, cudaMemcpyHostToDevice, stream));
   qd_host = qd;
   CK(cudaMemcpyAsync(d_orders.ptr, orders.data(), orders.size() * sizeof(OrderRec), cudaMemcpyHostToDevice, stream));
   CK(cudaMemcpyAsync(d_pair_off.ptr, pair_off.data(), pair_off.size() * 4, cudaMemcpyHostToDevice, stream));
@@ -507,8 +519,8 @@ int Engine::upload_qd() {
 // Batches
 // ---------------------------------------------------------------------------
 
-// Canonical order of the listed tuples: each (query, update) segment sorted
-// lexicographically, segments shared among host threads (largest first) when
+// Canonical order on the host, for a batch whose results the device had no
+// room to place: each (query, update) segment sorted lexicographically, segments shared among host threads (largest first) when
 // the batch listed enough tuples to pay for the threads.
 void Engine::sort_segments(BatchResult &R, const std::vector<uint64_t> &counts, uint32_t nq_live, uint32_t n,
                            size_t total) {

@@ -56,6 +56,7 @@ struct HostOut {
   HostBuf hdr;     // BatchHdr
   HostBuf segcnt, vtp, out_seg, out_tup, misc;
   cudaEvent_t ev0 = nullptr, ev_end = nullptr;  // batch start, results downloaded
+  cudaEvent_t ev_sort = nullptr, ev_sorted = nullptr;  // around the device sort
 };
 
 // One device batch from host preparation to result assembly.
@@ -78,8 +79,24 @@ struct Staged {
   Sched sc{};
   std::vector<unsigned long long> qlisted;
   int listed = 0, match_rc = 0;
-  size_t cnt = 0;  // listed tuples downloaded
-  float ms_match = 0, ms_upd = 0, ms_filter = 0;
+  size_t cnt = 0;  // table rows
+  bool placed = false;  // results leave the device placed and sorted (list.cu); else as table rows
+  size_t words = 0;     // their words
+  uint32_t *out = nullptr;  // where they lie on the device
+  float ms_match = 0, ms_upd = 0, ms_filter = 0, ms_sort = 0;
+};
+
+// Tuple words of a result: sized once, not cleared (every word is written).
+struct TupleBuf {
+  std::unique_ptr<uint32_t[]> p;
+  size_t n = 0;
+  void resize(size_t words) {
+    p.reset(words ? new uint32_t[words] : nullptr);
+    n = words;
+  }
+  size_t size() const { return n; }
+  uint32_t *data() { return p.get(); }
+  uint32_t &operator[](size_t i) { return p[i]; }
 };
 
 struct BatchResult {
@@ -89,7 +106,7 @@ struct BatchResult {
   std::vector<uint8_t> qlisted;  // per query: its tuples are listed
   std::vector<int8_t> signs;
   std::vector<uint64_t> counts, offsets;
-  std::vector<uint32_t> tuples;
+  TupleBuf tuples;
   int listed = 1;
   double device_ms = 0, match_ms = 0, host_prep_ms = 0, sort_ms = 0;
   uint64_t alg_bytes = 0, matches = 0, incomplete = 0;
@@ -214,7 +231,8 @@ struct Engine {
 
   // batch scratch
   DevBuf d_upd, d_bkey, d_bidx, d_binfo, d_gflag, d_vtp, d_dkey, d_dhead, d_dsel, d_seeds, d_sched, d_jobs,
-      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_bloom, d_fdev;
+      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_bloom, d_fdev,
+      d_widths, d_segoff, d_segcur, d_segchunk, d_listsum, d_list;
   std::vector<FilterDevice> fdev_host;  // what d_fdev holds
   HostBuf h_sched;    // Sched + the error words, read after the matcher
   HostBuf h_qlisted;  // per-query listing counters, read after the matcher
@@ -289,6 +307,8 @@ struct Engine {
   int run_front_and_finish(Staged &S);  // launch_front + finish_or_retry
   int finish_or_retry(Staged &S);       // finish_device; on a refused batch, compact and run it again
   int compact_arena(uint64_t extra_words);
+  ListArgs list_args(const Staged &S);
+  int place_results(Staged &S);
   int match_eager(Staged &S, MatchArgs &ma, SeedArgs &sa, int blocks);  // one launch, or one per query
   int seg_a_kernels(Staged &S, const ClearArgs &ca, const EdgeStateArgs &es, const AdjUpdateArgs &au,
                     const SeedArgs &sa, bool seeds);

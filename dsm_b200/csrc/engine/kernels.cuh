@@ -160,4 +160,28 @@ void launch_match(const MatchArgs &a, int blocks, cudaStream_t s);
 void launch_rows_arm(Sched *sc, const unsigned long long *rows_cnt, unsigned long long rows_cap, cudaStream_t s);
 int match_max_blocks_per_sm();
 
+// Listed results in canonical order on the device (list.cu).
+constexpr uint32_t kListBlocks = 256;
+struct ListArgs {
+  const BatchHdr *hdr;              // n, nseg
+  const unsigned long long *segcnt;
+  const unsigned long long *qlisted;
+  unsigned long long qlimit;
+  const uint32_t *widths;           // [nq_live] tuple words of each query
+  unsigned long long *off;          // [nseg + 1] first word of each segment's tuples
+  uint32_t *cursor;                 // [nseg] tuples placed
+  uint32_t *chunk;                  // [nseg + 1] first sort chunk of each segment
+  unsigned long long *partial;      // [3 * kListBlocks]
+  unsigned long long *totals;       // words, sort chunks, tuples of the largest segment
+};
+// Offsets and totals from the matcher's counts (sizes from the batch header).
+void launch_list_scan(const ListArgs &a, cudaStream_t s);
+// The table's cnt rows (W words each) to their segments' places in `out`.
+void launch_list_place(const ListArgs &a, const uint32_t *seg, const uint32_t *rows, uint32_t W,
+                       unsigned long long cnt, uint32_t *out, int num_sms, cudaStream_t s);
+// Sorts each segment of `out`; `scratch` holds as many words.  Returns the
+// kernels launched.
+int launch_list_sort(const ListArgs &a, uint32_t W, unsigned long long nseg, unsigned long long chunks,
+                     unsigned long long most, uint32_t *out, uint32_t *scratch, int num_sms, cudaStream_t s);
+
 }  // namespace dsm

@@ -296,7 +296,7 @@ void Engine::post_batch(InFlight &b) {
       o->tuples.resize(o->offsets.back());
       for (uint32_t ql = 0; ql < nql; ++ql) {  // each query's slice is contiguous
         const size_t a = R.offsets[(size_t)ql * N + s], e = R.offsets[(size_t)ql * N + s + n];
-        std::copy(R.tuples.begin() + a, R.tuples.begin() + e, o->tuples.begin() + o->offsets[(size_t)ql * n]);
+        if (e > a) std::memcpy(o->tuples.data() + o->offsets[(size_t)ql * n], R.tuples.data() + a, (e - a) * 4);
       }
     }
     o->device_ms = R.device_ms;
