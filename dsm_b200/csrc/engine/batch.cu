@@ -160,7 +160,7 @@ int Engine::launch_front(Staged &S) {
     return rc;
   uint32_t bloom_words = 64;
   while (bloom_words < m) bloom_words *= 2;
-  if ((rc = dalloc(d_bloom, (size_t)bloom_words * 4))) return rc;
+  if ((rc = dalloc(d_bloom, (size_t)bloom_words * 4)) || (rc = dalloc(d_etable, (size_t)bloom_words * 8))) return rc;
   S.work_limit = S.match ? work_limit : 0;
   if (S.work_limit && (rc = dalloc(d_segwork, S.nseg * 8))) return rc;
   if (S.match && (rc = dalloc(d_seeds, S.seed_cap * 16))) return rc;
@@ -220,10 +220,11 @@ int Engine::launch_front(Staged &S) {
   unsigned int *d_err = (unsigned int *)d_misc.ptr;
   unsigned long long *segwork = S.work_limit ? (unsigned long long *)d_segwork.ptr : nullptr;
   ClearArgs ca{dh, (uint32_t *)d_vtp.ptr, (unsigned long long *)d_segcnt.ptr, segwork,
-               (unsigned long long *)d_qlisted.ptr, (Sched *)d_sched.ptr, (uint32_t *)d_misc.ptr, (uint32_t *)d_bloom.ptr};
+               (unsigned long long *)d_qlisted.ptr, (Sched *)d_sched.ptr, (uint32_t *)d_misc.ptr, (uint32_t *)d_bloom.ptr,
+               (uint32_t *)d_etable.ptr};
   EdgeStateArgs es{g, dh, (const uint4 *)d_upd.ptr, (const unsigned long long *)d_bkey.ptr,
                    (const uint32_t *)d_bidx.ptr, (uint32_t *)d_binfo.ptr, (uint8_t *)d_gflag.ptr,
-                   (uint32_t *)d_vtp.ptr, (uint32_t *)d_bloom.ptr};
+                   (uint32_t *)d_vtp.ptr, (uint32_t *)d_bloom.ptr, (uint32_t *)d_etable.ptr};
   AdjUpdateArgs au{g, dh, (const unsigned long long *)d_dkey.ptr, (const uint32_t *)d_dhead.ptr,
                    (const unsigned long long *)d_bkey.ptr, (const uint8_t *)d_gflag.ptr, (uint32_t *)d_dsel.ptr,
                    d_err, (unsigned long long *)((char *)d_misc.ptr + 8),
@@ -235,7 +236,7 @@ int Engine::launch_front(Staged &S) {
   std::memset(&ma, 0, sizeof(ma));
   ma.g = g;
   ma.bt = DevBatchEdges{(const unsigned long long *)d_bkey.ptr, (const uint32_t *)d_binfo.ptr,
-                        (const uint32_t *)d_bloom.ptr, 0, 0};
+                        (const uint32_t *)d_bloom.ptr, (const uint32_t *)d_etable.ptr, 0, 0};
   ma.hdr = dh;
   ma.vtp = (const uint32_t *)d_vtp.ptr;
   ma.qd = (const QDev *)d_qd.ptr;
@@ -258,7 +259,6 @@ int Engine::launch_front(Staged &S) {
   ma.split_min = split_min;
   ma.donate_depth = donate_depth;
   ma.pack_max = pack_max;
-  ma.merge_max = merge_max;
   ma.out_seg = (uint32_t *)d_out_seg.ptr;
   ma.out_tup = (uint32_t *)d_out_tup.ptr;
   ma.cap = list_mode ? std::min<unsigned long long>(d_out_seg.bytes / 4, d_out_tup.bytes / 4 / ma.W) : 0;
@@ -546,7 +546,7 @@ int Engine::finish_device(Staged &S) {
       std::memset(&ma, 0, sizeof(ma));
       ma.g = g;
       ma.bt = DevBatchEdges{(const unsigned long long *)d_bkey.ptr, (const uint32_t *)d_binfo.ptr,
-                        (const uint32_t *)d_bloom.ptr, 0, 0};
+                        (const uint32_t *)d_bloom.ptr, (const uint32_t *)d_etable.ptr, 0, 0};
       ma.hdr = dh;
       ma.vtp = (const uint32_t *)d_vtp.ptr;
       ma.qd = (const QDev *)d_qd.ptr;
@@ -569,8 +569,7 @@ int Engine::finish_device(Staged &S) {
       ma.split_min = split_min;
       ma.donate_depth = donate_depth;
       ma.pack_max = pack_max;
-      ma.merge_max = merge_max;
-      ma.out_seg = (uint32_t *)d_out_seg.ptr;
+          ma.out_seg = (uint32_t *)d_out_seg.ptr;
       ma.out_tup = (uint32_t *)d_out_tup.ptr;
       ma.cap = std::min<unsigned long long>(d_out_seg.bytes / 4, d_out_tup.bytes / 4 / S.W);
       const int mblocks = num_sms * (warps_per_sm ? std::max(1, warps_per_sm / 8) : default_blocks_per_sm());
@@ -859,9 +858,9 @@ int Engine::compact_arena(uint64_t extra_words) {
 // ---------------------------------------------------------------------------
 // The matcher's result does not depend on its launch shape or on how work is
 // donated, so the batch's own matcher launch is repeated on the same union
-// graph (counts only) for each candidate -- first the intersection tile
-// (packed last level), then resident blocks per SM x range-split threshold x
-// donation depth at the best tile -- timed with events, and the fastest
+// graph (counts only) for each candidate -- first the plan (breadth-first
+// levels), then the batch (one partial embedding or 32), then resident blocks
+// per SM x range-split threshold x donation depth -- timed with events, and the fastest
 // becomes the engine's setting.  The first candidate runs twice and its first
 // run is not counted (it warms L2 for all).
 int Engine::autotune(MatchArgs &ma, const Staged &S, int &blocks) {
@@ -902,7 +901,6 @@ int Engine::autotune(MatchArgs &ma, const Staged &S, int &blocks) {
       t.split_min = c.split;
       t.donate_depth = c.dd;
       t.pack_max = c.pack;
-      t.merge_max = c.merge;
       CK(cudaEventRecord(e0, stream));
       if (int r = launch_match_seq(t, num_sms * c.bps, c.bfs)) return r;
       CK(cudaEventRecord(e1, stream));
@@ -923,7 +921,7 @@ int Engine::autotune(MatchArgs &ma, const Staged &S, int &blocks) {
     }
     return DSM_OK;
   };
-  const Cand cur{blocks / std::max(num_sms, 1), ma.split_min, ma.donate_depth, ma.pack_max, ma.merge_max,
+  const Cand cur{blocks / std::max(num_sms, 1), ma.split_min, ma.donate_depth, ma.pack_max, merge_max,
                  bfs_levels};
   // stage 0: depth-first or breadth-first rows for the first 1 or 2 levels
   std::vector<Cand> c0;
@@ -932,11 +930,10 @@ int Engine::autotune(MatchArgs &ma, const Staged &S, int &blocks) {
   Cand b0 = cur;
   if (d_rows.ptr)
     if (int rc = sweep(c0, true, b0, best0)) return rc;
-  // stage 1: the intersection tile -- packed last level x merge threshold --
-  // at the current launch shape
+  // stage 1: one partial embedding at a time or 32, at the current launch shape
   std::vector<Cand> c1;
-  for (uint32_t pk : {0u, 256u, 1024u, 4096u})
-    for (uint32_t mg : {0u, 64u, 256u}) c1.push_back({cur.bps, cur.split, cur.dd, pk, mg, b0.bfs});
+  for (uint32_t pk : {0u, cur.pack ? cur.pack : 1024u})
+    c1.push_back({cur.bps, cur.split, cur.dd, pk, cur.merge, b0.bfs});
   Cand b1 = b0, bc = b0;
   if (!stop)
     if (int rc = sweep(c1, !d_rows.ptr, b1, best1)) return rc;
@@ -958,7 +955,6 @@ int Engine::autotune(MatchArgs &ma, const Staged &S, int &blocks) {
     stats.tune_best_ms = best2;
   }
   ma.pack_max = pack_max;
-  ma.merge_max = merge_max;
   ma.split_min = split_min;
   ma.donate_depth = donate_depth;
   blocks = num_sms * (warps_per_sm ? std::max(1, warps_per_sm / 8) : default_blocks_per_sm());

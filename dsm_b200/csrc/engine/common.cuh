@@ -64,10 +64,13 @@ __device__ __forceinline__ const uint32_t *adj_list(const DevGraph &g, uint2 a) 
 // batch, one B200: 64 twelve-vertex queries x 32,768 updates on a hub-heavy
 // 2^22-edge graph 63 -> 53 ms, 256 queries x 1021 updates on a 2^22-edge
 // power-law graph 85 -> 76 ms, three queries x 4096 updates 6.7 -> 4.4 ms.
+// table: where a changed key's entries start in bkey (index + 1; 0: empty),
+// hashed with linear probing, 2 (bloom_mask + 1) slots: at most half full.
 struct DevBatchEdges {
   const unsigned long long *bkey;
   const uint32_t *binfo;
   const uint32_t *bloom;
+  const uint32_t *table;
   uint32_t n;           // keys (set by the matcher from the batch header)
   uint32_t bloom_mask;  // (set by the matcher from the batch header)
 };
@@ -90,17 +93,29 @@ __device__ __forceinline__ bool may_change(const DevBatchEdges &t, uint32_t x, u
   return (t.bloom[word] & bits) == bits;
 }
 
-// Edges of the union graph that the batch does not name were present before
+// The key's first slot in the batch's table (mask: slots - 1).
+__device__ __forceinline__ uint32_t table_slot(unsigned long long key, uint32_t mask) {
+  const uint32_t h = ((uint32_t)key * 0x9E3779B1u) ^ ((uint32_t)(key >> 32) * 0x85EBCA6Bu);
+  return (h ^ (h >> 15)) & mask;
+}
+
+// Edges of the union graph that the batch does not change were present before
 // it and stay; otherwise the last update before tp decides, else the initial
-// state.
+// state.  Three dependent loads through the table; a search of bkey took 15 on
+// a 32,768-update batch, and two of five chunks of a hub-heavy graph had one.
 __device__ __forceinline__ bool edge_live(const DevBatchEdges &t, uint32_t x, uint32_t y, uint32_t tp) {
-  unsigned long long key = canon_key(x, y);
-  uint32_t lo = 0, hi = t.n;
-  while (lo < hi) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (t.bkey[mid] < key) lo = mid + 1; else hi = mid;
+  const unsigned long long key = canon_key(x, y);
+  const uint32_t mask = 2 * t.bloom_mask + 1;
+  uint32_t lo = 0, s = table_slot(key, mask);
+  while (true) {
+    const uint32_t at = t.table[s];
+    if (at == 0) return true;
+    if (t.bkey[at - 1] == key) {
+      lo = at - 1;
+      break;
+    }
+    s = (s + 1) & mask;
   }
-  if (lo >= t.n || t.bkey[lo] != key) return true;
   uint32_t info = t.binfo[lo];
   bool live = (info >> 31) & 1u;
   for (uint32_t j = lo; j < t.n && t.bkey[j] == key; ++j) {
@@ -119,6 +134,21 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t *a, uint32_t 
     if (a[mid] < x) lo = mid + 1; else hi = mid;
   }
   return lo;
+}
+
+// Whether x is among the n entries of a sorted range.  Keeps the last entry
+// not above x in front: seven instructions a step, two fewer than lower_bound
+// (the matcher spends a quarter of its time here; interpolating the place, or
+// three probes a step, took fewer dependent loads and as long).
+__device__ __forceinline__ bool run_has(const uint32_t *a, uint32_t n, uint32_t x) {
+  if (n == 0) return false;
+#pragma unroll 1
+  while (n > 1) {
+    const uint32_t h = n >> 1;
+    if (a[h] <= x) a += h;
+    n -= h;
+  }
+  return *a == x;
 }
 
 __device__ __forceinline__ uint32_t lanemask_lt() {

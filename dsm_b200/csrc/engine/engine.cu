@@ -132,7 +132,7 @@ std::vector<DevBuf *> Engine::all_dev_bufs() {
                              &d_pair_off, &d_pair_ent, &d_upd, &d_bkey, &d_bidx, &d_binfo, &d_gflag,
                              &d_vtp, &d_dkey, &d_dhead, &d_dsel, &d_seeds, &d_sched, &d_jobs,
                              &d_job_seq, &d_out_seg, &d_out_tup, &d_segcnt, &d_misc, &d_hdr, &d_qlisted, &d_segwork,
-                             &d_rinfo, &d_rmark, &d_rlist, &d_rprev, &d_rows, &d_bloom, &d_fdev,
+                             &d_rinfo, &d_rmark, &d_rlist, &d_rprev, &d_rows, &d_bloom, &d_etable, &d_fdev,
                              &d_widths, &d_segoff, &d_segcur, &d_segchunk, &d_listsum, &d_list};
   for (auto &q : slots) v.push_back(&q.bitmap);
   for (auto &q : slots) v.push_back(&q.filter_scratch);
@@ -159,7 +159,7 @@ int Engine::init(int dev, size_t mem_budget) {
   list_limit_bytes = std::min<uint64_t>(list_limit_bytes, budget / 4);
   ev_pool.resize(8, nullptr);
   for (auto &ev : ev_pool) CK(cudaEventCreate(&ev));
-  int per_sm = match_max_blocks_per_sm();
+  int per_sm = match_max_blocks_per_sm(4);
   match_blocks_per_sm = std::max(1, std::min(per_sm, 8));
   // small fixed buffers
   if (int rc = dalloc(d_sched, sizeof(Sched))) return rc;

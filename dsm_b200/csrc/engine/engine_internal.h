@@ -164,8 +164,7 @@ struct Engine {
   int num_sms = 148;
   int clock_khz = 1965000;
   int match_blocks_per_sm = 2;  // most resident matcher blocks per SM (the tuner's upper end)
-  // untuned launch shape: 4 blocks per SM, the 64-register variant (the
-  // 48-register one spills; tuning on config 2 and 4 picked 4 and 3 blocks)
+  // untuned launch shape: 4 blocks per SM, all that 64 registers a thread allow
   int default_blocks_per_sm() const { return std::max(1, std::min(match_blocks_per_sm, 4)); }
   std::mutex mu;
   std::mutex emu;          // guards last_error (written by the serving worker too)
@@ -189,8 +188,8 @@ struct Engine {
   int label_quirk = 0;
   int sort_results = 1;
   uint32_t split_min = 0, donate_depth = 0;  // donation granularity (0 = kernel default)
-  uint32_t pack_max = 1024;                  // packed last level (entries per pass; 0: off)
-  uint32_t merge_max = 64;                   // merge intersection up to this probe range (0: off)
+  uint32_t pack_max = 1024;                  // 0: partial embeddings one at a time; else in batches
+  uint32_t merge_max = 64;                   // kept for its callers (the batches have no merges)
   uint32_t bfs_levels = 0;                   // breadth-first rows: levels beyond the seed (0: depth-first)
   uint64_t bfs_rows = 1u << 20;              // row table capacity
   DevBuf d_rows;
@@ -231,7 +230,7 @@ struct Engine {
 
   // batch scratch
   DevBuf d_upd, d_bkey, d_bidx, d_binfo, d_gflag, d_vtp, d_dkey, d_dhead, d_dsel, d_seeds, d_sched, d_jobs,
-      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_bloom, d_fdev,
+      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_bloom, d_etable, d_fdev,
       d_widths, d_segoff, d_segcur, d_segchunk, d_listsum, d_list;
   std::vector<FilterDevice> fdev_host;  // what d_fdev holds
   HostBuf h_sched;    // Sched + the error words, read after the matcher

@@ -32,7 +32,7 @@ struct ClearArgs {
   unsigned long long *qlisted;
   Sched *sc;
   uint32_t *misc;  // 64 words
-  uint32_t *bloom;
+  uint32_t *bloom, *table;  // of the changed edges (DevBatchEdges)
 };
 void launch_batch_clear(const ClearArgs &a, int blocks, cudaStream_t s);
 
@@ -47,7 +47,7 @@ struct EdgeStateArgs {
   uint32_t *binfo;                // [m] idx | op << 30 | init << 31
   uint8_t *gflag;                 // [m] 1: union insert, 2: final delete
   uint32_t *vtp;                  // [n] view time (updates applied) or kNoView
-  uint32_t *bloom;                // filter over the keys the batch changes (cleared before)
+  uint32_t *bloom, *table;        // filter and table of the keys the batch changes (cleared before)
 };
 void launch_edge_state(const EdgeStateArgs &a, int blocks, cudaStream_t s);
 
@@ -131,13 +131,8 @@ struct MatchArgs {
   // donated when at least donate_depth levels lie below them (1..4)
   uint32_t split_min;
   uint32_t donate_depth;
-  // packed last level (label-major runs): at most this many entries laid end
-  // to end in one pass over a chunk's candidates (0: candidates one at a time)
+  // 0: partial embeddings expanded one at a time; else 32 together
   uint32_t pack_max;
-  // merge intersection: a probe range of at most this many entries is
-  // walked in tiles against the whole chunk instead of searched per entry
-  // (0: always searched)
-  uint32_t merge_max;
   // breadth-first rows: in a launch with bfs_stop > 0, a task that finds
   // candidates completing bfs_stop positions (with at least two positions
   // left) writes each prefix as a row to rows_out instead of descending,
@@ -158,7 +153,9 @@ void launch_match(const MatchArgs &a, int blocks, cudaStream_t s);
 // with the rows written so far as its tasks (counters of work done, the
 // result-table position and the error word carry over).
 void launch_rows_arm(Sched *sc, const unsigned long long *rows_cnt, unsigned long long rows_cap, cudaStream_t s);
-int match_max_blocks_per_sm();
+// Resident matcher blocks per SM for queries of up to `width` vertices (0:
+// plain runs).
+int match_max_blocks_per_sm(uint32_t width);
 
 // Listed results in canonical order on the device (list.cu).
 constexpr uint32_t kListBlocks = 256;

@@ -2,30 +2,23 @@
 // the work queue of queue.cuh / job_queue.cuh).
 //
 // One warp per task.  A task fixes positions 0..depth-1 of a matching order
-// and enumerates the rest depth-first.  The stack is spread over the lanes:
-// lane p keeps the image f[p] of position p with its adjacency run, and the
-// iteration state of level p (pivot run, next chunk, pending candidates of the
-// current chunk).  Candidates of level p are produced 32 at a time from the
-// run of the backward neighbour with the fewest neighbours (the pivot): each
-// lane tests one element (label, injectivity, filter bit, membership in the
-// other backward neighbours' runs, liveness at the update's view time) and a
-// ballot gives the chunk's candidate mask.  Membership in a short range is
-// a warp merge over 32-entry tiles, in a long one a binary search; the last
-// level of a chunk's candidates is evaluated in one packed pass, with the
-// longest shared range staged in shared memory.  Nothing is materialised,
-// except, with breadth-first levels, the rows a first launch hands to a
-// second.
+// and enumerates the rest depth-first, up to 32 partial embeddings of a level
+// at a time, a lane each: their candidate ranges are laid end to end and
+// scanned 32 entries a step, each lane testing one entry (injectivity, filter
+// bit, membership in the other backward neighbours' label ranges, liveness at
+// the update's view time), and 32 survivors make the next level's batch.
+// Nothing is materialised, except, with breadth-first levels, the rows a first
+// launch hands to a second.
 //
 // Scheduling.  Tasks are first the seeds (one atomicAdd each), then donated
 // jobs.  An idle warp takes a ticket (one atomicAdd on pop_cnt) and waits for
 // its own job slot to be published, polling only that slot's flag with
 // exponential backoff.  Busy warps see pop_cnt - push_cnt warps waiting and
-// donate to them: pending candidates of their shallowest level with at least
-// two levels below it, or half of a long remaining run.  The warp whose task
+// donate to them from their shallowest level with a substantial piece: partial
+// embeddings with at least two levels below them, or half of the entries left.  The warp whose task
 // completion brings `outstanding` to zero sets `done` and marks every
 // still-waiting ticket's slot as finished.  Every wait is bounded by a clock
 // budget that restarts whenever busy warps show progress.
-#include <algorithm>
 
 #include "kernels.cuh"
 
@@ -39,28 +32,6 @@ __device__ __forceinline__ T ld_volatile(const T &x) {
 }
 
 constexpr unsigned long long kSeqDone = 1ull << 63;
-
-// One candidate of a packed last level: where its pivot range starts in the
-// concatenation (excl), its id, its own range of the last level's label
-// (run offset in 16-byte units, [a, b)), own (1: its own range is the pivot).
-struct alignas(16) PackEnt {
-  uint32_t excl, cw, off, a, b, own, pad0, pad1;
-};
-
-// Staged probe range of a packed last level (per warp, shared memory): the
-// longest last-level range in the run of a fixed position, whole when it has
-// at most kStage entries, else every 2^shift-th entry (fences); staged once
-// per level-(nq - 2) context, when first packed, if it has kStageMin entries
-// or more.  info = lane | shift << 5 | fences << 10, kStageNone: none,
-// kStageUnset: not decided yet for this context.
-constexpr uint32_t kStage = 512;
-constexpr uint32_t kStageMin = 32;
-constexpr uint32_t kStageNone = 0xFFFFFFFEu;
-constexpr uint32_t kStageUnset = 0xFFFFFFFFu;
-struct PackStage {
-  uint32_t fence[kStage];
-  uint32_t info;
-};
 
 // Lane 0 only.  Returns 1 (seed `slot`), 2 (job of ticket `slot`; the caller
 // releases the ring slot after reading it) or 0 (no more work).
@@ -133,58 +104,70 @@ __device__ void finish_task(const MatchArgs &P) {
     atomicExch(&P.job_seq[t & (P.job_ring - 1)], t | kSeqDone);
 }
 
-// kLM: label-major runs with slot offsets (the engine's graph); otherwise
-// plain id-sorted runs.  srng[L][j]: for level L and backward neighbour j,
-// the range of j's run holding the label of level L (label-major only).
+// ---------------------------------------------------------------------------
+// Label-major runs (the engine's graph)
+// ---------------------------------------------------------------------------
+// A task's search goes depth-first over batches: up to 32 partial embeddings
+// of one level, a lane each, are expanded together.  E(l) is the expansion of
+// the batch of level l (its partials fix positions 0..l) to level t = l + 1:
+// each lane reads its partial's ranges of t's label in the runs of t's
+// backward neighbours and takes the shortest as its pivot; the pivot ranges
+// are laid end to end (a warp scan of their lengths) and scanned 32 entries at
+// a time, each lane finding its entry's owner by a five-step search through
+// the scan.  Survivors are appended to level t's buffer; 32 of them, or the
+// rest when the ranges end, become the next batch.
 //
-// The level being scanned (the current level) keeps its iteration state in
-// warp-uniform registers (cur_*), so a chunk reads no lane's state; a level
-// with deeper levels running parks its state in lane L (lv_*) and takes it
-// back by shuffle when the search returns to it.
+// Bound by the warp's instructions and dependent loads, not by bandwidth (L2
+// hit 94 %, DRAM idle).  One partial at a time, a level's set-up, descent and
+// return were paid per candidate (about 2000 cycles each, half the matcher's
+// time on queries of 8 to 12 vertices) and a chunk of one short range left most
+// lanes idle; a batch pays them once for 32 and its chunks are full (31 of 32
+// lanes, where 16 to 19 had an entry).  About 370 instructions a chunk, a
+// quarter of them the search of the other ranges, at 0.6 issued a cycle (8
+// warps a scheduler at 64 registers).  Matcher time of one batch, one B200: 64
+// twelve-vertex queries x 32,768 updates on a hub-heavy 2^22-edge graph 51 ->
+// 18 ms; 256 queries x 1021 updates on a 2^22-edge power-law graph 75 -> 42 ms;
+// three queries x 4096 updates on a 2^24-edge one 86 -> 46 ms; one request of
+// 512 updates against 64 queries 5.5 -> 2.6 ms.
 //
-// Packed last level (label-major runs, P.pack_max > 0).  When a chunk of
-// level nq - 2 leaves candidates, the last level of all of them is evaluated
-// in one pass.  Candidate k's pivot range is the shortest of the last level's
-// backward ranges: those in the runs of fixed positions are the same for every
-// candidate (set up with level nq - 2), the one in the candidate's own run is
-// its own.  The pivot ranges are laid end to end (an inclusive warp scan of
-// their lengths) and scanned 32 entries at a time, each lane finding its
-// candidate by a five-step search over the scan, so short sibling ranges fill
-// whole chunks instead of one mostly idle chunk each.  When the ranges total
-// more than pack_max entries the candidates are expanded one at a time instead,
-// where long ranges can be split and donated.
-template <bool kLM>
+// Shared memory of a warp (W = widest query): the batch's images F[W][32]
+// (column k: the partial of lane k), up to kRows ranges per partial, the pivot
+// per partial, and a buffer of 64 survivors per level (id | parent << 27).
+constexpr uint32_t kRows = 3;  // backward neighbours with stored ranges; further ones are read when needed
+__host__ __device__ constexpr uint32_t warp_words(uint32_t W) {
+  return W * 32 + kRows * 128 + 128 + (W > 3 ? W - 3 : 1) * 64;
+}
+
 __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t nupd, uint32_t upd, uint32_t qo,
-                         uint32_t depth, uint32_t lo, uint32_t hi, uint32_t fval, uint2 (*srng)[16],
-                         PackEnt *spk, PackStage *stg) {
+                         uint32_t depth, uint32_t lo, uint32_t hi, uint32_t fval, uint32_t *sm) {
   const uint32_t lane = threadIdx.x & 31;
+  uint32_t(*const F)[32] = reinterpret_cast<uint32_t(*)[32]>(sm);
+  uint4(*const rows)[32] = reinterpret_cast<uint4(*)[32]>(sm + P.W * 32);
+  uint4 *const piv = reinterpret_cast<uint4 *>(sm + P.W * 32 + kRows * 128);
+  uint32_t(*const buf)[64] = reinterpret_cast<uint32_t(*)[64]>(sm + P.W * 32 + kRows * 128 + 128) - 2;  // from level 2
   const QDev &Q = P.qd[qo >> 8];
   const uint32_t nq = Q.nq;
   const OrderRec &R = P.orders[Q.order_base + (qo & 255)];
+  // lane p: position p's backward neighbours, label and query vertex; lane k:
+  // query vertex k's position
   const uint32_t q_vert = lane < 16 ? R.vert[lane] : 0;
-  const uint32_t q_pos = lane < 16 ? R.pos_of[lane] : 0;
-  const uint32_t q_bn = lane < 16 ? R.bn[lane] : 0;
-  const uint32_t q_lab = Q.label[q_vert & 15];
+  const uint32_t q_word = lane < 16 ? R.bn[lane] | (Q.label[q_vert & 15] << 16) | (q_vert << 21) |
+                                          ((uint32_t)R.pos_of[lane] << 25)
+                                    : 0u;
   const uint32_t tp = P.vtp[upd];
   const uint32_t *bitmap = Q.bitmap;
-  const uint32_t col_len = Q.col_len;
   const uint32_t seg = Q.local * nupd + upd;
+  unsigned long long task_cnt = 0, work = 0;  // warp-uniform
+  uint32_t alg = 0;                           // bytes, this lane's share
+  // what the segment had left of its work limit when this task last looked
+  // (at most 2^32 - 1): a task that alone exceeds it publishes at once
+  uint32_t work_left = 0xFFFFFFFFu;
 
-  uint32_t my_f = fval, my_off = 0, my_deg = 0, my_touch = 0;
-  if (lane < depth) {
-    uint2 a = P.g.adj[my_f];
-    my_off = a.x;
-    my_deg = a.y;
-    my_touch = P.g.lab[my_f] >> 31;
-  }
-  unsigned long long alg = 0, task_cnt = 0;  // warp-uniform
-
-  // The chunk's candidates m are embeddings: position L holds each lane's w,
-  // position pv (if any) each lane's cv, the others the stack.  Listing
-  // reserves slots in the result table; a query past its listing budget
-  // reserves none (its count stays exact, the host drops its partial tuples).
-  auto emit = [&](uint32_t m, uint32_t w, uint32_t L, uint32_t pv, uint32_t cv) {
-    uint32_t cnt = __popc(m);
+  // Listing reserves slots in the result table; a query past its listing
+  // budget reserves none (its count stays exact, the partial tuples are
+  // dropped).  Survivors m hold w at position t, F's column k before it.
+  auto emit = [&](uint32_t m, uint32_t w, uint32_t t, uint32_t k) {
+    const uint32_t cnt = __popc(m);
     if (cnt == 0) return;
     task_cnt += cnt;
     if (!P.list) return;
@@ -196,16 +179,14 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
     }
     base = __shfl_sync(kFull, base, 0);
     if (base == ~0ull) return;
-    alg += 4ull * (nq + 1) * cnt;  // the tuple and its segment id
-    bool mine = (m >> lane) & 1u;
-    unsigned long long s = base + __popc(m & lanemask_lt());
-    bool wr = mine && s < P.cap;
+    const unsigned long long s = base + __popc(m & lanemask_lt());
+    const bool wr = ((m >> lane) & 1u) && s < P.cap;
     if (wr) P.out_seg[s] = seg;
-    for (uint32_t k = 0; k < nq; ++k) {
-      uint32_t pk = __shfl_sync(kFull, q_pos, k);
-      uint32_t fk = __shfl_sync(kFull, my_f, pk & 31);
-      if (wr) P.out_tup[s * P.W + k] = (pk == L) ? w : (pk == pv ? cv : fk);
+    for (uint32_t v = 0; v < nq; ++v) {
+      const uint32_t p = __shfl_sync(kFull, q_word, v) >> 25;
+      if (wr) P.out_tup[s * P.W + v] = p == t ? w : F[p][k];
     }
+    if (wr) alg += 4 * (nq + 1);
   };
 
   // Work limit (P.work_limit > 0): `work` counts the valid partial
@@ -214,20 +195,428 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   // scheduling, so "the segment's total reached the limit" is deterministic:
   // whoever's addition crosses it sets bit 63 of the segment's count, and the
   // segment's tasks stop (its count is then partial, marked by that bit).
-  unsigned long long work = 0;
   auto publish_work = [&]() -> bool {  // true: the segment is over its limit
-    uint32_t over = 0;
+    uint32_t left = 0;
     if (lane == 0) {
       const unsigned long long before = work ? atomicAdd(&P.seg_work[seg], work) : ld_volatile(P.seg_work[seg]);
-      over = before + work >= P.work_limit;
-      if (work && before < P.work_limit && over) atomicOr(&P.seg_count[seg], kCountIncomplete);
+      if (before + work < P.work_limit) left = (uint32_t)min(P.work_limit - before - work, 0xFFFFFFFFull);
+      else if (work && before < P.work_limit) atomicOr(&P.seg_count[seg], kCountIncomplete);
     }
     work = 0;
-    return __shfl_sync(kFull, over, 0) != 0;
+    work_left = __shfl_sync(kFull, left, 0);
+    return work_left == 0;
   };
 
   auto flush = [&]() {
     if (P.work_limit && work) publish_work();
+    const uint32_t a0 = __reduce_add_sync(kFull, alg & 0xFFFFu), a1 = __reduce_add_sync(kFull, alg >> 16);
+    if (lane == 0) {
+      if (task_cnt) {
+        atomicAdd(&P.seg_count[seg], task_cnt);
+        atomicAdd(&P.sc->matches, task_cnt);
+      }
+      atomicAdd(&P.sc->alg_bytes, ((unsigned long long)a1 << 16) + a0);
+    }
+  };
+
+  __syncwarp();  // the last task's reads of the warp's shared memory are done
+  for (uint32_t p = 0; p < depth; ++p) F[p][lane] = __shfl_sync(kFull, fval, p);
+  __syncwarp();
+  if (depth >= nq) {  // a one-edge query: the seed is the embedding
+    emit(1u, 0, 0xFFFFFFFFu, 0);
+    flush();
+    return;
+  }
+  if (P.work_limit && publish_work()) return;  // a segment already over its limit
+
+  // the expansion at hand, E(l) to level t = l + 1 (warp-uniform): next and
+  // last entry of the ranges laid end to end, partials of the batch, survivors
+  // in t's buffer; t's backward neighbours, label, and the earlier positions
+  // with that label
+  uint32_t l = depth - 1, c = 0, e = 0, nb = 1, cnt = 0, t_bn = 0, t_lab = 0, t_same = 0;
+  uint32_t incl = 0, len = 0;               // lane k: scan of the pivot ranges, this partial's
+  // E(lane), parked while deeper ones run: lv_n = nb | cnt << 8 | partials
+  // whose range is not begun << 16
+  uint32_t lv_c = 0, lv_e = 0, lv_n = 0;
+  const uint32_t most = P.pack_max ? 32u : 1u;  // partials expanded together
+
+  // The ranges of E(l)'s partials (F holds the batch); returns their total.
+  auto setup = [&]() -> uint32_t {
+    const uint32_t tw = __shfl_sync(kFull, q_word, l + 1);
+    t_bn = tw & 0xFFFFu;
+    t_lab = (tw >> 16) & 31u;
+    t_same = __ballot_sync(kFull, lane <= l && ((q_word >> 16) & 31u) == t_lab);
+    uint32_t best = 0xFFFFFFFFu, pr = 0, pa = 0, poff = 0, r = 0;
+    for (uint32_t bits = t_bn; bits; bits &= bits - 1, ++r) {
+      uint32_t a = 0, b = 0, off = 0, touched = 0;
+      if (lane < nb && t_lab < P.g.nlt) {
+        const uint32_t x = F[__ffs(bits) - 1][lane];
+        const uint32_t *o = P.g.loff + (size_t)x * (P.g.nlt + 1) + t_lab;
+        a = o[0];
+        b = o[1];
+        off = P.g.adj[x].x;
+        touched = P.g.lab[x] >> 31;
+        alg += 8;
+      }
+      if (r < kRows) rows[r][lane] = make_uint4(off, a, b, touched);
+      if (b - a < best) {
+        best = b - a;
+        pr = r;
+        pa = a;
+        poff = off;
+      }
+    }
+    len = lane < nb ? best : 0u;
+    incl = len;
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+      const uint32_t x = __shfl_up_sync(kFull, incl, d);
+      if (lane >= d) incl += x;
+    }
+    const uint64_t start = (uint64_t)poff * 4 + pa - (incl - len);  // entry i of the scan is arena[start + i]
+    piv[lane] = make_uint4((uint32_t)start, (uint32_t)(start >> 32), pr, pa);
+    __syncwarp();
+    return __shfl_sync(kFull, incl, 31);
+  };
+
+  auto park = [&]() {
+    const uint32_t excl = incl - len;
+    const uint32_t todo = __popc(__ballot_sync(kFull, len && excl >= c && excl < e));
+    if (lane == l) {
+      lv_c = c;
+      lv_e = e;
+      lv_n = nb | (cnt << 8) | (todo << 16);
+    }
+  };
+
+  // F for the batch of level l from the buffers (levels depth..l).
+  auto rebuild = [&]() {
+    __syncwarp();
+    uint32_t k = lane;
+    for (uint32_t j = l; j >= depth; --j) {
+      const uint32_t x = buf[j][k];
+      F[j][lane] = x & kIdMask;
+      k = x >> kIdBits;
+    }
+    __syncwarp();
+  };
+
+  // The survivors m of E(l) (lane: image w, owner k) as rows of l + 2 fixed
+  // positions.  One reservation per chunk, all or nothing (a bounded
+  // compare-and-swap loop); false: no room, nothing written.
+  auto write_rows = [&](uint32_t m, uint32_t w, uint32_t k) -> bool {
+    const uint32_t n = __popc(m);
+    unsigned long long base = ~0ull;
+    if (lane == 0) {
+      unsigned long long cur = ld_volatile(*P.rows_cnt);
+      for (int tries = 0; tries < 64 && cur + n <= P.rows_cap; ++tries) {
+        const unsigned long long prev = atomicCAS(P.rows_cnt, cur, cur + n);
+        if (prev == cur) {
+          base = cur;
+          break;
+        }
+        cur = prev;
+      }
+    }
+    base = __shfl_sync(kFull, base, 0);
+    if (base == ~0ull) return false;
+    if ((m >> lane) & 1u) {
+      uint32_t *rec = reinterpret_cast<uint32_t *>(P.rows_out + base + __popc(m & lanemask_lt()));
+      __stcg(rec, upd);
+      __stcg(rec + 1, qo);
+      __stcg(rec + 2, l + 2);
+      for (uint32_t j = 0; j <= l; ++j) __stcg(rec + 8 + j, F[j][k]);
+      __stcg(rec + 9 + l, w);
+    }
+    return true;
+  };
+
+  e = setup();
+  if (hi) {  // a donated part [lo, hi) of the one partial's pivot range
+    const uint32_t pa = piv[0].w;
+    c = lo - pa;
+    e = min(e, hi - pa);
+  }
+  uint32_t hb = 0;     // chunks since the last heartbeat
+  int32_t dticks = 0;  // chunks since the last donation check (below zero: none for a while)
+  while (true) {
+    if (c < e && cnt < most) {
+      const uint32_t t = l + 1, pos = c + lane;
+      bool ok = pos < e;
+      uint32_t k = 0;  // the owner: the first lane with incl > pos
+#pragma unroll
+      for (uint32_t d = 16; d; d >>= 1) {
+        const uint32_t v = __shfl_sync(kFull, incl, k + d - 1);
+        if (v <= pos) k += d;
+      }
+      const uint4 pv = piv[k];
+      const uint32_t en = ok ? P.g.arena[((uint64_t)pv.y << 32 | pv.x) + pos] : 0u;
+      const uint32_t w = en & kIdMask;
+      if (ok) alg += 4;
+      c = min(c + 32, e);
+      if (t_lab >= 31)  // slot 31 holds every label >= 31
+        ok = ok && ((P.g.lab[w] & kLabelMask) == t_lab);
+      // injectivity: only earlier positions with the same label can hold w
+      for (uint32_t same = t_same; same; same &= same - 1) ok = ok && w != F[__ffs(same) - 1][k];
+      if (bitmap) {
+        const uint32_t qv = (__shfl_sync(kFull, q_word, t) >> 21) & 15u;
+        ok = ok && ((bitmap[(size_t)qv * Q.col_len + (w >> 5)] >> (w & 31)) & 1u);
+      }
+      uint32_t r = 0;
+      for (uint32_t bits = t_bn; bits; bits &= bits - 1, ++r) {
+        if (!ok) continue;
+        const uint32_t j = __ffs(bits) - 1;
+        uint4 row;
+        if (r < kRows) {
+          row = rows[r][k];
+        } else {
+          const uint32_t x = F[j][k];
+          const uint32_t *o = P.g.loff + (size_t)x * (P.g.nlt + 1) + t_lab;
+          row = make_uint4(P.g.adj[x].x, o[0], o[1], P.g.lab[x] >> 31);
+        }
+        if (r != pv.z) {
+          ok = run_has(P.g.arena + (uint64_t)row.x * 4 + row.y, row.z - row.y, en);
+          alg += 4;
+        }
+        // liveness: only edges of a touched vertex can have changed, and of
+        // those the filter turns away all that the batch does not change
+        if (ok && row.w) {
+          const uint32_t x = F[j][k];
+          if (may_change(bt, x, w)) ok = edge_live(bt, x, w, tp);
+        }
+      }
+      const uint32_t m = __ballot_sync(kFull, ok);
+      const uint32_t ns = __popc(m);
+      work += ns;
+      ++hb;
+      ++dticks;
+      if (t == nq - 1) {
+        emit(m, w, t, k);
+      } else if (m && !(P.bfs_stop == t + 1 && write_rows(m, w, k))) {
+        if (ok) buf[t][cnt + __popc(m & lanemask_lt())] = w | (k << kIdBits);
+        cnt += ns;
+      }
+      if (P.work_limit && work >= work_left) {
+        if (publish_work()) break;
+      }
+      if (hb >= 64) {
+        hb = 0;
+        unsigned int err = 0;
+        if (lane == 0) {
+          atomicAdd(&P.sc->progress.v, 1ull);
+          err = ld_volatile(P.sc->error);
+        }
+        if (__shfl_sync(kFull, err, 0)) break;
+        if (P.work_limit && publish_work()) break;
+      }
+      if (P.donate && dticks >= 8) {
+        dticks = 0;
+        unsigned long long h = 0;
+        if (lane == 0) {
+          const unsigned long long pc = ld_volatile(P.sc->pop_cnt.v), pu = ld_volatile(P.sc->push_cnt.v);
+          h = pc > pu ? pc - pu : 0;
+        }
+        h = __shfl_sync(kFull, h, 0);
+        if (h > 0) {
+          const uint32_t split_min = P.split_min > 64 ? P.split_min : (P.split_min ? 64u : 128u);
+          const uint32_t dd = P.donate_depth ? min(P.donate_depth, 4u) : 2u;
+          park();  // so that every expansion reads alike
+          // the shallowest expansion with a substantial piece of work: waiting
+          // survivors with dd or more levels below them, partials not begun,
+          // or a long rest of one range
+          const uint32_t above = __shfl_down_sync(kFull, lv_n, 1) & 0xFFu;  // its survivors already descended into
+          const uint32_t wait = ((lv_n >> 8) & 0xFFu) - (lane < l ? above : 0u);
+          const bool has = lane + 1 >= depth && lane <= l &&
+                           ((wait && lane + 1 + dd < nq) ||
+                            ((lv_n >> 16) && lane + dd < nq) || lv_e >= lv_c + split_min);
+          const uint32_t hm = __ballot_sync(kFull, has);
+          if (hm) {
+            __syncwarp();  // the survivors in the buffers are visible to every lane
+            const uint32_t l0 = l, i = __ffs(hm) - 1;
+            const uint32_t wi = __shfl_sync(kFull, wait, i);
+            if (i != l) {
+              l = i;
+              nb = __shfl_sync(kFull, lv_n, i) & 0xFFu;
+              rebuild();
+              setup();
+            }
+            const uint32_t ci = __shfl_sync(kFull, lv_c, i), ei = __shfl_sync(kFull, lv_e, i);
+            uint32_t ni = (__shfl_sync(kFull, lv_n, i) >> 8) & 0xFFu, todo = __shfl_sync(kFull, lv_n, i) >> 16, ecut = ei;
+            // this lane's job, if any: column jk of F, image jw of position
+            // i + 1 (jdepth = i + 2) or a range of it
+            bool mine = false;
+            uint32_t jk = 0, jw = 0, jdepth = i + 1, jlo = 0, jhi = 0, jobs = 0;
+            if (wi && i + 1 + dd < nq) {
+              jobs = min(wi, (uint32_t)min(h, 32ull));
+              mine = lane < jobs;
+              const uint32_t x = mine ? buf[i + 1][ni - jobs + lane] : 0u;
+              jk = x >> kIdBits;
+              jw = x & kIdMask;
+              jdepth = i + 2;
+            } else {
+              const uint32_t excl = incl - len;
+              uint32_t um = i + dd < nq ? __ballot_sync(kFull, len && excl >= ci && excl < ei) : 0u;
+              if (um) {  // whole partials, the last ones
+                jobs = min((uint32_t)__popc(um), (uint32_t)min(h, 32ull));
+                for (uint32_t x = __popc(um); x > jobs; --x) um &= um - 1;
+                mine = (um >> lane) & 1u;
+                jk = lane;
+                if (incl > ei) {  // the last one without what was cut off before
+                  jlo = piv[lane].w;
+                  jhi = jlo + (ei - excl);
+                }
+                ecut = __shfl_sync(kFull, excl, __ffs(um) - 1);
+                todo -= jobs;
+              } else if (ei >= ci + split_min) {
+                // half of what is left, a job for each partial it reaches into
+                // (the last ones, when fewer warps wait)
+                uint32_t mid = ci + (((ei - ci) / 2 + 31) & ~31u);
+                um = __ballot_sync(kFull, len && incl > mid && excl < ei);
+                jobs = min((uint32_t)__popc(um), (uint32_t)min(h, 32ull));
+                for (uint32_t x = __popc(um); x > jobs; --x) um &= um - 1;
+                if (um) {
+                  mine = (um >> lane) & 1u;
+                  jk = lane;
+                  mid = max(mid, __shfl_sync(kFull, excl, __ffs(um) - 1));
+                  jlo = piv[lane].w + (max(excl, mid) - excl);
+                  jhi = piv[lane].w + (min(incl, ei) - excl);
+                  ecut = mid;
+                  todo = __popc(__ballot_sync(kFull, len && excl >= ci && excl < ecut));
+                }
+              }
+            }
+            unsigned long long s0 = 0;
+            uint32_t okr = 0;
+            const unsigned long long rmask = P.job_ring - 1;
+            if (lane == 0 && jobs) {
+              // jobs <= waiting warps, so positions stay within one warp's worth
+              // of reservations per donor of pop_cnt: the slot of position p
+              // was last used by position p - ring, consumed long ago; wait
+              // (bounded) until its consumer has released it
+              atomicAdd(&P.sc->outstanding.v, (unsigned long long)jobs);
+              s0 = atomicAdd(&P.sc->push_cnt.v, (unsigned long long)jobs);
+              atomicAdd(&P.sc->donations, (unsigned long long)jobs);
+              okr = 1;
+              const long long tw = clock64();
+              for (uint32_t x = 0; x < jobs && okr; ++x)
+                while (ld_volatile(P.job_seq[(s0 + x) & rmask]) != s0 + x) {
+                  if (clock64() - tw > P.timeout_cycles) {
+                    atomicOr(&P.sc->error, kErrTimeout);
+                    okr = 0;
+                    break;
+                  }
+                  __nanosleep(64);
+                }
+            }
+            okr = __shfl_sync(kFull, okr, 0);
+            s0 = __shfl_sync(kFull, s0, 0);
+            if (okr) {
+              const uint32_t mm = __ballot_sync(kFull, mine);
+              if (mine) {
+                const unsigned long long at = s0 + __popc(mm & lanemask_lt());
+                uint32_t *rec = reinterpret_cast<uint32_t *>(P.jobs + (at & rmask));
+                __stcg(rec, upd);
+                __stcg(rec + 1, qo);
+                __stcg(rec + 2, jdepth);
+                __stcg(rec + 3, jlo);
+                __stcg(rec + 4, jhi);
+                for (uint32_t j = 0; j <= i; ++j) __stcg(rec + 8 + j, F[j][jk]);
+                if (jdepth == i + 2) __stcg(rec + 9 + i, jw);
+                __threadfence();
+                atomicExch(&P.job_seq[at & rmask], at + 1);
+              }
+              if (jdepth == i + 2) ni -= jobs;
+              if (lane == i) {
+                lv_e = ecut;
+                lv_n = (lv_n & 0xFFu) | (ni << 8) | (todo << 16);
+              }
+            } else {
+              dticks = -8;  // nothing to give, or a failed wait
+            }
+            if (i != l0) {
+              l = l0;
+              nb = __shfl_sync(kFull, lv_n, l) & 0xFFu;
+              rebuild();
+              setup();
+            }
+            e = __shfl_sync(kFull, lv_e, l);
+            cnt = (__shfl_sync(kFull, lv_n, l) >> 8) & 0xFFu;
+          }
+        }
+      }
+      continue;
+    }
+    if (cnt) {  // descend: up to 32 survivors become the next batch
+      park();
+      __syncwarp();
+      nb = min(cnt, most);
+      const uint32_t x = buf[l + 1][lane < nb ? lane : 0];
+      for (uint32_t j = depth; j <= l; ++j) {
+        const uint32_t v = F[j][x >> kIdBits];
+        __syncwarp();
+        F[j][lane] = v;
+      }
+      ++l;
+      F[l][lane] = x & kIdMask;
+      __syncwarp();
+      c = 0;
+      cnt = 0;
+      e = setup();
+      continue;
+    }
+    if (l + 1 == depth) break;
+    // back to E(l - 1): its buffer without the batch just done
+    const uint32_t done = nb;
+    --l;
+    c = __shfl_sync(kFull, lv_c, l);
+    e = __shfl_sync(kFull, lv_e, l);
+    nb = __shfl_sync(kFull, lv_n, l);
+    cnt = ((nb >> 8) & 0xFFu) - done;
+    nb &= 0xFFu;
+    if (cnt || c < e) {
+      __syncwarp();
+      uint32_t y[2];
+#pragma unroll
+      for (uint32_t h = 0; h < 2; ++h) y[h] = lane + 32 * h < cnt ? buf[l + 1][done + lane + 32 * h] : 0u;
+      __syncwarp();
+#pragma unroll
+      for (uint32_t h = 0; h < 2; ++h)
+        if (lane + 32 * h < cnt) buf[l + 1][lane + 32 * h] = y[h];
+      rebuild();
+      if (c < e) setup();
+    }
+  }
+  flush();
+}
+
+// ---------------------------------------------------------------------------
+// Plain id-sorted runs (the allocation-free entry point: counts on a fixed
+// graph, no listing, no work limit, every edge live)
+// ---------------------------------------------------------------------------
+// One partial embedding at a time, the stack spread over the lanes: lane p
+// keeps the image f[p] of position p with its run, and the iteration state of
+// level p.  The level being scanned keeps its state in warp-uniform registers
+// (cur_*); one with deeper levels running parks it in its own lane (lv_*).
+__device__ void run_task_plain(const MatchArgs &P, uint32_t nupd, uint32_t upd, uint32_t qo, uint32_t depth,
+                               uint32_t lo, uint32_t hi, uint32_t fval) {
+  const uint32_t lane = threadIdx.x & 31;
+  const QDev &Q = P.qd[qo >> 8];
+  const uint32_t nq = Q.nq;
+  const OrderRec &R = P.orders[Q.order_base + (qo & 255)];
+  const uint32_t q_vert = lane < 16 ? R.vert[lane] : 0;
+  const uint32_t q_bn = lane < 16 ? R.bn[lane] : 0;
+  const uint32_t q_lab = Q.label[q_vert & 15];
+  const uint32_t seg = Q.local * nupd + upd;
+
+  uint32_t my_f = fval, my_off = 0, my_deg = 0;
+  if (lane < depth) {
+    uint2 a = P.g.adj[my_f];
+    my_off = a.x;
+    my_deg = a.y;
+  }
+  unsigned long long alg = 0, task_cnt = 0;  // warp-uniform
+
+  auto flush = [&]() {
     if (lane == 0) {
       if (task_cnt) {
         atomicAdd(&P.seg_count[seg], task_cnt);
@@ -238,14 +627,10 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   };
 
   if (depth >= nq) {  // a one-edge query: the seed is the embedding
-    emit(1u, 0, 0xFFFFFFFFu, 0xFFFFFFFFu, 0);
+    task_cnt = 1;
     flush();
     return;
   }
-  if (P.work_limit && publish_work()) return;  // a segment already over its limit
-
-  const uint32_t pack_max = kLM ? P.pack_max : 0u;
-  const uint32_t merge_max = kLM ? P.merge_max : 0u;
   // the current level (warp-uniform): its pivot run, next entry, end, pending
   // candidates of the last chunk, that chunk's first entry; its label and
   // backward neighbours
@@ -254,65 +639,27 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   // level `lane`, parked while deeper levels run
   uint32_t lv_pos = 0, lv_end = 0, lv_mask = 0, lv_chunk = 0;
 
-  // Level L scans the run of its pivot: the backward neighbour with the
-  // fewest candidates (label-major: entries with L's label; plain: degree).
-  // [rlo, rhi) narrows the scan for a donated range (rhi = 0: all of it).
+  // Level L scans the run of its pivot: the backward neighbour of the smallest
+  // degree.  [rlo, rhi) narrows the scan for a donated range (rhi = 0: all).
   auto setup_level = [&](uint32_t L, uint32_t rlo, uint32_t rhi) {
     cur_bn = __shfl_sync(kFull, q_bn, L);
     cur_want = __shfl_sync(kFull, q_lab, L);
     const bool inb = (cur_bn >> lane) & 1u;
-    uint32_t a = 0, b = my_deg;
-    if constexpr (kLM) {
-      b = 0;
-      if (inb && cur_want < P.g.nlt) {
-        const uint32_t *t = P.g.loff + (size_t)my_f * (P.g.nlt + 1) + cur_want;
-        a = t[0];
-        b = t[1];
-      }
-      // with packing, level nq - 2 also sets up the last level's ranges in
-      // the runs of the positions before it (fixed while level nq - 2 runs)
-      uint32_t fa = 0, fb = 0;
-      bool fx = false;
-      if (pack_max && L + 2 == nq) {
-        const uint32_t bnn = __shfl_sync(kFull, q_bn, L + 1);
-        const uint32_t wn = __shfl_sync(kFull, q_lab, L + 1);
-        fx = lane < L && ((bnn >> lane) & 1u);
-        if (fx && wn < P.g.nlt) {
-          const uint32_t *t = P.g.loff + (size_t)my_f * (P.g.nlt + 1) + wn;
-          fa = t[0];
-          fb = t[1];
-        }
-        alg += 8ull * __popc(bnn & ((1u << L) - 1));
-      }
-      __syncwarp();  // lanes may still read these levels' previous ranges
-      if (inb) srng[L][lane] = make_uint2(a, b);
-      if (fx) srng[L + 1][lane] = make_uint2(fa, fb);
-      if (pack_max && L + 2 == nq && lane == 0) stg->info = kStageUnset;  // a new context
-      __syncwarp();
-      alg += 8ull * __popc(cur_bn);
-    }
-    const uint32_t key = inb ? ((min(b - a, 0x3FFFFFFu) << 5) | lane) : 0xFFFFFFFFu;
+    const uint32_t key = inb ? ((min(my_deg, 0x3FFFFFFu) << 5) | lane) : 0xFFFFFFFFu;
     cur_pivot = __reduce_min_sync(kFull, key) & 31;
     cur_base = __shfl_sync(kFull, my_off, cur_pivot);
-    const uint32_t pa = __shfl_sync(kFull, a, cur_pivot), pb = __shfl_sync(kFull, b, cur_pivot);
-    cur_pos = rhi ? rlo : pa;
-    cur_end = rhi ? min(rhi, pb) : pb;
+    const uint32_t end = __shfl_sync(kFull, my_deg, cur_pivot);
+    cur_pos = rhi ? rlo : 0;
+    cur_end = rhi ? min(rhi, end) : end;
     cur_mask = 0;
     cur_chunk = 0;
   };
 
-  // The pivot of a level whose ranges are staged (label-major) or whose
-  // backward neighbours' degrees are at hand (plain): the same choice
-  // setup_level made, recomputed instead of parked.
+  // The same choice, recomputed instead of parked.
   auto pivot_of = [&](uint32_t L) -> uint32_t {
     const uint32_t bnL = __shfl_sync(kFull, q_bn, L);
     const bool inb = (bnL >> lane) & 1u;
-    uint32_t len = my_deg;
-    if constexpr (kLM) {
-      const uint2 r = inb ? srng[L][lane] : make_uint2(0, 0);
-      len = r.y - r.x;
-    }
-    const uint32_t key = inb ? ((min(len, 0x3FFFFFFu) << 5) | lane) : 0xFFFFFFFFu;
+    const uint32_t key = inb ? ((min(my_deg, 0x3FFFFFFu) << 5) | lane) : 0xFFFFFFFFu;
     return __reduce_min_sync(kFull, key) & 31;
   };
   auto pivot_base = [&](uint32_t L) -> uint32_t { return __shfl_sync(kFull, my_off, pivot_of(L)); };
@@ -322,193 +669,6 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   };
 
   uint32_t hb = 0;  // chunks since the last heartbeat
-
-  // The packed last level over the candidates m of level L = nq - 2 (lane k:
-  // candidate cw).  False: more than pack_max entries (or
-  // one range longer than that), nothing done.
-  auto pack_last = [&](uint32_t L, uint32_t m, uint32_t cw) -> bool {
-    const uint32_t LL = L + 1;
-    const uint32_t bnn = __shfl_sync(kFull, q_bn, LL);
-    const uint32_t wn = __shfl_sync(kFull, q_lab, LL);
-    const bool dep = (bnn >> L) & 1u;  // the last level reads the candidate's own run
-    const uint32_t fixed = bnn & ~(1u << L);
-    uint2 fr = make_uint2(0, 0);
-    uint32_t fkey = 0xFFFFFFFFu;
-    if ((fixed >> lane) & 1u) {
-      fr = srng[LL][lane];
-      fkey = (min(fr.y - fr.x, 0x3FFFFFFu) << 5) | lane;
-    }
-    const uint32_t fmin = __reduce_min_sync(kFull, fkey);
-    const uint32_t fj = fmin & 31;  // the shortest fixed range (none: fmin = ~0)
-    const uint32_t f_off = __shfl_sync(kFull, my_off, fj);
-    const uint32_t f_a = __shfl_sync(kFull, fr.x, fj);
-    const uint32_t f_b = __shfl_sync(kFull, fr.y, fj);
-    const uint32_t f_len = fmin == 0xFFFFFFFFu ? 0xFFFFFFFFu : f_b - f_a;
-    const bool cand = (m >> lane) & 1u;
-    uint32_t o_off = 0, o_a = 0, o_b = 0;
-    if (cand && dep && wn < P.g.nlt) {
-      o_off = P.g.adj[cw].x;
-      const uint32_t *t = P.g.loff + (size_t)cw * (P.g.nlt + 1) + wn;
-      o_a = t[0];
-      o_b = t[1];
-    }
-    const bool own = dep && (o_b - o_a) < f_len;
-    const uint32_t len = cand ? (own ? o_b - o_a : f_len) : 0u;
-    if (__any_sync(kFull, len > pack_max)) return false;
-    uint32_t incl = len;
-#pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
-      const uint32_t t = __shfl_up_sync(kFull, incl, d);
-      if (lane >= d) incl += t;
-    }
-    const uint32_t total = __shfl_sync(kFull, incl, 31);
-    if (total > pack_max) return false;
-    if (dep) alg += 8ull * __popc(m);
-    // candidate k's entry, read by the lanes whose entries fall in its range
-    __syncwarp();  // the previous pass's lanes may still read the table
-    spk[lane] = PackEnt{incl - len, cw, o_off, o_a, o_b, own ? 1u : 0u, 0u, 0u};
-    uint32_t sinfo = stg->info;
-    __syncwarp();
-    if (sinfo == kStageUnset) {  // first pass of this context: stage the longest fixed range
-      const uint32_t lkey = ((fixed >> lane) & 1u) ? ((min(fr.y - fr.x, 0x3FFFFFFu) << 5) | lane) : 0u;
-      const uint32_t lmax = __reduce_max_sync(kFull, lkey);
-      const uint32_t slen = lmax >> 5, sj = lmax & 31;
-      sinfo = kStageNone;
-      if (slen >= kStageMin) {
-        uint32_t shift = 0;
-        while ((slen >> shift) > kStage) ++shift;
-        const uint32_t nf = (slen + (1u << shift) - 1) >> shift;
-        const uint32_t *src = P.g.arena + (uint64_t)__shfl_sync(kFull, my_off, sj) * 4 + __shfl_sync(kFull, fr.x, sj);
-        for (uint32_t i = lane; i < nf; i += 32) stg->fence[i] = src[(size_t)i << shift];
-        alg += 4ull * nf;
-        sinfo = sj | (shift << 5) | (nf << 10);
-      }
-      if (lane == 0) stg->info = sinfo;
-      __syncwarp();
-    }
-    const uint32_t st_j = sinfo < kStageNone ? (sinfo & 31) : 32u;
-    const uint32_t same = __ballot_sync(kFull, lane < L && q_lab == wn);
-    const bool sameP = cur_want == wn;
-    const uint32_t qvn = __shfl_sync(kFull, q_vert, LL);
-    // backward neighbours whose edges may not be live (the candidates' own
-    // marks are not read: the filter answers for them)
-    const uint32_t touched = bnn & (__ballot_sync(kFull, my_touch) | (1u << L));
-    for (uint32_t base = 0; base < total; base += 32) {
-      const uint32_t t = base + lane;
-      bool ok = t < total;
-      // the candidate whose range holds entry t: the first lane with incl > t
-      uint32_t k = 0;
-#pragma unroll
-      for (uint32_t s = 16; s; s >>= 1) {
-        const uint32_t v = __shfl_sync(kFull, incl, k + s - 1);
-        if (v <= t) k += s;
-      }
-      const PackEnt pe = spk[k];
-      const uint32_t kx = pe.excl, kc = pe.cw, ko = pe.off, ka = pe.a, kb = pe.b;
-      const bool kown = pe.own;
-      const uint64_t start = kown ? (uint64_t)ko * 4 + ka : (uint64_t)f_off * 4 + f_a;
-      const uint32_t e = ok ? P.g.arena[start + (t - kx)] : 0u;
-      const uint32_t w = e & kIdMask;
-      if (wn >= 31)  // slot 31 holds every label >= 31
-        ok = ok && ((P.g.lab[w] & kLabelMask) == wn);
-      for (uint32_t sm = same; sm; sm &= sm - 1) {
-        const uint32_t fjv = __shfl_sync(kFull, my_f, __ffs(sm) - 1);
-        ok = ok && (w != fjv);
-      }
-      if (sameP) ok = ok && (w != kc);
-      if (bitmap) ok = ok && ((bitmap[(size_t)qvn * col_len + (w >> 5)] >> (w & 31)) & 1u);
-      uint32_t probes = 0;
-      for (uint32_t bits = bnn; bits; bits &= bits - 1) {
-        const uint32_t j = __ffs(bits) - 1;
-        const uint32_t oj = __shfl_sync(kFull, my_off, j);
-        const bool piv = kown ? (j == L) : (j == fj);
-        if (ok && !piv) {
-          uint32_t ra, rb;
-          const uint32_t *lst;
-          if (j == L) {
-            lst = P.g.arena + (uint64_t)ko * 4;
-            ra = ka;
-            rb = kb;
-          } else {
-            const uint2 r = srng[LL][j];
-            lst = P.g.arena + (uint64_t)oj * 4;
-            ra = r.x;
-            rb = r.y;
-          }
-          if (j == st_j) {
-            // fences in shared memory: lo = first fence >= e; a miss there
-            // leaves the window between fences lo - 1 and lo in global memory
-            const uint32_t shift = (sinfo >> 5) & 31, nf = sinfo >> 10;
-            const uint32_t lo = lower_bound_u32(stg->fence, nf, e);
-            if (lo < nf && stg->fence[lo] == e) {
-              ok = true;
-            } else if (lo == 0 || shift == 0) {
-              ok = false;
-            } else {
-              const uint32_t wa = ra + ((lo - 1) << shift) + 1, wb = min(ra + (lo << shift), rb);
-              const uint32_t p = wa + lower_bound_u32(lst + wa, wb - wa, e);
-              ok = p < wb && lst[p] == e;
-            }
-          } else {
-            const uint32_t p = ra + lower_bound_u32(lst + ra, rb - ra, e);
-            ok = p < rb && lst[p] == e;
-          }
-          ++probes;
-        }
-      }
-      for (uint32_t bits = touched; bits; bits &= bits - 1) {
-        const uint32_t j = __ffs(bits) - 1;
-        uint32_t fjv = __shfl_sync(kFull, my_f, j);
-        if (j == L) fjv = kc;
-        if (ok && may_change(bt, fjv, w)) ok = edge_live(bt, fjv, w, tp);
-      }
-      const uint32_t m2 = __ballot_sync(kFull, ok);
-      work += __popc(m2);
-      alg += 4ull * min(32u, total - base) + 4ull * __reduce_add_sync(kFull, probes);
-      emit(m2, w, LL, L, kc);
-      ++hb;
-    }
-    return true;
-  };
-
-  // Breadth-first rows: the candidates m of level L (lane k: cw) become
-  // rows of L + 1 fixed positions.  One reservation per chunk, all or
-  // nothing (a bounded compare-and-swap loop); false: no room, nothing
-  // written.
-  auto write_rows = [&](uint32_t L, uint32_t m, uint32_t cw) -> bool {
-    const uint32_t cnt = __popc(m);
-    unsigned long long base = ~0ull;
-    if (lane == 0) {
-      unsigned long long cur = ld_volatile(*P.rows_cnt);
-      for (int tries = 0; tries < 64 && cur + cnt <= P.rows_cap; ++tries) {
-        const unsigned long long prev = atomicCAS(P.rows_cnt, cur, cur + cnt);
-        if (prev == cur) {
-          base = cur;
-          break;
-        }
-        cur = prev;
-      }
-    }
-    base = __shfl_sync(kFull, base, 0);
-    if (base == ~0ull) return false;
-    const uint32_t fsrc = __shfl_sync(kFull, my_f, (lane - 8) & 31);
-    uint32_t bits = m;
-    for (uint32_t r = 0; r < cnt; ++r) {
-      const uint32_t b = __ffs(bits) - 1;
-      bits &= bits - 1;
-      const uint32_t cb = __shfl_sync(kFull, cw, b);
-      uint32_t word = 0;
-      if (lane == 0) word = upd;
-      else if (lane == 1) word = qo;
-      else if (lane == 2) word = L + 1;
-      else if (lane >= 8 && lane < 24) {
-        const uint32_t fi = lane - 8;
-        word = fi < L ? fsrc : (fi == L ? cb : 0u);
-      }
-      __stcg(reinterpret_cast<uint32_t *>(P.rows_out + base + r) + lane, word);
-    }
-    return true;
-  };
 
   uint32_t L = depth;
   setup_level(L, lo, hi);
@@ -531,19 +691,13 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
       const uint32_t *run = P.g.arena + (uint64_t)cur_base * 4;
       const uint32_t i = pos + lane;
       bool ok = i < end;
-      const uint32_t e = ok ? run[i] : 0;  // entry (label-major) or id
-      const uint32_t w = kLM ? (e & kIdMask) : e;
+      const uint32_t w = ok ? run[i] : 0;
       const uint32_t want = cur_want;
-      // plain runs hold every label; slot 31 holds every label >= 31
-      if (!kLM || want >= 31) ok = ok && ((P.g.lab[w] & kLabelMask) == want);
+      ok = ok && ((P.g.lab[w] & kLabelMask) == want);
       // injectivity: only earlier positions with the same label can hold w
       for (uint32_t same = __ballot_sync(kFull, lane < L && q_lab == want); same; same &= same - 1) {
         const uint32_t fj = __shfl_sync(kFull, my_f, __ffs(same) - 1);
         ok = ok && (w != fj);
-      }
-      if (bitmap) {
-        const uint32_t qv = __shfl_sync(kFull, q_vert, L);
-        ok = ok && ((bitmap[(size_t)qv * col_len + (w >> 5)] >> (w & 31)) & 1u);
       }
       const uint32_t bnL = cur_bn;
       uint32_t others = bnL & ~(1u << cur_pivot);
@@ -551,68 +705,22 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
       while (others) {
         uint32_t j = __ffs(others) - 1;
         others &= others - 1;
-        const uint32_t oj = __shfl_sync(kFull, my_off, j);
-        if constexpr (kLM) {
-          const uint2 r = srng[L][j];
+        const uint32_t oj = __shfl_sync(kFull, my_off, j), dj = __shfl_sync(kFull, my_deg, j);
+        if (ok) {
           const uint32_t *lst = P.g.arena + (uint64_t)oj * 4;
-          const uint32_t nb = r.y - r.x;
-          if (nb <= merge_max) {
-            // merge: the chunk's entries (ascending across lanes) against
-            // the range in 32-entry tiles, each lane placing its entry in a
-            // tile by a five-step shuffle search; stops at the first tile
-            // that reaches the chunk's largest live entry
-            const uint32_t emax = __reduce_max_sync(kFull, ok ? e : 0u);
-            bool found = false;
-            for (uint32_t t = 0; t < nb; t += 32) {
-              const uint32_t bv = t + lane < nb ? lst[r.x + t + lane] : 0xFFFFFFFFu;
-              uint32_t k = 0;
-#pragma unroll
-              for (uint32_t sh = 16; sh; sh >>= 1)
-                if (__shfl_sync(kFull, bv, k + sh - 1) < e) k += sh;
-              const uint32_t at = __shfl_sync(kFull, bv, k);  // every lane shuffles
-              const uint32_t last = __shfl_sync(kFull, bv, 31);
-              if (at == e && t + k < nb) found = true;
-              if (last >= emax) break;
-            }
-            probes += ok ? 1u : 0u;
-            ok = ok && found;
-          } else if (ok) {
-            const uint32_t p = r.x + lower_bound_u32(lst + r.x, nb, e);
-            ok = p < r.y && lst[p] == e;
-            ++probes;
-          }
-        } else {
-          const uint32_t dj = __shfl_sync(kFull, my_deg, j);
-          if (ok) {
-            const uint32_t *lst = P.g.arena + (uint64_t)oj * 4;
-            uint32_t p = lower_bound_u32(lst, dj, w);
-            ok = p < dj && lst[p] == w;
-            ++probes;
-          }
+          const uint32_t p = lower_bound_u32(lst, dj, w);
+          ok = p < dj && lst[p] == w;
+          ++probes;
         }
       }
-      // liveness: only edges of a touched vertex can have changed, and of
-      // those the filter turns away all that the batch does not change
-      for (uint32_t bits = bnL & __ballot_sync(kFull, my_touch); bits; bits &= bits - 1) {
-        const uint32_t fj = __shfl_sync(kFull, my_f, __ffs(bits) - 1);
-        if (ok && may_change(bt, fj, w)) ok = edge_live(bt, fj, w, tp);
-      }
       const uint32_t m = __ballot_sync(kFull, ok);
-      work += __popc(m);
-      alg += (kLM ? 4ull : 8ull) * min(32u, end - pos) + 4ull * __reduce_add_sync(kFull, probes);
+      alg += 8ull * min(32u, end - pos) + 4ull * __reduce_add_sync(kFull, probes);
       cur_pos = pos + 32;
       cur_chunk = pos;
       ++hb;
       ++dticks;
-      if (L == nq - 1) {
-        emit(m, w, L, 0xFFFFFFFFu, 0);
-      } else if (kLM && pack_max && L + 2 == nq && m) {
-        if (!pack_last(L, m, w)) cur_mask = m;
-      } else if (P.bfs_stop == L + 1 && m) {
-        if (!write_rows(L, m, w)) cur_mask = m;
-      } else {
-        cur_mask = m;
-      }
+      if (L == nq - 1) task_cnt += __popc(m);
+      else cur_mask = m;
 
       if (hb >= 64) {
         hb = 0;
@@ -622,7 +730,6 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
           err = ld_volatile(P.sc->error);
         }
         if (__shfl_sync(kFull, err, 0)) break;
-        if (P.work_limit && publish_work()) break;
       }
       if (P.donate && dticks >= 8) {
         dticks = 0;
@@ -689,7 +796,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
             okr = __shfl_sync(kFull, okr, 0);
             s0 = __shfl_sync(kFull, s0, 0);
             if (okr) {
-              // level p's pivot run (its ranges are still staged)
+              // level p's pivot run 
               const uint32_t pbase = pivot_base(p);
               const uint32_t pchunk = __shfl_sync(kFull, lv_chunk, p);
               const uint32_t fsrc = __shfl_sync(kFull, my_f, (lane - 8) & 31);
@@ -701,7 +808,6 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
                   uint32_t b = __ffs(bits) - 1;
                   bits &= bits - 1;
                   cw = P.g.arena[(uint64_t)pbase * 4 + pchunk + b];
-                  if constexpr (kLM) cw &= kIdMask;
                   jdepth = p + 1;
                 } else {
                   jdepth = p;
@@ -739,8 +845,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
     }
     // descend into the lowest pending candidate of level L
     const uint32_t b = __ffs(cur_mask) - 1;
-    uint32_t w = P.g.arena[(uint64_t)cur_base * 4 + cur_chunk + b];
-    if constexpr (kLM) w &= kIdMask;
+    const uint32_t w = P.g.arena[(uint64_t)cur_base * 4 + cur_chunk + b];
     cur_mask &= cur_mask - 1;
     if (lane == L) {
       lv_pos = cur_pos;
@@ -751,13 +856,13 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
       uint2 a = P.g.adj[w];
       my_off = a.x;
       my_deg = a.y;
-      my_touch = P.g.lab[w] >> 31;
     }
     ++L;
     setup_level(L, 0, 0);
   }
   flush();
 }
+
 
 // phantom = 1 adds one outstanding task that nothing finishes (a test of the
 // bounded waits: the launch then ends only through their timeouts).
@@ -777,21 +882,18 @@ __global__ void k_sched_init(Sched *sc, const BatchHdr *hdr, unsigned long long 
   }
 }
 
-// kMinBlocks: resident blocks per SM the register allocation is sized for
-// (5: 48 registers a thread; 4: 64).  Launches of 5 or more blocks per SM
-// take the first, fewer the second.
-template <bool kLM, int kMinBlocks>
-__global__ void __launch_bounds__(256, kMinBlocks) k_match(MatchArgs P) {
-  __shared__ uint2 s_rng[kLM ? 8 : 1][16][16];
-  __shared__ PackEnt s_pack[kLM ? 8 : 1][32];
-  __shared__ PackStage s_stage[kLM ? 8 : 1];
+// kLM: label-major runs with slot offsets (the engine's graph); otherwise
+// plain id-sorted runs.
+template <bool kLM>
+__global__ void __launch_bounds__(256, kLM ? 4 : 5) k_match(MatchArgs P) {
+  extern __shared__ __align__(16) uint32_t smem[];
   const uint32_t lane = threadIdx.x & 31;
   if (*P.abort_flag & kErrArena) return;  // the batch was refused before its insert
   // an earlier launch of this batch failed (one read, the same for the warp:
   // the word can change while the kernel runs)
   if (__shfl_sync(kFull, lane == 0 ? ld_volatile(P.sc->error) : 0u, 0)) return;
   const uint32_t nupd = P.hdr->n;
-  const DevBatchEdges bt{P.bt.bkey, P.bt.binfo, P.bt.bloom, P.hdr->m, P.hdr->bloom_mask};
+  const DevBatchEdges bt{P.bt.bkey, P.bt.binfo, P.bt.bloom, P.bt.table, P.hdr->m, P.hdr->bloom_mask};
   bool seeds_done = false;
   while (true) {
     uint32_t kind = 0;
@@ -828,8 +930,10 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_match(MatchArgs P) {
       hi = __shfl_sync(kFull, word, 4);
       fval = __shfl_sync(kFull, word, (lane + 8) & 31);
     }
-    run_task<kLM>(P, bt, nupd, upd, qo, depth, lo, hi, fval, s_rng[kLM ? (threadIdx.x >> 5) : 0],
-                  s_pack[kLM ? (threadIdx.x >> 5) : 0], &s_stage[kLM ? (threadIdx.x >> 5) : 0]);
+    if constexpr (kLM)
+      run_task(P, bt, nupd, upd, qo, depth, lo, hi, fval, smem + (threadIdx.x >> 5) * warp_words(P.W));
+    else
+      run_task_plain(P, nupd, upd, qo, depth, lo, hi, fval);
     finish_task(P);
   }
 }
@@ -856,20 +960,25 @@ void launch_sched_init(Sched *sc, const BatchHdr *hdr, unsigned long long *job_s
 }
 
 void launch_match(const MatchArgs &a, int blocks, cudaStream_t s) {
-  int dev = 0, sms = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const bool wide = blocks < 5 * std::max(sms, 1);  // fewer than 5 blocks per SM: 64 registers
-  if (!a.g.loff) k_match<false, 5><<<blocks, 256, 0, s>>>(a);
-  else if (wide) k_match<true, 4><<<blocks, 256, 0, s>>>(a);
-  else k_match<true, 5><<<blocks, 256, 0, s>>>(a);
+  if (!a.g.loff) {
+    k_match<false><<<blocks, 256, 0, s>>>(a);
+    return;
+  }
+  const int smem = 8 * 4 * (int)warp_words(a.W);
+  cudaFuncSetAttribute(k_match<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  k_match<true><<<blocks, 256, smem, s>>>(a);
 }
 
-int match_max_blocks_per_sm() {
-  int n = 0, m = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_match<true, 5>, 256, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_match<false, 5>, 256, 0);
-  return n < m ? n : m;
+int match_max_blocks_per_sm(uint32_t width) {
+  int n = 0;
+  if (!width) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_match<false>, 256, 0);
+    return n;
+  }
+  const int smem = 8 * 4 * (int)warp_words(width);
+  cudaFuncSetAttribute(k_match<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_match<true>, 256, smem);
+  return n;
 }
 
 }  // namespace dsm

@@ -175,7 +175,7 @@ extern "C" int dsm_count_edge_embeddings_noalloc(int device, uint32_t nv, const 
   MatchArgs ma;
   std::memset(&ma, 0, sizeof(ma));
   ma.g = g;
-  ma.bt = DevBatchEdges{nullptr, nullptr, nullptr, 0, 0};  // a fixed graph: every edge is live
+  ma.bt = DevBatchEdges{nullptr, nullptr, nullptr, nullptr, 0, 0};  // a fixed graph: every edge is live
   ma.vtp = vtp;
   ma.hdr = dh;
   ma.abort_flag = (const unsigned int *)(base + kOffHdr + sizeof(BatchHdr));
@@ -192,7 +192,7 @@ extern "C" int dsm_count_edge_embeddings_noalloc(int device, uint32_t nv, const 
   ma.list = 0;
   ma.donate = 1;
   ma.timeout_cycles = 5000ll * (long long)(clk_khz > 0 ? clk_khz : 1965000);
-  int per_sm = std::max(1, std::min(match_max_blocks_per_sm(), 4));
+  int per_sm = std::max(1, std::min(match_max_blocks_per_sm(0), 4));
   launch_match(ma, std::max(sms, 1) * per_sm, s);
   if (cudaGetLastError() != cudaSuccess) return cuda_failed();
 

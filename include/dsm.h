@@ -76,14 +76,12 @@ const char *dsm_last_error(dsm_engine *e);
                                    this many levels below them (0 = default 2; 1..4) */
 #define DSM_OPT_AUTOTUNE 13     /* 1: the next batch times its matcher launch under each
                                    candidate setting on its own union graph -- first the
-                                   plan (DSM_OPT_BFS_LEVELS in {0, 1, 2}), then the
-                                   intersection tile (DSM_OPT_PACK_MAX in {0, 256, 1024,
-                                   4096} x DSM_OPT_MERGE_MAX in {0, 64, 256}), then resident
+                                   plan (DSM_OPT_BFS_LEVELS in {0, 1, 2}), then the batch
+                                   (DSM_OPT_PACK_MAX 0 or its setting), then resident
                                    blocks per SM x split threshold x donation depth -- and
                                    keeps the fastest in DSM_OPT_BFS_LEVELS /
-                                   DSM_OPT_PACK_MAX / DSM_OPT_MERGE_MAX /
-                                   DSM_OPT_WARPS_PER_SM / DSM_OPT_SPLIT_MIN /
-                                   DSM_OPT_DONATE_DEPTH; its results
+                                   DSM_OPT_PACK_MAX / DSM_OPT_WARPS_PER_SM /
+                                   DSM_OPT_SPLIT_MIN / DSM_OPT_DONATE_DEPTH; its results
                                    are those of any setting.  Reads 1 until that batch ran. */
 #define DSM_OPT_GRAPH 14        /* 1: each batch's two device segments (uploads .. matcher, and
                                    deletes .. downloads) are captured into CUDA graphs and
@@ -120,11 +118,11 @@ const char *dsm_last_error(dsm_engine *e);
                                    updates, falling back to every vertex when that region
                                    is large or the query's state is not the previous
                                    batch's; 0: every vertex, every batch.  Same bitmaps. */
-#define DSM_OPT_MERGE_MAX 21     /* matcher set intersection: a backward neighbour's label range
-                                   of at most this many entries is intersected with a whole
-                                   32-entry chunk by a ballot/shuffle merge over 32-entry tiles
-                                   instead of a binary search per entry (default 64; 0: always
-                                   searched; at most 4096).  Results do not depend on it. */
+#define DSM_OPT_MERGE_MAX 21     /* 0..4096 (default 64): accepted and kept for callers that set
+                                   it.  It bounded the probe ranges that a chunk of one
+                                   partial embedding intersected by merging; chunks now mix
+                                   partial embeddings and search every probe range.  Results
+                                   do not depend on it. */
 #define DSM_OPT_BFS_LEVELS 22    /* matcher plan: 0 (default) depth-first from the seeds; k in 1..8:
                                    the first launch expands every seed breadth-first to
                                    prefixes of 2 + k query vertices, written as rows (while
@@ -135,12 +133,10 @@ const char *dsm_last_error(dsm_engine *e);
                                    depend on it; DSM_OPT_AUTOTUNE tries 0, 1 and 2. */
 #define DSM_OPT_BFS_ROWS 23      /* row table capacity for DSM_OPT_BFS_LEVELS (default 2^20
                                    rows of 128 bytes) */
-#define DSM_OPT_PACK_MAX 19     /* matcher intersection tile: the candidates one 32-entry
-                                   chunk leaves at the second-to-last query vertex have
-                                   their last-level ranges laid end to end and scanned
-                                   together when they total at most this many entries
-                                   (default 1024; 0: each candidate scanned on its own;
-                                   at most 2^20).  Results do not depend on it. */
+#define DSM_OPT_PACK_MAX 19     /* matcher batches: 0: partial embeddings are expanded one at a
+                                   time; 1..2^20 (default 1024): up to 32 together, their
+                                   candidate ranges laid end to end.  Results do not depend
+                                   on it. */
 int dsm_engine_set_option(dsm_engine *e, int option, int64_t value);
 int dsm_engine_get_option(dsm_engine *e, int option, int64_t *value);
 

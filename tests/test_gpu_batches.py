@@ -1,0 +1,108 @@
+"""The matcher's batches of partial embeddings (match.cu): levels that leave
+around 31, 32, 33, 63, 64, 65 and many survivors, queries whose vertices have
+more backward neighbours than the stored ranges (cliques up to 7 vertices) and
+the widest query (16 vertices), donated pieces of every kind (long ranges,
+many partials, waiting survivors), each listed and counted.  All results are
+whole numbers and must equal the oracle's."""
+import numpy as np
+import pytest
+
+import dsm_b200 as d
+from tests.helpers import oracle_stream
+
+pytestmark = pytest.mark.gpu
+
+
+def _layers(m, r, seed):
+    """Vertex 0 (label 0) joins a hub (label 1) of m middles (label 2), each
+    with r leaves (label 3); half of the leaves also neighbour the hub."""
+    rng = np.random.default_rng(seed)
+    labels, edges = [0, 1], []
+    for _ in range(m):
+        mid = len(labels)
+        labels.append(2)
+        edges.append((1, mid))
+        for _ in range(r):
+            edges.append((mid, len(labels)))
+            if rng.random() < 0.5:
+                edges.append((1, len(labels)))
+            labels.append(3)
+    perm = rng.permutation(len(labels))
+    out = np.zeros(len(labels), np.uint32)
+    out[perm] = labels
+    e = perm[np.array(edges, np.int64)].astype(np.uint32)
+    return len(labels), out, e, np.array([[1, perm[0], perm[1], 0], [0, perm[0], perm[1], 0]], np.uint32)
+
+
+PATH = d.Query.from_edges([0, 1, 2, 3], [(0, 1), (1, 2), (2, 3)])
+CLOSED = d.Query.from_edges([0, 1, 2, 3], [(0, 1), (1, 2), (2, 3), (1, 3)])
+TWO = d.Query.from_edges([0, 1, 2, 3, 2], [(0, 1), (1, 2), (2, 3), (1, 4)])
+
+
+def _check(nv, labels, edges, batches, queries, listed, **opts):
+    e = d.Engine(0)
+    e.set_option(d.OPT_LIST, listed)
+    for k, v in opts.items():
+        e.set_option(getattr(d, k), v)
+    e.load_graph_edges(nv, labels, edges)
+    ids = [e.register(q) for q in queries]
+    sts = [oracle_stream(nv, labels, edges, q) for q in queries]
+    total = 0
+    for b in batches:
+        r = e.run_batch(b)
+        for qid, st in zip(ids, sts):
+            s, c, t = st.apply(b, listed=bool(listed))
+            assert np.array_equal(r.signs, s)
+            assert np.array_equal(r.counts[r.query_index(qid)], c)
+            total += int(c.sum())
+            for i in range(len(b) if listed else 0):
+                assert np.array_equal(r.tuples_of(qid, i), t[i])
+    stats = e.stats()
+    e.close()
+    return total, stats
+
+
+@pytest.mark.parametrize("listed", [0, 1])
+@pytest.mark.parametrize("m,r", [(1, 1), (1, 33), (31, 1), (32, 2), (33, 1), (63, 3), (64, 1), (65, 2), (7, 40), (200, 9)])
+def test_levels_around_a_batch(m, r, listed):
+    nv, labels, edges, ups = _layers(m, r, m * 100 + r)
+    for opts in ({}, {"OPT_PACK_MAX": 0}, {"OPT_BFS_LEVELS": 1}, {"OPT_BFS_LEVELS": 2, "OPT_BFS_ROWS": 64}):
+        total, _ = _check(nv, labels, edges, [ups], [PATH, CLOSED, TWO], listed, **opts)
+        assert total > 0
+
+
+@pytest.mark.parametrize("nq", [3, 4, 5, 6, 7])
+def test_cliques_have_more_backward_neighbours_than_stored_ranges(nq):
+    rng = np.random.default_rng(nq)
+    nv = 26
+    pairs = [(a, b) for a in range(nv) for b in range(a)]
+    edges = np.array([p for p in pairs if rng.random() < 0.6], np.uint32)
+    labels = (rng.random(nv) < 0.3).astype(np.uint32)
+    q = d.Query.from_edges(labels[:nq], [(a, b) for a in range(nq) for b in range(a)])
+    pick = rng.choice(len(pairs), 40)
+    ups = np.array([[rng.integers(2), *pairs[k], 0] for k in pick], np.uint32)
+    total, _ = _check(nv, labels, edges, [ups, ups[::-1].copy()], [q], 1)
+    assert total > 0 or nq == 7
+
+
+def test_sixteen_vertices():
+    """Paths and cycles of 16 vertices around a ring with chords."""
+    nv = 40
+    edges = [(k, (k + 1) % nv) for k in range(nv)] + [(k, k + 7) for k in range(0, nv - 7, 5)]
+    labels = np.array([k % 4 for k in range(nv)], np.uint32)
+    path = d.Query.from_edges([k % 4 for k in range(16)], [(k, k + 1) for k in range(15)])
+    cycle = d.Query.from_edges([k % 4 for k in range(16)], [(k, (k + 1) % 16) for k in range(16)])
+    ups = np.array([[0, 3, 4, 0], [1, 4, 3, 0], [1, 0, 15, 0], [0, 10, 11, 0], [1, 10, 11, 0], [1, 21, 36, 0]], np.uint32)
+    total, _ = _check(nv, labels, np.array(edges, np.uint32), [ups], [path, cycle], 1)
+    assert total > 0
+
+
+@pytest.mark.parametrize("split,dd", [(0, 0), (64, 1), (512, 4)])
+@pytest.mark.parametrize("m,r", [(3, 4000), (900, 12), (2500, 1)])
+def test_donated_pieces(m, r, split, dd):
+    """One update feeds every warp: a few long ranges, many partials, one
+    range of many short ones."""
+    nv, labels, edges, ups = _layers(m, r, 5)
+    total, s = _check(nv, labels, edges, [ups], [PATH, CLOSED, TWO], 0, OPT_SPLIT_MIN=split, OPT_DONATE_DEPTH=dd)
+    assert total > 0 and s["donations"] > 0
+    _check(nv, labels, edges, [ups], [PATH, CLOSED, TWO], 0, OPT_DONATE=0)
