@@ -158,9 +158,9 @@ int Engine::launch_front(Staged &S) {
       (rc = dalloc(d_dkey, dd * 8)) || (rc = dalloc(d_dhead, (dd + 1) * 4)) || (rc = dalloc(d_dsel, dd * 4)) ||
       (rc = dalloc(d_segcnt, S.nseg * 8)) || (rc = dalloc(d_qlisted, std::max<size_t>(S.nq_live, 1) * 8)))
     return rc;
-  uint32_t bloom_words = 64;
-  while (bloom_words < m) bloom_words *= 2;
-  if ((rc = dalloc(d_bloom, (size_t)bloom_words * 4)) || (rc = dalloc(d_etable, (size_t)bloom_words * 8))) return rc;
+  size_t bloom_words = 64;
+  while (bloom_words < 4ull * m) bloom_words *= 2;
+  if ((rc = dalloc(d_bloom, bloom_words * 4)) || (rc = dalloc(d_etable, bloom_words * 2))) return rc;
   S.work_limit = S.match ? work_limit : 0;
   if (S.work_limit && (rc = dalloc(d_segwork, S.nseg * 8))) return rc;
   if (S.match && (rc = dalloc(d_seeds, S.seed_cap * 16))) return rc;
@@ -200,7 +200,7 @@ int Engine::launch_front(Staged &S) {
   hd.nq_live = S.nq_live;
   hd.seed_cap = S.seed_cap;
   hd.nseg = (unsigned long long)S.nq_live * n;
-  hd.bloom_mask = bloom_words - 1;
+  hd.bloom_mask = (uint32_t)(bloom_words - 1);
   hd.pad = 0;
 
   // uploads (plain copies from the slot's pinned staging)
@@ -236,7 +236,8 @@ int Engine::launch_front(Staged &S) {
   std::memset(&ma, 0, sizeof(ma));
   ma.g = g;
   ma.bt = DevBatchEdges{(const unsigned long long *)d_bkey.ptr, (const uint32_t *)d_binfo.ptr,
-                        (const uint32_t *)d_bloom.ptr, (const uint32_t *)d_etable.ptr, 0, 0};
+                        (const uint32_t *)d_bloom.ptr, (const uint32_t *)d_etable.ptr,
+                        (const unsigned long long *)d_dkey.ptr, 0, 0};
   ma.hdr = dh;
   ma.vtp = (const uint32_t *)d_vtp.ptr;
   ma.qd = (const QDev *)d_qd.ptr;
@@ -546,7 +547,8 @@ int Engine::finish_device(Staged &S) {
       std::memset(&ma, 0, sizeof(ma));
       ma.g = g;
       ma.bt = DevBatchEdges{(const unsigned long long *)d_bkey.ptr, (const uint32_t *)d_binfo.ptr,
-                        (const uint32_t *)d_bloom.ptr, (const uint32_t *)d_etable.ptr, 0, 0};
+                        (const uint32_t *)d_bloom.ptr, (const uint32_t *)d_etable.ptr,
+                        (const unsigned long long *)d_dkey.ptr, 0, 0};
       ma.hdr = dh;
       ma.vtp = (const uint32_t *)d_vtp.ptr;
       ma.qd = (const QDev *)d_qd.ptr;

@@ -54,10 +54,11 @@ __device__ __forceinline__ const uint32_t *adj_list(const DevGraph &g, uint2 a) 
 // Sorted edge table of the batch, for "is edge {x,y} live after the first
 // `tp` updates of the batch".  bkey: canonical keys (min << 32 | max) sorted,
 // ties in update order; binfo: update index | op << 30 | initially-present << 31.
-// bloom: a filter over the keys the batch changes, three bits of one word per
-// key (bloom_mask + 1 words, a power of two >= the keys: at most three of a
-// word's 32 bits on average, so one load turns away all but about one in a
-// thousand of the edges the batch does not change).  Without it every
+// bloom: a filter over the keys the batch changes and over (endpoint, label
+// slot of the other end) of each, three bits of one word per key (bloom_mask + 1
+// words, a power of two >= 4 n: at most nine bits of four words, so one load
+// turns away all but about one in a thousand of the edges the batch does not
+// change).  Without it every
 // candidate marked as an update's endpoint (on power-law graphs most of a
 // large batch's candidates) was searched for in bkey, 12 to 16 dependent
 // loads, after a gather of its label word for the mark.  Matcher time of one
@@ -65,12 +66,14 @@ __device__ __forceinline__ const uint32_t *adj_list(const DevGraph &g, uint2 a) 
 // 2^22-edge graph 63 -> 53 ms, 256 queries x 1021 updates on a 2^22-edge
 // power-law graph 85 -> 76 ms, three queries x 4096 updates 6.7 -> 4.4 ms.
 // table: where a changed key's entries start in bkey (index + 1; 0: empty),
-// hashed with linear probing, 2 (bloom_mask + 1) slots: at most half full.
+// hashed with linear probing, (bloom_mask + 1) / 2 slots: at most half full.
+// dkey: both directions (x << 32 | entry of y) sorted, 2 n keys.
 struct DevBatchEdges {
   const unsigned long long *bkey;
   const uint32_t *binfo;
   const uint32_t *bloom;
   const uint32_t *table;
+  const unsigned long long *dkey;
   uint32_t n;           // keys (set by the matcher from the batch header)
   uint32_t bloom_mask;  // (set by the matcher from the batch header)
 };
@@ -86,7 +89,9 @@ __device__ __forceinline__ uint32_t bloom_bits(uint32_t x, uint32_t y, uint32_t 
   word = (g * 0xC2B2AE35u >> 5) & mask;
   return (1u << (g & 31)) | (1u << ((g >> 5) & 31)) | (1u << ((g >> 10) & 31));
 }
-// False: the batch does not change edge {x, y}.
+// Stands for "some neighbour with this label slot" beside vertex ids (< 2^27).
+__device__ __forceinline__ uint32_t slot_key(uint32_t slot) { return 0xF0000000u | slot; }
+// False: the batch does not change edge {x, y} (y may be a slot_key).
 __device__ __forceinline__ bool may_change(const DevBatchEdges &t, uint32_t x, uint32_t y) {
   uint32_t word;
   const uint32_t bits = bloom_bits(x, y, t.bloom_mask, word);
@@ -105,7 +110,7 @@ __device__ __forceinline__ uint32_t table_slot(unsigned long long key, uint32_t 
 // a 32,768-update batch, and two of five chunks of a hub-heavy graph had one.
 __device__ __forceinline__ bool edge_live(const DevBatchEdges &t, uint32_t x, uint32_t y, uint32_t tp) {
   const unsigned long long key = canon_key(x, y);
-  const uint32_t mask = 2 * t.bloom_mask + 1;
+  const uint32_t mask = t.bloom_mask >> 1;
   uint32_t lo = 0, s = table_slot(key, mask);
   while (true) {
     const uint32_t at = t.table[s];
@@ -124,6 +129,26 @@ __device__ __forceinline__ bool edge_live(const DevBatchEdges &t, uint32_t x, ui
     live = (inf >> 30) & 1u;
   }
   return live;
+}
+
+// Entries of x's run with label slot `slot` whose edge is not live after the
+// first `tp` updates: of the batch's edges at x, those it changes (the run
+// holds the union graph, so each is in it) and that are not live then.
+__device__ __forceinline__ uint32_t dead_entries(const DevBatchEdges &t, uint32_t x, uint32_t slot, uint32_t tp) {
+  const unsigned long long first = ((unsigned long long)x << 32) | ((unsigned long long)slot << kIdBits);
+  uint32_t lo = 0, hi = 2 * t.n;
+  while (lo < hi) {
+    uint32_t mid = (lo + hi) >> 1;
+    if (t.dkey[mid] < first) lo = mid + 1; else hi = mid;
+  }
+  uint32_t dead = 0;
+  for (unsigned long long prev = ~0ull; lo < 2 * t.n; ++lo) {
+    const unsigned long long k = t.dkey[lo];
+    if ((k >> kIdBits) != (first >> kIdBits)) break;
+    if (k != prev) dead += !edge_live(t, x, (uint32_t)k & kIdMask, tp);
+    prev = k;
+  }
+  return dead;
 }
 
 // lower_bound over a sorted run

@@ -62,10 +62,15 @@ __global__ void k_edge_state(EdgeStateArgs A) {
     atomicOr(&A.g.lab[a], kTouchBit);
     atomicOr(&A.g.lab[b], kTouchBit);
     uint32_t word;
-    const uint32_t bits = bloom_bits(a, b, A.hdr->bloom_mask, word);
+    const uint32_t bmask = A.hdr->bloom_mask;
+    uint32_t bits = bloom_bits(a, b, bmask, word);
+    atomicOr(&A.bloom[word], bits);
+    bits = bloom_bits(a, slot_key(label_slot(A.g.lab[b] & kLabelMask)), bmask, word);
+    atomicOr(&A.bloom[word], bits);
+    bits = bloom_bits(b, slot_key(label_slot(A.g.lab[a] & kLabelMask)), bmask, word);
     atomicOr(&A.bloom[word], bits);
     // at most half of the slots are ever taken, so a free one is found
-    const uint32_t mask = 2 * A.hdr->bloom_mask + 1;
+    const uint32_t mask = bmask >> 1;
     for (uint32_t sl = table_slot(key, mask); atomicCAS(&A.table[sl], 0u, j + 1) != 0u; sl = (sl + 1) & mask) {
     }
   }
@@ -385,7 +390,7 @@ __global__ void k_batch_clear(ClearArgs A) {
   for (size_t i = t; i < sizeof(Sched) / 4; i += stride) sc[i] = 0;
   for (size_t i = t; i < 64; i += stride) A.misc[i] = 0;
   for (size_t i = t; i <= h.bloom_mask; i += stride) A.bloom[i] = 0;
-  for (size_t i = t; i <= 2ull * h.bloom_mask + 1; i += stride) A.table[i] = 0;
+  for (size_t i = t; i <= h.bloom_mask >> 1; i += stride) A.table[i] = 0;
 }
 
 // ---------------------------------------------------------------------------

@@ -175,7 +175,7 @@ extern "C" int dsm_count_edge_embeddings_noalloc(int device, uint32_t nv, const 
   MatchArgs ma;
   std::memset(&ma, 0, sizeof(ma));
   ma.g = g;
-  ma.bt = DevBatchEdges{nullptr, nullptr, nullptr, nullptr, 0, 0};  // a fixed graph: every edge is live
+  ma.bt = DevBatchEdges{};  // a fixed graph: every edge is live
   ma.vtp = vtp;
   ma.hdr = dh;
   ma.abort_flag = (const unsigned int *)(base + kOffHdr + sizeof(BatchHdr));

@@ -106,3 +106,49 @@ def test_donated_pieces(m, r, split, dd):
     total, s = _check(nv, labels, edges, [ups], [PATH, CLOSED, TWO], 0, OPT_SPLIT_MIN=split, OPT_DONATE_DEPTH=dd)
     assert total > 0 and s["donations"] > 0
     _check(nv, labels, edges, [ups], [PATH, CLOSED, TWO], 0, OPT_DONATE=0)
+
+
+@pytest.mark.parametrize("nlab", [1, 2])
+@pytest.mark.parametrize("limit", [0, 300, 5000])
+@pytest.mark.parametrize("listed", [0, 1])
+def test_leaves_counted_without_a_scan(nlab, limit, listed):
+    """Leaves on hubs of 700 neighbours: their ranges are counted, not read
+    (with a listing, once the query is over its budget).  The batch toggles
+    the hubs' edges, so ranges hold entries that are not live, and with one or
+    two labels they hold images of earlier vertices."""
+    rng = np.random.default_rng(nlab * 7 + limit)
+    nv = 1600
+    edges = {(0, 1)}
+    for h, deg in ((0, 700), (1, 650)):
+        edges |= {(h, int(w)) for w in rng.choice(np.arange(2, nv), deg, replace=False)}
+    while len(edges) < 1700:
+        a, b = sorted(int(x) for x in rng.integers(2, nv, 2))
+        if a != b:
+            edges.add((a, b))
+    edges = np.array(sorted(edges), np.uint32)
+    labels = rng.integers(0, nlab, nv).astype(np.uint32)
+    pairs = edges[rng.choice(np.nonzero(edges[:, 0] < 2)[0], 24)].tolist() + [[0, 1]]
+    pairs += [[int(rng.integers(2)), int(w)] for w in rng.integers(2, nv, 6)]
+    ups = np.array([[rng.integers(2), *pairs[rng.integers(len(pairs))], 0] for _ in range(70)], np.uint32)
+    shapes = [(3, [(0, 1), (1, 2)]), (4, [(0, 1), (1, 2), (2, 3)]), (4, [(0, 1), (1, 2), (0, 2), (0, 3)])]
+    queries = [d.Query.from_edges(rng.integers(0, nlab, n), es) for n, es in shapes]
+    e = d.Engine(0)
+    e.set_option(d.OPT_LIST, listed)
+    e.set_option(d.OPT_WORK_LIMIT, limit)
+    e.set_option(d.OPT_QUERY_LIST_LIMIT, 500 if listed else 0)
+    e.load_graph_edges(nv, labels, edges)
+    ids = [e.register(q) for q in queries]
+    for b in (ups, ups[::-1].copy()):
+        r = e.run_batch(b)
+        for k, (qid, q) in enumerate(zip(ids, queries)):
+            st = oracle_stream(nv, labels, edges, q)
+            st.set_work_limit(limit)
+            if b is not ups:
+                st.apply_graph(ups)
+            s, c, t = st.apply(b, listed=False)
+            got, over = r.counts[r.query_index(qid)], (c & d.INCOMPLETE) != 0
+            assert np.array_equal((got & d.INCOMPLETE) != 0, over)
+            assert np.array_equal(got[~over], c[~over])
+            if listed and not over.any():
+                assert r.query_listed[r.query_index(qid)] == (int(c.sum()) <= 500)
+    e.close()
