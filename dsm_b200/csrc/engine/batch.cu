@@ -74,6 +74,7 @@ int Engine::prepare(const dsm_update *ups, uint32_t n, Staged &S, int slot) {
   for (uint32_t i = 0; i < n; ++i) {
     const uint32_t a = ups[i].src, b = ups[i].dst;
     if (a == b) continue;
+    S.inserts += ups[i].op != 0;
     und.push_back({a < b ? ((uint64_t)a << 32) | b : ((uint64_t)b << 32) | a, i});
   }
   std::sort(und.begin(), und.end());
@@ -177,6 +178,12 @@ int Engine::launch_front(Staged &S) {
     S.placed = !dalloc(d_segoff, (S.nseg + 1) * 8) && !dalloc(d_segcur, S.nseg * 4) &&
                !dalloc(d_segchunk, (S.nseg + 1) * 4) && !dalloc(d_listsum, 3 * kListBlocks * 8);
   }
+  // the edge filter anew once it holds as many deleted edges as words, or has
+  // outgrown them (a pass over the runs per as many updates)
+  if (flt_words && (flt_removed > flt_words || flt_added > 2 * flt_words))
+    if ((rc = build_edge_filter(flt_edges + flt_added))) return rc;
+  flt_added += S.inserts;
+  flt_removed += m - S.inserts;
   // what allocates, synchronises or copies pageable memory runs before the
   // segments, so that each segment can be captured into a CUDA graph
   if (!(S.match && filter_mode > 0) && d_rinfo.ptr && n)  // the graph changes unfiltered

@@ -45,6 +45,8 @@ struct DevGraph {
   uint32_t nlt;
   uint64_t arena_words;
   unsigned long long *arena_top;  // next free 16-byte unit
+  uint32_t *flt;       // edge filter (see may_have), or null
+  uint32_t flt_mask;   // its words, less one
 };
 
 __device__ __forceinline__ const uint32_t *adj_list(const DevGraph &g, uint2 a) {
@@ -89,6 +91,15 @@ __device__ __forceinline__ uint32_t bloom_bits(uint32_t x, uint32_t y, uint32_t 
   word = (g * 0xC2B2AE35u >> 5) & mask;
   return (1u << (g & 31)) | (1u << ((g >> 5) & 31)) | (1u << ((g >> 10) & 31));
 }
+// The edge filter of the whole graph: three bits of one word per edge, a word
+// per one to two edges.  False: {x, y} is not an edge.  Deleted edges leave
+// their bits (the engine builds the filter anew once they are many).
+__device__ __forceinline__ bool may_have(const DevGraph &g, uint32_t x, uint32_t y) {
+  uint32_t word;
+  const uint32_t bits = bloom_bits(x, y, g.flt_mask, word);
+  return (g.flt[word] & bits) == bits;
+}
+
 // Stands for "some neighbour with this label slot" beside vertex ids (< 2^27).
 __device__ __forceinline__ uint32_t slot_key(uint32_t slot) { return 0xF0000000u | slot; }
 // False: the batch does not change edge {x, y} (y may be a slot_key).

@@ -128,7 +128,7 @@ Engine::~Engine() {
 }
 
 std::vector<DevBuf *> Engine::all_dev_bufs() {
-  std::vector<DevBuf *> v = {&d_lab, &d_adj, &d_cap, &d_arena, &d_arena_top, &d_loff, &d_qd, &d_orders,
+  std::vector<DevBuf *> v = {&d_lab, &d_adj, &d_cap, &d_arena, &d_arena_top, &d_loff, &d_flt, &d_qd, &d_orders,
                              &d_pair_off, &d_pair_ent, &d_upd, &d_bkey, &d_bidx, &d_binfo, &d_gflag,
                              &d_vtp, &d_dkey, &d_dhead, &d_dsel, &d_seeds, &d_sched, &d_jobs,
                              &d_job_seq, &d_out_seg, &d_out_tup, &d_segcnt, &d_misc, &d_hdr, &d_qlisted, &d_segwork,
@@ -256,7 +256,27 @@ int Engine::load_graph(uint32_t nv_, const uint32_t *labels, std::vector<uint64_
   graph_loaded = true;
   label_host.assign(labels, labels + nv_);
   for (auto &q : slots) q.filter_dirty = true;
-  return region_init();
+  if (int r = region_init()) return r;
+  return build_edge_filter(keys.size());
+}
+
+// The matcher's edge filter from the graph on the device (`edges`: at least as
+// many as it has): a word per one to two edges (a power of two, 2^27 at most).
+// Without room for it the matcher searches every run.
+int Engine::build_edge_filter(uint64_t edges) {
+  uint64_t words = 1024;
+  while (words * 2 < edges && words < (1ull << 27)) words *= 2;
+  flt_words = 0;
+  if (dalloc(d_flt, words * 4)) return DSM_OK;
+  flt_words = words;
+  flt_edges = edges;
+  flt_added = flt_removed = 0;
+  CK(cudaMemsetAsync(d_flt.ptr, 0, words * 4, stream));
+  launch_edge_filter(dev_graph(), num_sms * 8, stream);
+  ++stats.kernel_launches;
+  CK(cudaGetLastError());
+  ++query_gen;  // captured graphs hold the old filter
+  return DSM_OK;
 }
 
 // The incremental filter's region buffers for a new graph: marks cleared,
@@ -303,6 +323,8 @@ DevGraph Engine::dev_graph() {
   g.nlt = nlt;
   g.arena_words = arena_words;
   g.arena_top = (unsigned long long *)d_arena_top.ptr;
+  g.flt = flt_words ? (uint32_t *)d_flt.ptr : nullptr;
+  g.flt_mask = flt_words ? (uint32_t)(flt_words - 1) : 0u;
   return g;
 }
 

@@ -63,6 +63,7 @@ struct HostOut {
 struct Staged {
   const dsm_update *ups = nullptr;  // the caller's updates, valid until assemble
   uint32_t n = 0, m = 0, ngroups = 0;
+  uint32_t inserts = 0;  // of the m
   size_t ndir = 0;
   size_t o_up = 0, o_bk = 0, o_bi = 0, o_dk = 0, o_dh = 0;  // offsets in the staging buffer
   int slot = 0;
@@ -215,6 +216,11 @@ struct Engine {
   uint32_t nlt = 0;  // label slots in use (slot offsets per vertex: nlt + 1)
   std::vector<uint32_t> label_host;
   DevBuf d_lab, d_adj, d_cap, d_arena, d_arena_top, d_loff;
+  // edge filter of the matcher: words in use (0: none), edges it was built
+  // with, inserts and deletes since
+  DevBuf d_flt;
+  uint64_t flt_words = 0, flt_edges = 0, flt_added = 0, flt_removed = 0;
+  int build_edge_filter(uint64_t edges);
   // incremental filter region (filter.cuh RegionInfo)
   DevBuf d_rinfo, d_rmark, d_rlist, d_rprev;
   uint64_t region_batches = 0;  // filtered batches since the region buffers were set up

@@ -55,7 +55,14 @@ __global__ void k_edge_state(EdgeStateArgs A) {
     state = op;
   }
   uint8_t flag = 0;
-  if (!init && inserted) flag |= 1;             // must join the union graph now
+  if (!init && inserted) {
+    flag |= 1;  // must join the union graph now
+    if (A.g.flt) {
+      uint32_t word;
+      const uint32_t bits = bloom_bits(a, b, A.g.flt_mask, word);
+      atomicOr(&A.g.flt[word], bits);
+    }
+  }
   if (!state && (init || inserted)) flag |= 2;  // must leave it after matching
   for (uint32_t k = j; k < e; ++k) A.gflag[k] = flag;
   if (any_change) {
@@ -377,6 +384,22 @@ __global__ void k_arena_move(DevGraph g, const uint2 *nadj, uint32_t *narena) {
   }
 }
 
+__global__ void k_edge_filter(DevGraph g) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < g.nv; v += warps) {
+    const uint2 a = g.adj[v];
+    const uint32_t *run = adj_list(g, a);
+    for (uint32_t i = lane; i < a.y; i += 32) {
+      const uint32_t w = run[i] & kIdMask;
+      if (w < v) continue;  // each edge once
+      uint32_t word;
+      const uint32_t bits = bloom_bits(v, w, g.flt_mask, word);
+      atomicOr(&g.flt[word], bits);
+    }
+  }
+}
+
 __global__ void k_batch_clear(ClearArgs A) {
   const BatchHdr h = *A.hdr;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -445,6 +468,8 @@ void launch_arena_check(const AdjUpdateArgs &a, int blocks, cudaStream_t s) {
 void launch_arena_move(DevGraph g, const uint2 *nadj, uint32_t *narena, int blocks, cudaStream_t s) {
   k_arena_move<<<blocks, 256, 0, s>>>(g, nadj, narena);
 }
+
+void launch_edge_filter(DevGraph g, int blocks, cudaStream_t s) { k_edge_filter<<<blocks, 256, 0, s>>>(g); }
 
 void launch_adj_insert(const AdjUpdateArgs &a, int blocks, cudaStream_t s) {
   k_adj_insert<<<blocks, 256, 0, s>>>(a);

@@ -76,6 +76,8 @@ void launch_adj_insert(const AdjUpdateArgs &a, int blocks, cudaStream_t s);
 // Compaction: copies every run to its new place (nadj: {start in 16-byte
 // units, degree} per vertex) in another arena.
 void launch_arena_move(DevGraph g, const uint2 *nadj, uint32_t *narena, int blocks, cudaStream_t s);
+// The graph's edge filter (g.flt, cleared before) from its runs.
+void launch_edge_filter(DevGraph g, int blocks, cudaStream_t s);
 void launch_adj_delete(const AdjUpdateArgs &a, int blocks, cudaStream_t s);
 void launch_clear_touch(DevGraph g, const BatchHdr *hdr, const uint4 *upd, int blocks, cudaStream_t s);
 

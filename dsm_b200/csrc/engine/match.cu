@@ -130,12 +130,22 @@ __device__ void finish_task(const MatchArgs &P) {
 // three queries x 4096 updates on a 2^24-edge one 86 -> 46 ms; one request of
 // 512 updates against 64 queries 5.5 -> 2.6 ms.
 //
+// A level with several backward neighbours is scanned in two steps.  The
+// graph's edge filter answers for the neighbours beside the pivot in one load
+// each, where a search of a run takes 8 to 14 dependent ones, and most entries
+// are turned away (on a 2^24-edge power-law graph 27 of 32): those that pass
+// are gathered, and 32 of them searched together.  Three queries x 4096
+// updates on that graph 44 -> 31 ms, 256 queries x 1021 updates 34 -> 27 ms;
+// where most entries pass (a hub-heavy graph with 8 labels) it neither gains
+// nor costs (15 ms).
+//
 // Shared memory of a warp (W = widest query): the batch's images F[W][32]
 // (column k: the partial of lane k), up to kRows ranges per partial, the pivot
-// per partial, and a buffer of 64 survivors per level (id | parent << 27).
+// per partial, 64 candidates (position in the ranges, id | owner << 27), and a
+// buffer of 64 survivors per level (id | parent << 27).
 constexpr uint32_t kRows = 3;  // backward neighbours with stored ranges; further ones are read when needed
 __host__ __device__ constexpr uint32_t warp_words(uint32_t W) {
-  return W * 32 + kRows * 128 + 128 + (W > 3 ? W - 3 : 1) * 64;
+  return W * 32 + kRows * 128 + 128 + 128 + (W > 3 ? W - 3 : 1) * 64;
 }
 
 __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t nupd, uint32_t upd, uint32_t qo,
@@ -144,7 +154,8 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   uint32_t(*const F)[32] = reinterpret_cast<uint32_t(*)[32]>(sm);
   uint4(*const rows)[32] = reinterpret_cast<uint4(*)[32]>(sm + P.W * 32);
   uint4 *const piv = reinterpret_cast<uint4 *>(sm + P.W * 32 + kRows * 128);
-  uint32_t(*const buf)[64] = reinterpret_cast<uint32_t(*)[64]>(sm + P.W * 32 + kRows * 128 + 128) - 2;  // from level 2
+  uint2 *const cand = reinterpret_cast<uint2 *>(sm + P.W * 32 + kRows * 128 + 128);
+  uint32_t(*const buf)[64] = reinterpret_cast<uint32_t(*)[64]>(sm + P.W * 32 + kRows * 128 + 256) - 2;  // from level 2
   const QDev &Q = P.qd[qo >> 8];
   const uint32_t nq = Q.nq;
   const OrderRec &R = P.orders[Q.order_base + (qo & 255)];
@@ -387,21 +398,53 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   }
   uint32_t hb = 0;     // chunks since the last heartbeat
   int32_t dticks = 0;  // chunks since the last donation check (below zero: none for a while)
+  uint32_t nc = 0;  // candidates that passed the edge filter
   while (true) {
-    if (c < e && cnt < most) {
-      const uint32_t t = l + 1, pos = c + lane;
-      bool ok = pos < e;
-      uint32_t k = 0;  // the owner: the first lane with incl > pos
+    if (cnt < most && (c < e || nc)) {
+      const uint32_t t = l + 1;
+      const bool two = P.g.flt && (t_bn & (t_bn - 1));
+      bool ok = false, test = true;
+      uint32_t k = 0, w = 0;
+      if (!two || (nc < 32 && c < e)) {  // a chunk of the ranges
+        const uint32_t pos = c + lane;
+        ok = pos < e;
 #pragma unroll
-      for (uint32_t d = 16; d; d >>= 1) {
-        const uint32_t v = __shfl_sync(kFull, incl, k + d - 1);
-        if (v <= pos) k += d;
+        for (uint32_t d = 16; d; d >>= 1) {  // the owner: the first lane with incl > pos
+          const uint32_t v = __shfl_sync(kFull, incl, k + d - 1);
+          if (v <= pos) k += d;
+        }
+        const uint4 pv = piv[k];
+        if (ok) {
+          w = P.g.arena[((uint64_t)pv.y << 32 | pv.x) + pos] & kIdMask;
+          alg += 4;
+        }
+        c = min(c + 32, e);
+        if (two) {
+          uint32_t r = 0;
+          for (uint32_t bits = t_bn; bits; bits &= bits - 1, ++r)
+            if (ok && r != pv.z) {
+              ok = may_have(P.g, F[__ffs(bits) - 1][k], w);
+              alg += 4;
+            }
+          const uint32_t m = __ballot_sync(kFull, ok);
+          if (ok) cand[nc + __popc(m & lanemask_lt())] = make_uint2(pos, w | (k << kIdBits));
+          nc += __popc(m);
+          test = nc >= 32 || c >= e;
+          __syncwarp();
+        }
       }
-      const uint4 pv = piv[k];
-      const uint32_t en = ok ? P.g.arena[((uint64_t)pv.y << 32 | pv.x) + pos] : 0u;
-      const uint32_t w = en & kIdMask;
-      if (ok) alg += 4;
-      c = min(c + 32, e);
+      if (two && test) {  // up to 32 of those that passed
+        const uint32_t n = min(nc, 32u);
+        const uint2 x = cand[lane], y = cand[32 + lane];
+        __syncwarp();
+        if (32 + lane < nc) cand[lane] = y;
+        ok = lane < n;
+        w = x.y & kIdMask;
+        k = ok ? x.y >> kIdBits : 0u;
+        nc -= n;
+      }
+      const uint32_t en = (t_lab << kIdBits) | w;
+      ok = ok && test;
       if (t_lab >= 31)  // slot 31 holds every label >= 31
         ok = ok && ((P.g.lab[w] & kLabelMask) == t_lab);
       // injectivity: only earlier positions with the same label can hold w
@@ -422,7 +465,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
           const uint32_t *o = P.g.loff + (size_t)x * (P.g.nlt + 1) + t_lab;
           row = make_uint4(P.g.adj[x].x, o[0], o[1], P.g.lab[x] >> 31);
         }
-        if (r != pv.z) {
+        if (r != piv[k].z) {
           ok = run_has(P.g.arena + (uint64_t)row.x * 4 + row.y, row.z - row.y, en);
           alg += 4;
         }
@@ -596,6 +639,10 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
       continue;
     }
     if (cnt) {  // descend: up to 32 survivors become the next batch
+      if (nc) {  // candidates not tested yet are read again
+        c = cand[0].x;
+        nc = 0;
+      }
       park();
       __syncwarp();
       nb = min(cnt, most);

@@ -152,3 +152,53 @@ def test_leaves_counted_without_a_scan(nlab, limit, listed):
             if listed and not over.any():
                 assert r.query_listed[r.query_index(qid)] == (int(c.sum()) <= 500)
     e.close()
+
+
+def _dense(nv, m, seed):
+    rng = np.random.default_rng(seed)
+    edges = set()
+    while len(edges) < m:
+        a, b = sorted(int(x) for x in rng.integers(0, nv, 2))
+        if a != b:
+            edges.add((a, b))
+    return rng, np.array(sorted(edges), np.uint32), rng.integers(0, 3, nv).astype(np.uint32)
+
+
+def test_edge_filter_is_built_anew():
+    """More deletes, then more inserts, than the edge filter's words: it is
+    built anew between batches, grows, and every batch equals the oracle."""
+    rng, edges, labels = _dense(300, 4000, 3)
+    q = [d.Query.from_edges(labels[:4], [(0, 1), (1, 2), (2, 3), (0, 3), (0, 2)]),
+         d.Query.from_edges(labels[4:7], [(0, 1), (1, 2), (0, 2)])]
+    batches = []
+    for k in range(6):
+        op = k % 2
+        pick = edges[rng.permutation(len(edges))[:3000]] if k < 4 else rng.integers(0, 300, (3000, 2))
+        batches.append(np.concatenate([np.full((3000, 1), op), pick, np.zeros((3000, 1))], 1).astype(np.uint32))
+    batches[4][:, 0] = 1  # a random graph on top, denser than the one loaded
+    total, _ = _check(300, labels, edges, batches, q, 0)
+    assert total > 0
+
+
+def test_without_room_for_the_edge_filter():
+    """An engine whose budget ends before the filter searches every run."""
+    rng, edges, labels = _dense(300, 4000, 4)
+    q = d.Query.from_edges(labels[:4], [(0, 1), (1, 2), (2, 3), (0, 3), (0, 2)])
+    e = d.Engine(0)
+    e.load_graph_edges(300, labels, edges)
+    full = e.stats()["device_bytes_in_use"]
+    e.close()
+    pick = edges[rng.permutation(len(edges))[:200]]
+    ups = np.concatenate([np.zeros((200, 1)), pick, np.zeros((200, 1))], 1).astype(np.uint32)
+    want = oracle_stream(300, labels, edges, q).apply(ups)
+    for budget in (full - 1, 0):
+        e = d.Engine(0, budget)
+        e.load_graph_edges(300, labels, edges)
+        assert (e.stats()["device_bytes_in_use"] < full) == (budget > 0)
+        e.set_option(d.OPT_MEM_BUDGET, 8 << 30)
+        qid = e.register(q)
+        r = e.run_batch(ups)
+        assert np.array_equal(r.counts[0], want[1])
+        for i in range(len(ups)):
+            assert np.array_equal(r.tuples_of(qid, i), want[2][i])
+        e.close()
