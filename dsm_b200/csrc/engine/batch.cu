@@ -95,12 +95,13 @@ int Engine::prepare(const dsm_update *ups, uint32_t n, Staged &S, int slot) {
   S.ndir = dir.size();
   const size_t up_bytes = (size_t)n * 16, bk_bytes = (size_t)S.m * 8, bi_bytes = (size_t)S.m * 4,
                dk_bytes = dir.size() * 8, dh_bytes = dhead.size() * 4;
-  S.o_up = 0;
-  S.o_bk = up_bytes;
+  S.o_up = kHdrBytes;  // behind the header, written at launch
+  S.o_bk = S.o_up + up_bytes;
   S.o_bi = S.o_bk + bk_bytes;
   S.o_dk = (S.o_bi + bi_bytes + 7) & ~(size_t)7;
   S.o_dh = S.o_dk + dk_bytes;
-  if (int rc = halloc(H.stage, S.o_dh + dh_bytes + 64)) return rc;
+  S.stage_bytes = S.o_dh + dh_bytes;
+  if (int rc = halloc(H.stage, S.stage_bytes)) return rc;
   char *st = (char *)H.stage.ptr;
   std::memcpy(st + S.o_up, ups, up_bytes);
   for (uint32_t j = 0; j < S.m; ++j) {
@@ -128,12 +129,29 @@ int Engine::seg_a_kernels(Staged &S, const ClearArgs &ca, const EdgeStateArgs &e
   if (S.match) {
     if (int r = launch_filters()) return r;  // per query, on the union graph
     if (seeds) {
-      launch_seeds(sa, blocks, stream);
-      launch_sched_init((Sched *)d_sched.ptr, (const BatchHdr *)d_hdr.ptr, (unsigned long long *)d_job_seq.ptr,
-                        job_ring, stream, stall_test);
-      stats.kernel_launches += 2;
+      launch_seeds(sa, blocks, stream);  // its last block arms the scheduler
+      ++stats.kernel_launches;
     }
   }
+  return DSM_OK;
+}
+
+// The scheduler, the error block and the listing counters lie in one piece,
+// so that one copy reads them back (d_misc and d_qlisted are views of d_sched,
+// h_qlisted of h_sched).
+int Engine::sched_block(uint32_t nq) {
+  const size_t bytes = sizeof(Sched) + kMiscBytes + std::max<size_t>(nq, 1) * 8;
+  if (int rc = dalloc(d_sched, bytes)) return rc;
+  if (int rc = halloc(h_sched, bytes)) return rc;
+  d_misc.ptr = (char *)d_sched.ptr + sizeof(Sched);
+  d_qlisted.ptr = (char *)d_misc.ptr + kMiscBytes;
+  h_qlisted.ptr = (char *)h_sched.ptr + sizeof(Sched) + kMiscBytes;
+  return DSM_OK;
+}
+
+int Engine::read_sched(uint32_t nq) {
+  CK(cudaMemcpyAsync(h_sched.ptr, d_sched.ptr, sizeof(Sched) + kMiscBytes + (size_t)nq * 8, cudaMemcpyDeviceToHost,
+                     stream));
   return DSM_OK;
 }
 
@@ -157,7 +175,8 @@ int Engine::launch_front(Staged &S) {
   if ((rc = dalloc(d_upd, nn * 16)) || (rc = dalloc(d_bkey, mm * 8)) || (rc = dalloc(d_bidx, mm * 4)) ||
       (rc = dalloc(d_binfo, mm * 4)) || (rc = dalloc(d_gflag, mm)) || (rc = dalloc(d_vtp, nn * 4)) ||
       (rc = dalloc(d_dkey, dd * 8)) || (rc = dalloc(d_dhead, (dd + 1) * 4)) || (rc = dalloc(d_dsel, dd * 4)) ||
-      (rc = dalloc(d_segcnt, S.nseg * 8)) || (rc = dalloc(d_qlisted, std::max<size_t>(S.nq_live, 1) * 8)))
+      (rc = dalloc(d_segcnt, S.nseg * 8)) || (rc = sched_block(S.nq_live)) || (rc = dalloc(d_stage, S.stage_bytes)) ||
+      (rc = dalloc(d_pack, 64 + kPackBytes)))
     return rc;
   size_t bloom_words = 64;
   while (bloom_words < 4ull * m) bloom_words *= 2;
@@ -191,16 +210,17 @@ int Engine::launch_front(Staged &S) {
   if (qd_dirty)
     if ((rc = upload_qd())) return rc;
   if (S.match && (rc = prepare_filters())) return rc;
-  if ((rc = halloc(H.segcnt, S.nseg * 8)) || (rc = halloc(H.vtp, nn * 4)) || (rc = halloc(H.misc, 256)) ||
-      (rc = halloc(H.hdr, sizeof(BatchHdr))) || (rc = halloc(h_qlisted, std::max<size_t>(S.nq_live, 1) * 8)))
-    return rc;
+  // what the host reads of the batch: error block, counts, view times
+  const size_t counted = (size_t)S.nq_live * n * 8;
+  S.pack = counted + (size_t)n * 4 <= kPackBytes;
+  if ((rc = halloc(H.back, 64 + S.nseg * 8 + nn * 4))) return rc;
   if (!H.ev0) {
     CK(cudaEventCreate(&H.ev0));
     CK(cudaEventCreate(&H.ev_end));
     CK(cudaEventCreate(&H.ev_sort));
     CK(cudaEventCreate(&H.ev_sorted));
   }
-  BatchHdr &hd = *(BatchHdr *)H.hdr.ptr;
+  BatchHdr &hd = *(BatchHdr *)H.stage.ptr;
   hd.n = n;
   hd.m = m;
   hd.ngroups = S.ngroups;
@@ -208,25 +228,25 @@ int Engine::launch_front(Staged &S) {
   hd.seed_cap = S.seed_cap;
   hd.nseg = (unsigned long long)S.nq_live * n;
   hd.bloom_mask = (uint32_t)(bloom_words - 1);
-  hd.pad = 0;
+  hd.pack = S.pack;
+  hd.o_up = S.o_up;
+  hd.o_bk = S.o_bk;
+  hd.o_bi = S.o_bi;
+  hd.o_dk = S.o_dk;
+  hd.o_dh = S.o_dh;
 
-  // uploads (plain copies from the slot's pinned staging)
+  // one upload from the slot's pinned staging
   CK(cudaEventRecord(H.ev0, stream));
-  const char *st = (const char *)H.stage.ptr;
-  CK(cudaMemcpyAsync(d_hdr.ptr, H.hdr.ptr, sizeof(BatchHdr), cudaMemcpyHostToDevice, stream));
-  if (n) CK(cudaMemcpyAsync(d_upd.ptr, st + S.o_up, (size_t)n * 16, cudaMemcpyHostToDevice, stream));
-  if (m) {
-    CK(cudaMemcpyAsync(d_bkey.ptr, st + S.o_bk, (size_t)m * 8, cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(d_bidx.ptr, st + S.o_bi, (size_t)m * 4, cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(d_dkey.ptr, st + S.o_dk, S.ndir * 8, cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(d_dhead.ptr, st + S.o_dh, (S.ngroups + 1) * 4, cudaMemcpyHostToDevice, stream));
-  }
+  CK(cudaMemcpyAsync(d_stage.ptr, H.stage.ptr, S.stage_bytes, cudaMemcpyHostToDevice, stream));
 
   DevGraph g = dev_graph();
   const BatchHdr *dh = (const BatchHdr *)d_hdr.ptr;
   unsigned int *d_err = (unsigned int *)d_misc.ptr;
   unsigned long long *segwork = S.work_limit ? (unsigned long long *)d_segwork.ptr : nullptr;
-  ClearArgs ca{dh, (uint32_t *)d_vtp.ptr, (unsigned long long *)d_segcnt.ptr, segwork,
+  ClearArgs ca{(const unsigned char *)d_stage.ptr, (BatchHdr *)d_hdr.ptr, (uint4 *)d_upd.ptr,
+               (unsigned long long *)d_bkey.ptr, (unsigned long long *)d_dkey.ptr, (uint32_t *)d_bidx.ptr,
+               (uint32_t *)d_dhead.ptr, (unsigned long long *)d_job_seq.ptr, S.match && !S.plain ? job_ring : 0ull,
+               (uint32_t *)d_vtp.ptr, (unsigned long long *)d_segcnt.ptr, segwork,
                (unsigned long long *)d_qlisted.ptr, (Sched *)d_sched.ptr, (uint32_t *)d_misc.ptr, (uint32_t *)d_bloom.ptr,
                (uint32_t *)d_etable.ptr};
   EdgeStateArgs es{g, dh, (const uint4 *)d_upd.ptr, (const unsigned long long *)d_bkey.ptr,
@@ -238,7 +258,7 @@ int Engine::launch_front(Staged &S) {
                    (unsigned long long *)((char *)d_misc.ptr + 16)};
   SeedArgs sa{g, dh, (const uint4 *)d_upd.ptr, (const uint32_t *)d_vtp.ptr, (const uint32_t *)d_pair_off.ptr,
               (const uint32_t *)d_pair_ent.ptr, (const QDev *)d_qd.ptr, (const OrderRec *)d_orders.ptr,
-              (uint4 *)d_seeds.ptr, (Sched *)d_sched.ptr, kAllSlots};
+              (uint4 *)d_seeds.ptr, (Sched *)d_sched.ptr, kAllSlots, S.plain ? 0u : 1u, (uint32_t)stall_test, 0u};
   MatchArgs ma;
   std::memset(&ma, 0, sizeof(ma));
   ma.g = g;
@@ -274,13 +294,7 @@ int Engine::launch_front(Staged &S) {
 
   const bool tuning = tune_next && S.match && !S.plain;
   const bool graphed = use_graph && !tuning && !S.plain;
-  auto read_back = [&]() -> int {
-    CK(cudaMemcpyAsync(h_sched.ptr, d_sched.ptr, sizeof(Sched), cudaMemcpyDeviceToHost, stream));
-    CK(cudaMemcpyAsync((char *)h_sched.ptr + sizeof(Sched), d_misc.ptr, 64, cudaMemcpyDeviceToHost, stream));
-    if (S.nq_live)
-      CK(cudaMemcpyAsync(h_qlisted.ptr, d_qlisted.ptr, (size_t)S.nq_live * 8, cudaMemcpyDeviceToHost, stream));
-    return DSM_OK;
-  };
+  auto read_back = [&]() -> int { return read_sched(S.nq_live); };
   const ListArgs la = list_args(S);
   if (S.match && filter_mode > 0) filter_timed = true;  // a replayed graph records the filter events too
   if (graphed) {
@@ -311,10 +325,7 @@ int Engine::launch_front(Staged &S) {
         if (int r = rec(ev_pool[2])) return r;
         if (int r = launch_match_seq(ma, blocks, bfs_levels)) return r;
         if (int r = rec(ev_pool[3])) return r;
-        if (S.placed) {
-          launch_list_scan(la, stream);
-          stats.kernel_launches += 2;
-        }
+        if (S.placed) stats.kernel_launches += launch_list_scan(la, 0, stream);
       }
       return read_back();
     });
@@ -375,15 +386,8 @@ int Engine::match_eager(Staged &S, MatchArgs &ma, SeedArgs &sa, int blocks) {
     if (int r = rec(ev_pool[2])) return r;
     if (int r = launch_match_seq(ma, blocks, bfs_levels)) return r;
     if (int r = rec(ev_pool[3])) return r;
-    if (S.placed) {
-      launch_list_scan(list_args(S), stream);
-      stats.kernel_launches += 2;
-    }
-    CK(cudaMemcpyAsync(h_sched.ptr, d_sched.ptr, sizeof(Sched), cudaMemcpyDeviceToHost, stream));
-    CK(cudaMemcpyAsync((char *)h_sched.ptr + sizeof(Sched), d_misc.ptr, 64, cudaMemcpyDeviceToHost, stream));
-    if (S.nq_live)
-      CK(cudaMemcpyAsync(h_qlisted.ptr, d_qlisted.ptr, (size_t)S.nq_live * 8, cudaMemcpyDeviceToHost, stream));
-    return DSM_OK;
+    if (S.placed) stats.kernel_launches += launch_list_scan(list_args(S), (size_t)S.nq_live * S.n, stream);
+    return read_sched(S.nq_live);
   }
   // plain: query by query, the result table filling on from where the last
   // query left it
@@ -416,10 +420,7 @@ int Engine::match_eager(Staged &S, MatchArgs &ma, SeedArgs &sa, int blocks) {
   total.out_count.v = out;
   if (int r = rec(ev_pool[3])) return r;
   std::memcpy(hs, &total, sizeof(Sched));
-  if (S.placed) {
-    launch_list_scan(list_args(S), stream);
-    stats.kernel_launches += 2;
-  }
+  if (S.placed) stats.kernel_launches += launch_list_scan(list_args(S), (size_t)S.nq_live * S.n, stream);
   CK(cudaMemcpyAsync((char *)h_sched.ptr + sizeof(Sched), d_misc.ptr, 64, cudaMemcpyDeviceToHost, stream));
   if (S.nq_live)
     CK(cudaMemcpyAsync(h_qlisted.ptr, d_qlisted.ptr, (size_t)S.nq_live * 8, cudaMemcpyDeviceToHost, stream));
@@ -490,9 +491,11 @@ int Engine::finish_device(Staged &S) {
                    (unsigned int *)d_misc.ptr, (unsigned long long *)((char *)d_misc.ptr + 8),
                    (unsigned long long *)((char *)d_misc.ptr + 16)};
   const int blocks = num_sms * 4;
+  const PackArgs pk{(unsigned char *)d_pack.ptr, (const uint32_t *)d_misc.ptr,
+                    (const unsigned long long *)d_segcnt.ptr, (const uint32_t *)d_vtp.ptr};
   if (arena_short) {
     // nothing was written to the arena; the marks still go
-    launch_clear_touch(g, dh, (const uint4 *)d_upd.ptr, blocks, stream);
+    launch_clear_touch(g, dh, (const uint4 *)d_upd.ptr, pk, blocks, stream);
     CK(cudaStreamSynchronize(stream));
     if (int rc = compact_arena(arena_need16 * 4)) return rc;
     return kRetryArena;
@@ -584,7 +587,7 @@ int Engine::finish_device(Staged &S) {
       const int mblocks = num_sms * (warps_per_sm ? std::max(1, warps_per_sm / 8) : default_blocks_per_sm());
       SeedArgs sa{g, dh, (const uint4 *)d_upd.ptr, (const uint32_t *)d_vtp.ptr, (const uint32_t *)d_pair_off.ptr,
                   (const uint32_t *)d_pair_ent.ptr, (const QDev *)d_qd.ptr, (const OrderRec *)d_orders.ptr,
-                  (uint4 *)d_seeds.ptr, (Sched *)d_sched.ptr, kAllSlots};
+                  (uint4 *)d_seeds.ptr, (Sched *)d_sched.ptr, kAllSlots, 0u, 0u, 0u};
       if (S.plain) {
         if (int rc = match_eager(S, ma, sa, mblocks)) {
           S.match_rc = rc;
@@ -594,15 +597,8 @@ int Engine::finish_device(Staged &S) {
         if (int r = rec(ev_pool[2])) return r;
         if (int r = launch_match_seq(ma, mblocks, bfs_levels)) return r;
         if (int r = rec(ev_pool[3])) return r;
-        if (S.placed) {
-          launch_list_scan(list_args(S), stream);
-          stats.kernel_launches += 2;
-        }
-        CK(cudaMemcpyAsync(h_sched.ptr, d_sched.ptr, sizeof(Sched), cudaMemcpyDeviceToHost, stream));
-        CK(cudaMemcpyAsync((char *)h_sched.ptr + sizeof(Sched), d_misc.ptr, 64, cudaMemcpyDeviceToHost, stream));
-        if (S.nq_live)
-          CK(cudaMemcpyAsync(h_qlisted.ptr, d_qlisted.ptr, (size_t)S.nq_live * 8, cudaMemcpyDeviceToHost,
-                             stream));
+        if (S.placed) stats.kernel_launches += launch_list_scan(list_args(S), (size_t)S.nq_live * S.n, stream);
+        if (int r = read_sched(S.nq_live)) return r;
       }
       CK(cudaStreamSynchronize(stream));
       std::memcpy(&S.sc, h_sched.ptr, sizeof(Sched));
@@ -632,19 +628,20 @@ int Engine::finish_device(Staged &S) {
   const bool graphed = use_graph && !S.plain;
   auto seg_b = [&]() -> int {
     launch_adj_delete(au, blocks, stream);
-    launch_clear_touch(g, dh, (const uint4 *)d_upd.ptr, blocks, stream);
+    launch_clear_touch(g, dh, (const uint4 *)d_upd.ptr, pk, blocks, stream);
     stats.kernel_launches += 2;
     return DSM_OK;
   };
   if (graphed) {
     std::string key;
     key_append(key, au);
+    key_append(key, pk);
     key_append(key, blocks);
     if (int rc = run_segment(1, key, seg_b)) return rc;
   } else if (int rc = seg_b()) {
     return rc;
   }
-  const size_t nn = std::max<uint32_t>(S.n, 1);
+  const size_t counted = (size_t)S.nq_live * S.n * 8;
   if (S.placed) {
     if (S.words)
       CK(cudaMemcpyAsync(H.out_tup.ptr, S.out, S.words * 4, cudaMemcpyDeviceToHost, stream));
@@ -652,11 +649,14 @@ int Engine::finish_device(Staged &S) {
     CK(cudaMemcpyAsync(H.out_seg.ptr, d_out_seg.ptr, S.cnt * 4, cudaMemcpyDeviceToHost, stream));
     CK(cudaMemcpyAsync(H.out_tup.ptr, d_out_tup.ptr, S.cnt * S.W * 4, cudaMemcpyDeviceToHost, stream));
   }
-  if (S.nq_live && S.n)
-    CK(cudaMemcpyAsync(H.segcnt.ptr, d_segcnt.ptr, (size_t)S.nq_live * S.n * 8, cudaMemcpyDeviceToHost, stream));
-  CK(cudaMemcpyAsync(H.vtp.ptr, d_vtp.ptr, nn * 4, cudaMemcpyDeviceToHost, stream));
-  CK(cudaMemcpyAsync(H.misc.ptr, d_misc.ptr, 64, cudaMemcpyDeviceToHost, stream));
-  CK(cudaMemcpyAsync((char *)H.misc.ptr + 64, d_arena_top.ptr, 8, cudaMemcpyDeviceToHost, stream));
+  char *back = (char *)H.back.ptr;
+  if (S.pack) {
+    CK(cudaMemcpyAsync(back, d_pack.ptr, 64 + counted + (size_t)S.n * 4, cudaMemcpyDeviceToHost, stream));
+  } else {
+    CK(cudaMemcpyAsync(back, d_misc.ptr, 64, cudaMemcpyDeviceToHost, stream));
+    if (counted) CK(cudaMemcpyAsync(back + 64, d_segcnt.ptr, counted, cudaMemcpyDeviceToHost, stream));
+    CK(cudaMemcpyAsync(back + 64 + counted, d_vtp.ptr, (size_t)S.n * 4, cudaMemcpyDeviceToHost, stream));
+  }
   CK(cudaEventRecord(H.ev_end, stream));
   CK(cudaGetLastError());
   // a long-running stream abandons the old runs of relocated lists: compact
@@ -686,10 +686,10 @@ int Engine::run_front_and_finish(Staged &S) {
 int Engine::assemble(Staged &S, BatchResult &R) {
   HostOut &H = hout[S.slot];
   CK(cudaEventSynchronize(H.ev_end));
-  const unsigned int *err = (const unsigned int *)H.misc.ptr;
-  unsigned long long reloc = 0, top16 = 0;
-  std::memcpy(&reloc, (const char *)H.misc.ptr + 8, 8);
-  std::memcpy(&top16, (const char *)H.misc.ptr + 64, 8);
+  const char *back = (const char *)H.back.ptr;  // error block, counts, view times
+  const unsigned int *err = (const unsigned int *)back;
+  unsigned long long reloc = 0;
+  std::memcpy(&reloc, back + 8, 8);
   if (err[0] & kErrArena) return fail(DSM_ERR_OOM, "adjacency arena full (relocation failed)");
   if (S.match_rc) return S.match_rc;
   float ms_total = 0;
@@ -699,11 +699,11 @@ int Engine::assemble(Staged &S, BatchResult &R) {
   R.qids = S.qids;
   R.widths = S.widths;
   R.signs.assign(n, 0);
-  const uint32_t *vtp = (const uint32_t *)H.vtp.ptr;
+  const uint32_t *vtp = (const uint32_t *)(back + 64 + (size_t)nql * n * 8);
   for (uint32_t i = 0; i < n; ++i)
     if (vtp[i] != kNoView) R.signs[i] = S.ups[i].op ? 1 : -1;
   R.counts.assign((size_t)nql * n, 0);
-  if (nql && n) std::memcpy(R.counts.data(), H.segcnt.ptr, (size_t)nql * n * 8);
+  if (nql && n) std::memcpy(R.counts.data(), back + 64, (size_t)nql * n * 8);
   R.qlisted.assign(nql, S.listed ? 1 : 0);
   if (S.listed && S.qlimit)
     for (uint32_t ql = 0; ql < nql; ++ql)
@@ -799,7 +799,6 @@ int Engine::assemble(Staged &S, BatchResult &R) {
     stats.last_filter_ms = S.ms_filter;
     stats.last_sort_ms = R.sort_ms;
   }
-  (void)top16;
   return DSM_OK;
 }
 

@@ -228,7 +228,7 @@ struct Sched {
   unsigned long long alg_bytes;
   unsigned long long matches;  // embeddings counted (listed or not)
   unsigned int error;
-  unsigned int pad;
+  unsigned int armed;          // blocks of the seed kernel that have finished
   unsigned long long seeds;    // seeds of the batch, kept when a second launch takes rows as tasks
 };
 

@@ -112,10 +112,9 @@ Engine::~Engine() {
   for (auto &x : gexec)
     if (x) cudaGraphExecDestroy(x);
   for (DevBuf *b : all_dev_bufs()) dfree(*b);
-  for (HostBuf *b : {&h_sched, &h_qlisted})
-    if (b->ptr) cudaFreeHost(b->ptr);
+  if (h_sched.ptr) cudaFreeHost(h_sched.ptr);
   for (HostOut &H : hout) {
-    for (HostBuf *b : {&H.stage, &H.hdr, &H.segcnt, &H.vtp, &H.out_seg, &H.out_tup, &H.misc})
+    for (HostBuf *b : {&H.stage, &H.back, &H.out_seg, &H.out_tup})
       if (b->ptr) cudaFreeHost(b->ptr);
     if (H.ev0) cudaEventDestroy(H.ev0);
     if (H.ev_end) cudaEventDestroy(H.ev_end);
@@ -131,7 +130,7 @@ std::vector<DevBuf *> Engine::all_dev_bufs() {
   std::vector<DevBuf *> v = {&d_lab, &d_adj, &d_cap, &d_arena, &d_arena_top, &d_loff, &d_flt, &d_qd, &d_orders,
                              &d_pair_off, &d_pair_ent, &d_upd, &d_bkey, &d_bidx, &d_binfo, &d_gflag,
                              &d_vtp, &d_dkey, &d_dhead, &d_dsel, &d_seeds, &d_sched, &d_jobs,
-                             &d_job_seq, &d_out_seg, &d_out_tup, &d_segcnt, &d_misc, &d_hdr, &d_qlisted, &d_segwork,
+                             &d_job_seq, &d_out_seg, &d_out_tup, &d_segcnt, &d_hdr, &d_segwork, &d_stage, &d_pack,
                              &d_rinfo, &d_rmark, &d_rlist, &d_rprev, &d_rows, &d_bloom, &d_etable, &d_fdev,
                              &d_widths, &d_segoff, &d_segcur, &d_segchunk, &d_listsum, &d_list};
   for (auto &q : slots) v.push_back(&q.bitmap);
@@ -162,11 +161,9 @@ int Engine::init(int dev, size_t mem_budget) {
   int per_sm = match_max_blocks_per_sm(4);
   match_blocks_per_sm = std::max(1, std::min(per_sm, 8));
   // small fixed buffers
-  if (int rc = dalloc(d_sched, sizeof(Sched))) return rc;
+  if (int rc = sched_block(64)) return rc;
   if (int rc = dalloc(d_arena_top, 256)) return rc;
-  if (int rc = dalloc(d_misc, 256)) return rc;
   if (int rc = dalloc(d_hdr, 256)) return rc;
-  if (int rc = halloc(h_sched, sizeof(Sched) + 64)) return rc;
   return DSM_OK;
 }
 
@@ -314,6 +311,7 @@ RegionDevice Engine::region_dev() {
 
 DevGraph Engine::dev_graph() {
   DevGraph g;
+  std::memset(&g, 0, sizeof(g));  // compared bytewise (run_segment)
   g.nv = nv;
   g.lab = (uint32_t *)d_lab.ptr;
   g.adj = (uint2 *)d_adj.ptr;

@@ -52,9 +52,9 @@ struct Slot {
 // Pinned host side of one device batch in flight (two sets, so the serving
 // loop can assemble batch k on the host while batch k + 1 runs).
 struct HostOut {
-  HostBuf stage;   // uploads: updates, sorted keys, indices, directed pairs, group heads
-  HostBuf hdr;     // BatchHdr
-  HostBuf segcnt, vtp, out_seg, out_tup, misc;
+  HostBuf stage;   // the upload: BatchHdr, updates, sorted keys, indices, directed pairs, group heads
+  HostBuf back;    // the download: error block, counts, view times
+  HostBuf out_seg, out_tup;
   cudaEvent_t ev0 = nullptr, ev_end = nullptr;  // batch start, results downloaded
   cudaEvent_t ev_sort = nullptr, ev_sorted = nullptr;  // around the device sort
 };
@@ -66,6 +66,8 @@ struct Staged {
   uint32_t inserts = 0;  // of the m
   size_t ndir = 0;
   size_t o_up = 0, o_bk = 0, o_bi = 0, o_dk = 0, o_dh = 0;  // offsets in the staging buffer
+  size_t stage_bytes = 0;
+  bool pack = false;  // small enough for one download
   int slot = 0;
   bool match = true;  // false: apply the updates to the graph only
   double host_prep_ms = 0;
@@ -236,11 +238,12 @@ struct Engine {
 
   // batch scratch
   DevBuf d_upd, d_bkey, d_bidx, d_binfo, d_gflag, d_vtp, d_dkey, d_dhead, d_dsel, d_seeds, d_sched, d_jobs,
-      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_bloom, d_etable, d_fdev,
+      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_stage, d_pack, d_bloom, d_etable, d_fdev,
       d_widths, d_segoff, d_segcur, d_segchunk, d_listsum, d_list;
   std::vector<FilterDevice> fdev_host;  // what d_fdev holds
-  HostBuf h_sched;    // Sched + the error words, read after the matcher
-  HostBuf h_qlisted;  // per-query listing counters, read after the matcher
+  static constexpr size_t kMiscBytes = 256;
+  HostBuf h_sched;    // Sched, the error block and the listing counters, read after the matcher
+  HostBuf h_qlisted;  // view of the last
   HostOut hout[2];
   int next_slot = 0;
   uint64_t compactions = 0;
@@ -313,6 +316,8 @@ struct Engine {
   int finish_or_retry(Staged &S);       // finish_device; on a refused batch, compact and run it again
   int compact_arena(uint64_t extra_words);
   ListArgs list_args(const Staged &S);
+  int sched_block(uint32_t nq);
+  int read_sched(uint32_t nq);
   int place_results(Staged &S);
   int match_eager(Staged &S, MatchArgs &ma, SeedArgs &sa, int blocks);  // one launch, or one per query
   int seg_a_kernels(Staged &S, const ClearArgs &ca, const EdgeStateArgs &es, const AdjUpdateArgs &au,

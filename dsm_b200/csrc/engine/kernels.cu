@@ -364,8 +364,17 @@ __global__ void __launch_bounds__(256) k_adj_delete(AdjUpdateArgs A) {
   }
 }
 
-__global__ void k_clear_touch(DevGraph g, const BatchHdr *hdr, const uint4 *upd) {
+__global__ void k_clear_touch(DevGraph g, const BatchHdr *hdr, const uint4 *upd, PackArgs P) {
   const uint32_t n = hdr->n;
+  if (hdr->pack) {
+    const size_t stride = (size_t)gridDim.x * blockDim.x, t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t *o32 = reinterpret_cast<uint32_t *>(P.out);
+    unsigned long long *o64 = reinterpret_cast<unsigned long long *>(P.out + 64);
+    for (size_t i = t; i < 16; i += stride) o32[i] = P.misc[i];
+    for (size_t i = t; i < hdr->nseg; i += stride) o64[i] = P.segcnt[i];
+    o32 = reinterpret_cast<uint32_t *>(o64 + hdr->nseg);
+    for (size_t i = t; i < n; i += stride) o32[i] = P.vtp[i];
+  }
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     uint4 u = upd[i];
     if (u.y < g.nv) atomicAnd(&g.lab[u.y], kLabelMask);
@@ -401,9 +410,20 @@ __global__ void k_edge_filter(DevGraph g) {
 }
 
 __global__ void k_batch_clear(ClearArgs A) {
-  const BatchHdr h = *A.hdr;
+  const BatchHdr h = *reinterpret_cast<const BatchHdr *>(A.stage);
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) *A.hdr = h;
+  auto copy = [&](void *to, unsigned long long from, size_t words) {
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(A.stage + from);
+    for (size_t i = t; i < words; i += stride) static_cast<uint32_t *>(to)[i] = src[i];
+  };
+  copy(A.upd, h.o_up, 4ull * h.n);
+  copy(A.bkey, h.o_bk, 2ull * h.m);
+  copy(A.bidx, h.o_bi, h.m);
+  copy(A.dkey, h.o_dk, 4ull * h.m);
+  copy(A.dhead, h.o_dh, h.m ? h.ngroups + 1ull : 0ull);
+  for (size_t i = t; i < A.job_ring; i += stride) A.job_seq[i] = i;
   for (size_t i = t; i < h.n; i += stride) A.vtp[i] = kNoView;
   for (size_t i = t; i < h.nseg; i += stride) A.segcnt[i] = 0;
   if (A.segwork)
@@ -449,6 +469,20 @@ __global__ void k_seeds(SeedArgs A) {
     if (s < seed_cap) A.seeds[s] = make_uint4(i, ent, a, b);
   }
   }
+  if (!A.arm) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&A.sc->armed, 1u) == gridDim.x - 1) {  // every block's seeds are counted
+      unsigned long long total = ld_volatile(A.sc->nseeds);
+      if (total > seed_cap) {
+        A.sc->nseeds = total = seed_cap;
+        atomicOr(&A.sc->error, kErrSeeds);
+      }
+      A.sc->outstanding.v = total + A.phantom;
+      A.sc->done.v = total + A.phantom == 0 ? 1ull : 0ull;
+    }
+  }
 }
 
 }  // namespace
@@ -479,8 +513,9 @@ void launch_adj_delete(const AdjUpdateArgs &a, int blocks, cudaStream_t s) {
   k_adj_delete<<<blocks, 256, 0, s>>>(a);
 }
 
-void launch_clear_touch(DevGraph g, const BatchHdr *hdr, const uint4 *upd, int blocks, cudaStream_t s) {
-  k_clear_touch<<<blocks, 256, 0, s>>>(g, hdr, upd);
+void launch_clear_touch(DevGraph g, const BatchHdr *hdr, const uint4 *upd, const PackArgs &p, int blocks,
+                        cudaStream_t s) {
+  k_clear_touch<<<blocks, 256, 0, s>>>(g, hdr, upd, p);
 }
 
 void launch_seeds(const SeedArgs &a, int blocks, cudaStream_t s) {

@@ -18,14 +18,27 @@ struct BatchHdr {
   unsigned long long seed_cap;  // seed table capacity
   unsigned long long nseg;      // nq_live * n counters
   uint32_t bloom_mask;          // words of the changed-edge filter, less one (DevBatchEdges)
-  uint32_t pad;
+  uint32_t pack;                // 1: the batch's results are packed for one download (PackArgs)
+  // where the batch lies in the upload that starts with this header (bytes):
+  // updates, sorted keys, their updates, directed keys, source groups
+  unsigned long long o_up, o_bk, o_bi, o_dk, o_dh;
 };
+constexpr size_t kHdrBytes = 128;  // of the upload
+static_assert(sizeof(BatchHdr) <= kHdrBytes, "header fits its place in the upload");
 
-// Clears what a batch must start from: view times (kNoView), per-(query,
-// update) counts, per-query listing counters, the scheduler and the error
-// word.  Sizes from the header.
+// Starts a batch: its one upload (header, updates, keys) goes to the arrays the
+// batch's kernels read, whose addresses stay the same from batch to batch, and
+// what must start from nothing is cleared: view times (kNoView), per-(query,
+// update) counts, per-query listing counters, the scheduler, the error word,
+// the donation ring (job_ring slots; 0: left alone).  Sizes from the header.
 struct ClearArgs {
-  const BatchHdr *hdr;
+  const unsigned char *stage;
+  BatchHdr *hdr;
+  uint4 *upd;
+  unsigned long long *bkey, *dkey;
+  uint32_t *bidx, *dhead;
+  unsigned long long *job_seq;
+  unsigned long long job_ring;
   uint32_t *vtp;
   unsigned long long *segcnt;
   unsigned long long *segwork;  // null: no work limit this batch
@@ -79,7 +92,18 @@ void launch_arena_move(DevGraph g, const uint2 *nadj, uint32_t *narena, int bloc
 // The graph's edge filter (g.flt, cleared before) from its runs.
 void launch_edge_filter(DevGraph g, int blocks, cudaStream_t s);
 void launch_adj_delete(const AdjUpdateArgs &a, int blocks, cudaStream_t s);
-void launch_clear_touch(DevGraph g, const BatchHdr *hdr, const uint4 *upd, int blocks, cudaStream_t s);
+// Ends a batch: the endpoints' marks go and, with hdr->pack, what the host
+// downloads of it is laid out in one piece: 64 bytes of the error block, the
+// counts, the view times.
+struct PackArgs {
+  unsigned char *out;
+  const uint32_t *misc;
+  const unsigned long long *segcnt;
+  const uint32_t *vtp;
+};
+constexpr size_t kPackBytes = 1u << 18;  // at most, after the error block
+void launch_clear_touch(DevGraph g, const BatchHdr *hdr, const uint4 *upd, const PackArgs &p, int blocks,
+                        cudaStream_t s);
 
 // Seeds: one per (update, ordered query edge whose end labels match).
 struct SeedArgs {
@@ -94,6 +118,9 @@ struct SeedArgs {
   uint4 *seeds;               // {update, slot<<8|o, a, b}
   Sched *sc;
   uint32_t only_slot;         // seeds of this query slot only (kAllSlots: every query)
+  // 1: the last block to finish arms the matcher's scheduler (as
+  // launch_sched_init does, the ring's slots apart); phantom: see there
+  uint32_t arm, phantom, pad;
 };
 constexpr uint32_t kAllSlots = 0xFFFFFFFFu;
 void launch_seeds(const SeedArgs &a, int blocks, cudaStream_t s);
@@ -173,8 +200,10 @@ struct ListArgs {
   unsigned long long *partial;      // [3 * kListBlocks]
   unsigned long long *totals;       // words, sort chunks, tuples of the largest segment
 };
-// Offsets and totals from the matcher's counts (sizes from the batch header).
-void launch_list_scan(const ListArgs &a, cudaStream_t s);
+// Offsets and totals from the matcher's counts (sizes from the batch header;
+// nseg: the segments, or 0 in a captured launch that serves every size).
+// Returns the kernels launched.
+int launch_list_scan(const ListArgs &a, size_t nseg, cudaStream_t s);
 // The table's cnt rows (W words each) to their segments' places in `out`.
 void launch_list_place(const ListArgs &a, const uint32_t *seg, const uint32_t *rows, uint32_t W,
                        unsigned long long cnt, uint32_t *out, int num_sms, cudaStream_t s);

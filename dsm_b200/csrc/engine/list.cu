@@ -90,6 +90,8 @@ __global__ void __launch_bounds__(256) k_list_sum(ListArgs A) {
   }
 }
 
+// kAlone: one block for all segments, which sums them itself.
+template <bool kAlone>
 __global__ void __launch_bounds__(256) k_list_offsets(ListArgs A) {
   __shared__ unsigned long long s_words[8];
   __shared__ uint32_t s_chunks[8];
@@ -98,7 +100,14 @@ __global__ void __launch_bounds__(256) k_list_offsets(ListArgs A) {
   const unsigned long long lo = min(blockIdx.x * per, nseg), hi = min(lo + per, nseg);
   // the blocks before this one (the grid is kListBlocks = 256 blocks)
   Totals before{0, 0, 0}, all{0, 0, 0};
-  if (t < gridDim.x) {
+  if constexpr (kAlone) {
+    for (unsigned long long s = t; s < nseg; s += 256) {
+      const unsigned long long c = listed(A, n, s);
+      all.words += c * A.widths[s / n];
+      all.chunks += chunks_of(c);
+      all.most = max(all.most, c);
+    }
+  } else if (t < gridDim.x) {
     all = Totals{A.partial[3 * t], A.partial[3 * t + 1], A.partial[3 * t + 2]};
     if (t < blockIdx.x) before = all;
   }
@@ -302,9 +311,14 @@ __global__ void __launch_bounds__(256) k_list_merge(ListArgs A, const uint32_t *
 
 }  // namespace
 
-void launch_list_scan(const ListArgs &a, cudaStream_t s) {
+int launch_list_scan(const ListArgs &a, size_t nseg, cudaStream_t s) {
+  if (nseg && nseg <= 2048) {  // eight rounds of one block: no longer than the launch it saves (4 us)
+    k_list_offsets<true><<<1, 256, 0, s>>>(a);
+    return 1;
+  }
   k_list_sum<<<kListBlocks, 256, 0, s>>>(a);
-  k_list_offsets<<<kListBlocks, 256, 0, s>>>(a);
+  k_list_offsets<false><<<kListBlocks, 256, 0, s>>>(a);
+  return 2;
 }
 
 void launch_list_place(const ListArgs &a, const uint32_t *seg, const uint32_t *rows, uint32_t W,

@@ -165,7 +165,7 @@ extern "C" int dsm_count_edge_embeddings_noalloc(int device, uint32_t nv, const 
   const BatchHdr *dh = (const BatchHdr *)(base + kOffHdr);
   SeedArgs sa{g, dh, reinterpret_cast<const uint4 *>(d_updates), vtp, (const uint32_t *)(base + kOffPairOff),
               (const uint32_t *)(base + kOffPairEnt), (const QDev *)(base + kOffQd),
-              (const OrderRec *)(base + kOffOrders), (uint4 *)(base + kOffSeeds), sc, kAllSlots};
+              (const OrderRec *)(base + kOffOrders), (uint4 *)(base + kOffSeeds), sc, kAllSlots, 0u, 0u, 0u};
   int sms = 0, clk_khz = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&clk_khz, cudaDevAttrClockRate, device);

@@ -146,3 +146,26 @@ def test_without_room_the_host_places_and_sorts():
     for i in range(len(ups)):
         assert np.array_equal(r.tuples_of(qid, i), t[i])
     e.close()
+
+
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 40000])
+def test_batches_around_the_scan_and_the_packed_download(n):
+    """As many (query, update) segments as one block scans, one more, and more
+    counts than the packed download holds."""
+    nv, labels, edges, ups = _hubs([5, 40, 1], 0)
+    q = _query(0, False)
+    # toggles of the three hub edges and edges that change nothing
+    rng = np.random.default_rng(n)
+    pick = ups[rng.integers(0, len(ups), n)].copy()
+    pick[:, 0] = rng.integers(0, 2, n)
+    e = d.Engine(0)
+    e.load_graph_edges(nv, labels, edges)
+    qid = e.register(q)
+    st = oracle_stream(nv, labels, edges, q)
+    for b in (pick, pick[:3], pick[::-1].copy()):
+        r = e.run_batch(b)
+        s, c, t = st.apply(b)
+        assert np.array_equal(r.signs, s)
+        assert np.array_equal(r.counts[0], c)
+        assert np.array_equal(r.tuples.reshape(-1, 3), np.concatenate(t))
+    e.close()
