@@ -281,9 +281,10 @@ class BatchResult:
         self.widths = _arr(view.widths, nq)
         self.signs = _arr(view.signs, n, np.int8)
         self.counts = _arr(view.counts, nq * n, np.uint64).reshape(nq, n) if nq else np.zeros((0, n), np.uint64)
-        self.offsets = _arr(view.offsets, nq * n + 1, np.uint64)
-        self.tuples = _arr(view.tuples, int(self.offsets[-1]) if len(self.offsets) else 0)
         self.listed = bool(view.listed)
+        # without a listing every offset is 0
+        self.offsets = _arr(view.offsets, nq * n + 1, np.uint64) if self.listed else np.zeros(nq * n + 1, np.uint64)
+        self.tuples = _arr(view.tuples, int(self.offsets[-1]) if len(self.offsets) else 0)
         self.query_listed = _arr(view.query_listed, nq, np.uint8).astype(bool)
         self.num_updates = n
 

@@ -52,6 +52,24 @@ double ms_since(std::chrono::steady_clock::time_point t0) {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
+// Sorts v by bits [lo, hi) of its elements, stably: counting passes of 11 bits.
+void sort_by_bits(std::vector<uint64_t> &v, std::vector<uint64_t> &tmp, uint32_t lo, uint32_t hi) {
+  tmp.resize(v.size());
+  for (uint32_t b = lo; b < hi; b += 11) {
+    const uint64_t mask = (1ull << std::min(11u, hi - b)) - 1;
+    size_t at[2048] = {0};
+    for (const uint64_t x : v) ++at[(x >> b) & mask];
+    size_t sum = 0;
+    for (size_t &c : at) {
+      const size_t k = c;
+      c = sum;
+      sum += k;
+    }
+    for (const uint64_t x : v) tmp[at[(x >> b) & mask]++] = x;
+    v.swap(tmp);
+  }
+}
+
 template <class T>
 void key_append(std::string &k, const T &x) {
   k.append(reinterpret_cast<const char *>(&x), sizeof(T));
@@ -77,16 +95,40 @@ int Engine::prepare(const dsm_update *ups, uint32_t n, Staged &S, int slot) {
     S.inserts += ups[i].op != 0;
     und.push_back({a < b ? ((uint64_t)a << 32) | b : ((uint64_t)b << 32) | a, i});
   }
-  std::sort(und.begin(), und.end());
   S.m = (uint32_t)und.size();
-  std::vector<uint64_t> dir;
-  dir.reserve(2 * (size_t)S.m);
-  for (auto &e : und) {  // x << 32 | entry of y, so each group is in run order
-    const uint32_t a = (uint32_t)(e.first >> 32), b = (uint32_t)e.first;
-    dir.push_back(((uint64_t)a << 32) | entry_of(b));
-    dir.push_back(((uint64_t)b << 32) | entry_of(a));
+  // Sorted by key, ties in update order; then both directions, x << 32 | entry
+  // of y, so each group is in run order.  The ids use few of the 64 bits:
+  // large batches pack (key, update) into them and sort by counting, 11 bits a
+  // pass (33,000 updates: 8 ms by comparison, 1.5 ms so).
+  const uint32_t ib = std::max<uint32_t>(32 - __builtin_clz(std::max<uint32_t>(nv, 2) - 1), 1);
+  const uint32_t nb = 32 - __builtin_clz(n | 1);
+  std::vector<uint64_t> dir(2 * (size_t)S.m), tmp;
+  if (S.m >= 512 && 2 * ib + nb <= 64) {
+    std::vector<uint64_t> v(S.m);
+    for (uint32_t j = 0; j < S.m; ++j)
+      v[j] = ((und[j].first >> 32) << (ib + nb)) | ((uint64_t)(uint32_t)und[j].first << nb) | und[j].second;
+    sort_by_bits(v, tmp, nb, nb + 2 * ib);
+    const uint64_t im = (1ull << ib) - 1;
+    for (uint32_t j = 0; j < S.m; ++j)
+      und[j] = {((v[j] >> (ib + nb)) << 32) | ((v[j] >> nb) & im), (uint32_t)(v[j] & ((1ull << nb) - 1))};
+    for (uint32_t j = 0; j < S.m; ++j) {
+      const uint64_t a = und[j].first >> 32, b = (uint32_t)und[j].first;
+      const uint64_t sa = label_slot(label_host[a]), sb = label_slot(label_host[b]);
+      dir[2 * j] = a << (5 + ib) | sb << ib | b;
+      dir[2 * j + 1] = b << (5 + ib) | sa << ib | a;
+    }
+    sort_by_bits(dir, tmp, 0, 2 * ib + 5);
+    for (uint64_t &k : dir)
+      k = (k >> (5 + ib)) << 32 | ((k >> ib) & 31) << kIdBits | (k & im);
+  } else {
+    std::sort(und.begin(), und.end());
+    for (uint32_t j = 0; j < S.m; ++j) {
+      const uint32_t a = (uint32_t)(und[j].first >> 32), b = (uint32_t)und[j].first;
+      dir[2 * j] = ((uint64_t)a << 32) | entry_of(b);
+      dir[2 * j + 1] = ((uint64_t)b << 32) | entry_of(a);
+    }
+    std::sort(dir.begin(), dir.end());
   }
-  std::sort(dir.begin(), dir.end());
   std::vector<uint32_t> dhead;
   for (size_t j = 0; j < dir.size(); ++j)
     if (j == 0 || (dir[j] >> 32) != (dir[j - 1] >> 32)) dhead.push_back((uint32_t)j);
@@ -702,30 +744,44 @@ int Engine::assemble(Staged &S, BatchResult &R) {
   const uint32_t *vtp = (const uint32_t *)(back + 64 + (size_t)nql * n * 8);
   for (uint32_t i = 0; i < n; ++i)
     if (vtp[i] != kNoView) R.signs[i] = S.ups[i].op ? 1 : -1;
-  R.counts.assign((size_t)nql * n, 0);
-  if (nql && n) std::memcpy(R.counts.data(), back + 64, (size_t)nql * n * 8);
+  const size_t nseg = (size_t)nql * n;
+  R.counts.resize(nseg);
   R.qlisted.assign(nql, S.listed ? 1 : 0);
   if (S.listed && S.qlimit)
     for (uint32_t ql = 0; ql < nql; ++ql)
       if (S.qlisted[ql] > S.qlimit) R.qlisted[ql] = 0;
   // a segment over the work limit (bit 63) lists nothing and its count is
   // partial; the batch's exact matches leave it out
-  uint64_t exact = 0, incomplete = 0;
-  for (uint64_t c : R.counts) {
-    if (c & kCountIncomplete) ++incomplete;
-    else exact += c;
-  }
-  R.offsets.assign((size_t)nql * n + 1, 0);
-  for (uint32_t ql = 0; ql < nql; ++ql)
-    for (uint32_t i = 0; i < n; ++i) {
-      const size_t s = (size_t)ql * n + i;
-      const bool lst = R.qlisted[ql] && !(R.counts[s] & kCountIncomplete);
-      R.offsets[s + 1] = R.offsets[s] + (lst ? R.counts[s] * R.widths[ql] : 0);
+  std::atomic<uint64_t> exact_sum{0}, incomplete_sum{0};
+  parallel_for(nseg, 1u << 18, [&](size_t lo, size_t hi) {
+    const uint64_t *from = (const uint64_t *)(back + 64);
+    uint64_t *to = R.counts.data(), ex = 0, inc = 0;
+    for (size_t s = lo; s < hi; ++s) {
+      const uint64_t c = from[s];
+      to[s] = c;
+      if (c & kCountIncomplete) ++inc;
+      else ex += c;
     }
+    exact_sum += ex;
+    incomplete_sum += inc;
+  });
+  const uint64_t exact = exact_sum, incomplete = incomplete_sum;
+  if (S.listed) {
+    R.offsets.resize(nseg + 1);
+    R.offsets[0] = 0;
+    for (uint32_t ql = 0; ql < nql; ++ql)
+      for (uint32_t i = 0; i < n; ++i) {
+        const size_t s = (size_t)ql * n + i;
+        const bool lst = R.qlisted[ql] && !(R.counts[s] & kCountIncomplete);
+        R.offsets[s + 1] = R.offsets[s] + (lst ? R.counts[s] * R.widths[ql] : 0);
+      }
+  } else {
+    R.offsets.zeros(nseg + 1);
+  }
   R.listed = S.listed;
   R.tuples.resize(0);
   if (S.placed) {
-    if (S.words != R.offsets.back()) return fail(DSM_ERR_CUDA, "listed words differ from the counts");
+    if (S.words != R.offsets[nseg]) return fail(DSM_ERR_CUDA, "listed words differ from the counts");
     R.tuples.resize(S.words);
     const uint32_t *from = (const uint32_t *)H.out_tup.ptr;
     uint32_t *to = R.tuples.data();
@@ -734,9 +790,8 @@ int Engine::assemble(Staged &S, BatchResult &R) {
     if (S.sort && S.words) elapsed(H.ev_sort, H.ev_sorted, &ms);
     R.sort_ms = ms;
   } else if (S.listed) {
-    R.tuples.resize(R.offsets.back());
+    R.tuples.resize(R.offsets[nseg]);
     const uint32_t *hs = (const uint32_t *)H.out_seg.ptr, *ht = (const uint32_t *)H.out_tup.ptr;
-    const size_t nseg = (size_t)nql * n;
     if (S.cnt < (1u << 16)) {
       std::vector<uint64_t> cur(R.offsets.begin(), R.offsets.end() - 1);
       for (size_t r = 0; r < S.cnt; ++r) {
@@ -765,7 +820,7 @@ int Engine::assemble(Staged &S, BatchResult &R) {
       });
     }
     if (S.sort) {
-      std::vector<uint64_t> cnt_listed(R.counts);
+      std::vector<uint64_t> cnt_listed(R.counts.begin(), R.counts.end());
       for (uint32_t ql = 0; ql < nql; ++ql)
         for (uint32_t i = 0; i < n; ++i) {
           uint64_t &c = cnt_listed[(size_t)ql * n + i];

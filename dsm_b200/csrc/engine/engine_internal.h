@@ -8,11 +8,13 @@
 #include <chrono>
 #include <condition_variable>
 #include <cstdint>
+#include <cstdlib>
 #include <deque>
 #include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <set>
 #include <string>
 #include <thread>
@@ -89,17 +91,30 @@ struct Staged {
   float ms_match = 0, ms_upd = 0, ms_filter = 0, ms_sort = 0;
 };
 
-// Tuple words of a result: sized once, not cleared (every word is written).
-struct TupleBuf {
-  std::unique_ptr<uint32_t[]> p;
+// An array of a result: sized once, not cleared (every element is written), or
+// all zeros in pages the system hands out untouched (clearing and filling
+// vectors of two million counts took longer than the download of them).
+template <class T>
+struct ResultArray {
+  struct Free {
+    void operator()(void *q) const { std::free(q); }
+  };
+  std::unique_ptr<T, Free> p;
   size_t n = 0;
-  void resize(size_t words) {
-    p.reset(words ? new uint32_t[words] : nullptr);
-    n = words;
-  }
+  void resize(size_t count) { take(count ? std::malloc(count * sizeof(T)) : nullptr, count); }
+  void zeros(size_t count) { take(count ? std::calloc(count, sizeof(T)) : nullptr, count); }
   size_t size() const { return n; }
-  uint32_t *data() { return p.get(); }
-  uint32_t &operator[](size_t i) { return p[i]; }
+  T *data() { return p.get(); }
+  T &operator[](size_t i) { return p.get()[i]; }
+  T *begin() { return p.get(); }
+  T *end() { return p.get() + n; }
+
+ private:
+  void take(void *q, size_t count) {
+    if (count && !q) throw std::bad_alloc();
+    p.reset(static_cast<T *>(q));
+    n = count;
+  }
 };
 
 struct BatchResult {
@@ -108,8 +123,8 @@ struct BatchResult {
   std::vector<uint32_t> qids, widths;
   std::vector<uint8_t> qlisted;  // per query: its tuples are listed
   std::vector<int8_t> signs;
-  std::vector<uint64_t> counts, offsets;
-  TupleBuf tuples;
+  ResultArray<uint64_t> counts, offsets;
+  ResultArray<uint32_t> tuples;
   int listed = 1;
   double device_ms = 0, match_ms = 0, host_prep_ms = 0, sort_ms = 0;
   uint64_t alg_bytes = 0, matches = 0, incomplete = 0;

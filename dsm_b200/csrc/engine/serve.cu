@@ -285,15 +285,17 @@ void Engine::post_batch(InFlight &b) {
     o->listed = R.listed;
     o->signs.assign(R.signs.begin() + s, R.signs.begin() + s + n);
     o->counts.resize((size_t)nql * n);
-    o->offsets.assign((size_t)nql * n + 1, 0);
+    if (R.listed) o->offsets.resize((size_t)nql * n + 1);
+    else o->offsets.zeros((size_t)nql * n + 1);
+    if (R.listed) o->offsets[0] = 0;
     for (uint32_t ql = 0; ql < nql; ++ql)
       for (uint32_t i = 0; i < n; ++i) {
         const size_t src = (size_t)ql * N + s + i, dst = (size_t)ql * n + i;
         o->counts[dst] = R.counts[src];
-        o->offsets[dst + 1] = o->offsets[dst] + (R.offsets[src + 1] - R.offsets[src]);
+        if (R.listed) o->offsets[dst + 1] = o->offsets[dst] + (R.offsets[src + 1] - R.offsets[src]);
       }
     if (R.listed) {
-      o->tuples.resize(o->offsets.back());
+      o->tuples.resize(o->offsets[(size_t)nql * n]);
       for (uint32_t ql = 0; ql < nql; ++ql) {  // each query's slice is contiguous
         const size_t a = R.offsets[(size_t)ql * N + s], e = R.offsets[(size_t)ql * N + s + n];
         if (e > a) std::memcpy(o->tuples.data() + o->offsets[(size_t)ql * n], R.tuples.data() + a, (e - a) * 4);

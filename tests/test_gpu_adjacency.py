@@ -55,3 +55,32 @@ def test_hub_run_grows_and_shrinks(deg, nlab):
         for x, y in zip(e.export_graph(), st.export()):
             assert np.array_equal(x, y), k
     e.close()
+
+
+@pytest.mark.parametrize("n", [511, 512, 513, 3000])
+@pytest.mark.parametrize("nv,nlab", [(1024, 3), (1025, 31), (70_000, 40)])
+def test_batches_around_the_counting_sort(n, nv, nlab):
+    """Batches of as many updates as are sorted by counting, and fewer; vertex
+    ids of 10, 11 and 17 bits; labels on both sides of the shared slot; each
+    edge named several times.  Graph, signs and counts equal the oracle's."""
+    rng = np.random.default_rng(n + nv)
+    labels = rng.integers(0, nlab, nv).astype(np.uint32)
+    edges = rng.integers(0, nv, (2000, 2)).astype(np.uint32)
+    edges = edges[edges[:, 0] != edges[:, 1]]
+    pool = np.concatenate([edges[:200], rng.integers(0, nv, (200, 2)), [[0, nv - 1], [nv - 1, nv - 2], [4, 4]]])
+    q = d.Query.from_edges([labels[edges[0, 0]] % 32, labels[edges[0, 1]] % 32], [(0, 1)])
+    e = d.Engine(0)
+    e.set_option(d.OPT_LIST, 0)
+    e.load_graph_edges(nv, labels, edges)
+    qid = e.register(q)
+    st = oracle_stream(nv, labels, edges, q)
+    for _ in range(2):
+        pick = pool[rng.integers(0, len(pool), n)]
+        b = np.concatenate([rng.integers(0, 2, (n, 1)), pick, np.zeros((n, 1))], 1).astype(np.uint32)
+        r = e.run_batch(b)
+        s, c, _t = st.apply(b, listed=False)
+        assert np.array_equal(r.signs, s)
+        assert np.array_equal(r.counts[r.query_index(qid)], c)
+        for x, y in zip(e.export_graph(), st.export()):
+            assert np.array_equal(x, y)
+    e.close()
