@@ -182,8 +182,7 @@ void launch_match(const MatchArgs &a, int blocks, cudaStream_t s);
 // with the rows written so far as its tasks (counters of work done, the
 // result-table position and the error word carry over).
 void launch_rows_arm(Sched *sc, const unsigned long long *rows_cnt, unsigned long long rows_cap, cudaStream_t s);
-// Resident matcher blocks per SM for queries of up to `width` vertices (0:
-// plain runs).
+// Resident matcher blocks per SM for queries of up to `width` vertices.
 int match_max_blocks_per_sm(uint32_t width);
 
 // Listed results in canonical order on the device (list.cu).

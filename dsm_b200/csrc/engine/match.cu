@@ -104,9 +104,6 @@ __device__ void finish_task(const MatchArgs &P) {
     atomicExch(&P.job_seq[t & (P.job_ring - 1)], t | kSeqDone);
 }
 
-// ---------------------------------------------------------------------------
-// Label-major runs (the engine's graph)
-// ---------------------------------------------------------------------------
 // A task's search goes depth-first over batches: up to 32 partial embeddings
 // of one level, a lane each, are expanded together.  E(l) is the expansion of
 // the batch of level l (its partials fix positions 0..l) to level t = l + 1:
@@ -139,15 +136,22 @@ __device__ void finish_task(const MatchArgs &P) {
 // where most entries pass (a hub-heavy graph with 8 labels) it neither gains
 // nor costs (15 ms).
 //
+// kLM: label-major runs with slot offsets (the engine's graph); otherwise plain
+// id-sorted runs (the allocation-free entry point): a position's range is then
+// the whole run and every entry's label is read.
+//
 // Shared memory of a warp (W = widest query): the batch's images F[W][32]
 // (column k: the partial of lane k), up to kRows ranges per partial, the pivot
 // per partial, 64 candidates (position in the ranges, id | owner << 27), and a
-// buffer of 64 survivors per level (id | parent << 27).
+// buffer of 64 survivors per level (id | parent << 27; plain runs, whose ids may
+// take all 32 bits, keep the parents behind the ids).
 constexpr uint32_t kRows = 3;  // backward neighbours with stored ranges; further ones are read when needed
+template <bool kLM>
 __host__ __device__ constexpr uint32_t warp_words(uint32_t W) {
-  return W * 32 + kRows * 128 + 128 + 128 + (W > 3 ? W - 3 : 1) * 64;
+  return W * 32 + kRows * 128 + 128 + 128 + (W > 3 ? W - 3 : 1) * (kLM ? 64 : 128);
 }
 
+template <bool kLM>
 __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t nupd, uint32_t upd, uint32_t qo,
                          uint32_t depth, uint32_t lo, uint32_t hi, uint32_t fval, uint32_t *sm) {
   const uint32_t lane = threadIdx.x & 31;
@@ -155,7 +159,22 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   uint4(*const rows)[32] = reinterpret_cast<uint4(*)[32]>(sm + P.W * 32);
   uint4 *const piv = reinterpret_cast<uint4 *>(sm + P.W * 32 + kRows * 128);
   uint2 *const cand = reinterpret_cast<uint2 *>(sm + P.W * 32 + kRows * 128 + 128);
-  uint32_t(*const buf)[64] = reinterpret_cast<uint32_t(*)[64]>(sm + P.W * 32 + kRows * 128 + 256) - 2;  // from level 2
+  constexpr uint32_t kBuf = kLM ? 64 : 128;
+  uint32_t(*const buf)[kBuf] = reinterpret_cast<uint32_t(*)[kBuf]>(sm + P.W * 32 + kRows * 128 + 256) - 2;  // from level 2
+  // survivor i of level t: its image, and the lane of its partial below
+  auto put = [&](uint32_t t, uint32_t i, uint2 x) {
+    if constexpr (kLM) {
+      buf[t][i] = x.x | (x.y << kIdBits);
+    } else {
+      buf[t][i] = x.x;
+      buf[t][64 + i] = x.y;
+    }
+  };
+  auto get = [&](uint32_t t, uint32_t i) -> uint2 {
+    const uint32_t x = buf[t][i];
+    if constexpr (kLM) return make_uint2(x & kIdMask, x >> kIdBits);
+    else return make_uint2(x, buf[t][64 + i]);
+  };
   const QDev &Q = P.qd[qo >> 8];
   const uint32_t nq = Q.nq;
   const OrderRec &R = P.orders[Q.order_base + (qo & 255)];
@@ -260,14 +279,20 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
     uint32_t best = 0xFFFFFFFFu, pr = 0, pa = 0, poff = 0, r = 0;
     for (uint32_t bits = t_bn; bits; bits &= bits - 1, ++r) {
       uint32_t a = 0, b = 0, off = 0, touched = 0;
-      if (lane < nb && t_lab < P.g.nlt) {
-        const uint32_t x = F[__ffs(bits) - 1][lane];
-        const uint32_t *o = P.g.loff + (size_t)x * (P.g.nlt + 1) + t_lab;
-        a = o[0];
-        b = o[1];
-        off = P.g.adj[x].x;
-        touched = P.g.lab[x] >> 31;
-        alg += 8;
+      if constexpr (kLM) {
+        if (lane < nb && t_lab < P.g.nlt) {
+          const uint32_t x = F[__ffs(bits) - 1][lane];
+          const uint32_t *o = P.g.loff + (size_t)x * (P.g.nlt + 1) + t_lab;
+          a = o[0];
+          b = o[1];
+          off = P.g.adj[x].x;
+          touched = P.g.lab[x] >> 31;
+          alg += 8;
+        }
+      } else if (lane < nb) {
+        const uint2 x = P.g.adj[F[__ffs(bits) - 1][lane]];
+        off = x.x;
+        b = x.y;
       }
       if (r < kRows) rows[r][lane] = make_uint4(off, a, b, touched);
       if (b - a < best) {
@@ -305,9 +330,9 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
     __syncwarp();
     uint32_t k = lane;
     for (uint32_t j = l; j >= depth; --j) {
-      const uint32_t x = buf[j][k];
-      F[j][lane] = x & kIdMask;
-      k = x >> kIdBits;
+      const uint2 x = get(j, k);
+      F[j][lane] = x.x;
+      k = x.y & 31;
     }
     __syncwarp();
   };
@@ -384,7 +409,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   // screened 8-vertex queries lost 5 to 15 %, from 256 on none; 256 queries x
   // 1021 updates gain 10 % at any bound up to 512).
   auto leaf = [&]() -> bool {
-    return cnt_only && l + 2 == nq && e >= 256 && (t_bn & (t_bn - 1)) == 0 && t_lab < 31;
+    return kLM && cnt_only && l + 2 == nq && e >= 256 && (t_bn & (t_bn - 1)) == 0 && t_lab < 31;
   };
 
   e = setup();
@@ -402,7 +427,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   while (true) {
     if (cnt < most && (c < e || nc)) {
       const uint32_t t = l + 1;
-      const bool two = P.g.flt && (t_bn & (t_bn - 1));
+      const bool two = kLM && P.g.flt && (t_bn & (t_bn - 1));
       bool ok = false, test = true;
       uint32_t k = 0, w = 0;
       if (!two || (nc < 32 && c < e)) {  // a chunk of the ranges
@@ -415,7 +440,8 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
         }
         const uint4 pv = piv[k];
         if (ok) {
-          w = P.g.arena[((uint64_t)pv.y << 32 | pv.x) + pos] & kIdMask;
+          w = P.g.arena[((uint64_t)pv.y << 32 | pv.x) + pos];
+          if constexpr (kLM) w &= kIdMask;
           alg += 4;
         }
         c = min(c + 32, e);
@@ -443,9 +469,9 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
         k = ok ? x.y >> kIdBits : 0u;
         nc -= n;
       }
-      const uint32_t en = (t_lab << kIdBits) | w;
+      const uint32_t en = kLM ? (t_lab << kIdBits) | w : w;
       ok = ok && test;
-      if (t_lab >= 31)  // slot 31 holds every label >= 31
+      if (!kLM || t_lab >= 31)  // plain runs hold every label, slot 31 every label >= 31
         ok = ok && ((P.g.lab[w] & kLabelMask) == t_lab);
       // injectivity: only earlier positions with the same label can hold w
       for (uint32_t same = t_same; same; same &= same - 1) ok = ok && w != F[__ffs(same) - 1][k];
@@ -462,8 +488,13 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
           row = rows[r][k];
         } else {
           const uint32_t x = F[j][k];
-          const uint32_t *o = P.g.loff + (size_t)x * (P.g.nlt + 1) + t_lab;
-          row = make_uint4(P.g.adj[x].x, o[0], o[1], P.g.lab[x] >> 31);
+          if constexpr (kLM) {
+            const uint32_t *o = P.g.loff + (size_t)x * (P.g.nlt + 1) + t_lab;
+            row = make_uint4(P.g.adj[x].x, o[0], o[1], P.g.lab[x] >> 31);
+          } else {
+            const uint2 a = P.g.adj[x];
+            row = make_uint4(a.x, 0, a.y, 0);
+          }
         }
         if (r != piv[k].z) {
           ok = run_has(P.g.arena + (uint64_t)row.x * 4 + row.y, row.z - row.y, en);
@@ -471,7 +502,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
         }
         // liveness: only edges of a touched vertex can have changed, and of
         // those the filter turns away all that the batch does not change
-        if (ok && row.w) {
+        if (kLM && ok && row.w) {
           const uint32_t x = F[j][k];
           if (may_change(bt, x, w)) ok = edge_live(bt, x, w, tp);
         }
@@ -484,7 +515,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
       if (t == nq - 1) {
         emit(m, w, t, k);
       } else if (m && !(P.bfs_stop == t + 1 && write_rows(m, w, k))) {
-        if (ok) buf[t][cnt + __popc(m & lanemask_lt())] = w | (k << kIdBits);
+        if (ok) put(t, cnt + __popc(m & lanemask_lt()), make_uint2(w, k));
         cnt += ns;
       }
       if (P.work_limit && work >= work_left) {
@@ -541,9 +572,9 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
             if (wi && i + 1 + dd < nq) {
               jobs = min(wi, (uint32_t)min(h, 32ull));
               mine = lane < jobs;
-              const uint32_t x = mine ? buf[i + 1][ni - jobs + lane] : 0u;
-              jk = x >> kIdBits;
-              jw = x & kIdMask;
+              const uint2 x = mine ? get(i + 1, ni - jobs + lane) : make_uint2(0, 0);
+              jk = x.y;
+              jw = x.x;
               jdepth = i + 2;
             } else {
               const uint32_t excl = incl - len;
@@ -646,14 +677,14 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
       park();
       __syncwarp();
       nb = min(cnt, most);
-      const uint32_t x = buf[l + 1][lane < nb ? lane : 0];
+      const uint2 x = get(l + 1, lane < nb ? lane : 0);
       for (uint32_t j = depth; j <= l; ++j) {
-        const uint32_t v = F[j][x >> kIdBits];
+        const uint32_t v = F[j][x.y];
         __syncwarp();
         F[j][lane] = v;
       }
       ++l;
-      F[l][lane] = x & kIdMask;
+      F[l][lane] = x.x;
       __syncwarp();
       c = 0;
       cnt = 0;
@@ -679,294 +710,20 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
     nb &= 0xFFu;
     if (cnt || c < e) {
       __syncwarp();
-      uint32_t y[2];
+      uint2 y[2];
 #pragma unroll
-      for (uint32_t h = 0; h < 2; ++h) y[h] = lane + 32 * h < cnt ? buf[l + 1][done + lane + 32 * h] : 0u;
+      for (uint32_t h = 0; h < 2; ++h)
+        y[h] = lane + 32 * h < cnt ? get(l + 1, done + lane + 32 * h) : make_uint2(0, 0);
       __syncwarp();
 #pragma unroll
       for (uint32_t h = 0; h < 2; ++h)
-        if (lane + 32 * h < cnt) buf[l + 1][lane + 32 * h] = y[h];
+        if (lane + 32 * h < cnt) put(l + 1, lane + 32 * h, y[h]);
       rebuild();
       if (c < e) setup();
     }
   }
   flush();
 }
-
-// ---------------------------------------------------------------------------
-// Plain id-sorted runs (the allocation-free entry point: counts on a fixed
-// graph, no listing, no work limit, every edge live)
-// ---------------------------------------------------------------------------
-// One partial embedding at a time, the stack spread over the lanes: lane p
-// keeps the image f[p] of position p with its run, and the iteration state of
-// level p.  The level being scanned keeps its state in warp-uniform registers
-// (cur_*); one with deeper levels running parks it in its own lane (lv_*).
-__device__ void run_task_plain(const MatchArgs &P, uint32_t nupd, uint32_t upd, uint32_t qo, uint32_t depth,
-                               uint32_t lo, uint32_t hi, uint32_t fval) {
-  const uint32_t lane = threadIdx.x & 31;
-  const QDev &Q = P.qd[qo >> 8];
-  const uint32_t nq = Q.nq;
-  const OrderRec &R = P.orders[Q.order_base + (qo & 255)];
-  const uint32_t q_vert = lane < 16 ? R.vert[lane] : 0;
-  const uint32_t q_bn = lane < 16 ? R.bn[lane] : 0;
-  const uint32_t q_lab = Q.label[q_vert & 15];
-  const uint32_t seg = Q.local * nupd + upd;
-
-  uint32_t my_f = fval, my_off = 0, my_deg = 0;
-  if (lane < depth) {
-    uint2 a = P.g.adj[my_f];
-    my_off = a.x;
-    my_deg = a.y;
-  }
-  unsigned long long alg = 0, task_cnt = 0;  // warp-uniform
-
-  auto flush = [&]() {
-    if (lane == 0) {
-      if (task_cnt) {
-        atomicAdd(&P.seg_count[seg], task_cnt);
-        atomicAdd(&P.sc->matches, task_cnt);
-      }
-      atomicAdd(&P.sc->alg_bytes, alg);
-    }
-  };
-
-  if (depth >= nq) {  // a one-edge query: the seed is the embedding
-    task_cnt = 1;
-    flush();
-    return;
-  }
-  // the current level (warp-uniform): its pivot run, next entry, end, pending
-  // candidates of the last chunk, that chunk's first entry; its label and
-  // backward neighbours
-  uint32_t cur_base = 0, cur_pos = 0, cur_end = 0, cur_mask = 0, cur_chunk = 0, cur_pivot = 0;
-  uint32_t cur_want = 0, cur_bn = 0;
-  // level `lane`, parked while deeper levels run
-  uint32_t lv_pos = 0, lv_end = 0, lv_mask = 0, lv_chunk = 0;
-
-  // Level L scans the run of its pivot: the backward neighbour of the smallest
-  // degree.  [rlo, rhi) narrows the scan for a donated range (rhi = 0: all).
-  auto setup_level = [&](uint32_t L, uint32_t rlo, uint32_t rhi) {
-    cur_bn = __shfl_sync(kFull, q_bn, L);
-    cur_want = __shfl_sync(kFull, q_lab, L);
-    const bool inb = (cur_bn >> lane) & 1u;
-    const uint32_t key = inb ? ((min(my_deg, 0x3FFFFFFu) << 5) | lane) : 0xFFFFFFFFu;
-    cur_pivot = __reduce_min_sync(kFull, key) & 31;
-    cur_base = __shfl_sync(kFull, my_off, cur_pivot);
-    const uint32_t end = __shfl_sync(kFull, my_deg, cur_pivot);
-    cur_pos = rhi ? rlo : 0;
-    cur_end = rhi ? min(rhi, end) : end;
-    cur_mask = 0;
-    cur_chunk = 0;
-  };
-
-  // The same choice, recomputed instead of parked.
-  auto pivot_of = [&](uint32_t L) -> uint32_t {
-    const uint32_t bnL = __shfl_sync(kFull, q_bn, L);
-    const bool inb = (bnL >> lane) & 1u;
-    const uint32_t key = inb ? ((min(my_deg, 0x3FFFFFFu) << 5) | lane) : 0xFFFFFFFFu;
-    return __reduce_min_sync(kFull, key) & 31;
-  };
-  auto pivot_base = [&](uint32_t L) -> uint32_t { return __shfl_sync(kFull, my_off, pivot_of(L)); };
-  auto resume_pivot = [&](uint32_t L) {
-    cur_pivot = pivot_of(L);
-    cur_base = __shfl_sync(kFull, my_off, cur_pivot);
-  };
-
-  uint32_t hb = 0;  // chunks since the last heartbeat
-
-  uint32_t L = depth;
-  setup_level(L, lo, hi);
-  uint32_t dticks = 0;  // chunks since the last donation check
-  while (true) {
-    if (cur_mask == 0) {
-      if (cur_pos >= cur_end) {
-        if (L == depth) break;
-        --L;  // back to the parked level
-        cur_pos = __shfl_sync(kFull, lv_pos, L);
-        cur_end = __shfl_sync(kFull, lv_end, L);
-        cur_mask = __shfl_sync(kFull, lv_mask, L);
-        cur_chunk = __shfl_sync(kFull, lv_chunk, L);
-        cur_bn = __shfl_sync(kFull, q_bn, L);
-        cur_want = __shfl_sync(kFull, q_lab, L);
-        resume_pivot(L);
-        continue;
-      }
-      const uint32_t pos = cur_pos, end = cur_end;
-      const uint32_t *run = P.g.arena + (uint64_t)cur_base * 4;
-      const uint32_t i = pos + lane;
-      bool ok = i < end;
-      const uint32_t w = ok ? run[i] : 0;
-      const uint32_t want = cur_want;
-      ok = ok && ((P.g.lab[w] & kLabelMask) == want);
-      // injectivity: only earlier positions with the same label can hold w
-      for (uint32_t same = __ballot_sync(kFull, lane < L && q_lab == want); same; same &= same - 1) {
-        const uint32_t fj = __shfl_sync(kFull, my_f, __ffs(same) - 1);
-        ok = ok && (w != fj);
-      }
-      const uint32_t bnL = cur_bn;
-      uint32_t others = bnL & ~(1u << cur_pivot);
-      uint32_t probes = 0;
-      while (others) {
-        uint32_t j = __ffs(others) - 1;
-        others &= others - 1;
-        const uint32_t oj = __shfl_sync(kFull, my_off, j), dj = __shfl_sync(kFull, my_deg, j);
-        if (ok) {
-          const uint32_t *lst = P.g.arena + (uint64_t)oj * 4;
-          const uint32_t p = lower_bound_u32(lst, dj, w);
-          ok = p < dj && lst[p] == w;
-          ++probes;
-        }
-      }
-      const uint32_t m = __ballot_sync(kFull, ok);
-      alg += 8ull * min(32u, end - pos) + 4ull * __reduce_add_sync(kFull, probes);
-      cur_pos = pos + 32;
-      cur_chunk = pos;
-      ++hb;
-      ++dticks;
-      if (L == nq - 1) task_cnt += __popc(m);
-      else cur_mask = m;
-
-      if (hb >= 64) {
-        hb = 0;
-        unsigned int err = 0;
-        if (lane == 0) {
-          atomicAdd(&P.sc->progress.v, 1ull);
-          err = ld_volatile(P.sc->error);
-        }
-        if (__shfl_sync(kFull, err, 0)) break;
-      }
-      if (P.donate && dticks >= 8) {
-        dticks = 0;
-        const uint32_t split_min = P.split_min > 64 ? P.split_min : (P.split_min ? 64u : 128u);
-        const uint32_t dd = P.donate_depth ? min(P.donate_depth, 4u) : 2u;
-        unsigned long long h = 0;
-        if (lane == 0) {
-          unsigned long long pc = ld_volatile(P.sc->pop_cnt.v), pu = ld_volatile(P.sc->push_cnt.v);
-          h = pc > pu ? pc - pu : 0;
-        }
-        h = __shfl_sync(kFull, h, 0);
-        if (h > 0) {
-          if (lane == L) {  // park the current level, so every level reads alike
-            lv_pos = cur_pos;
-            lv_end = cur_end;
-            lv_mask = cur_mask;
-            lv_chunk = cur_chunk;
-          }
-          // shallowest level with a substantial piece of work: pending
-          // candidates with dd or more levels below them, or a remaining
-          // range of split_min entries or more
-          bool has = lane >= depth && lane <= L &&
-                     ((lv_mask != 0 && lane + dd < nq) || lv_end >= lv_pos + split_min);
-          uint32_t hm = __ballot_sync(kFull, has);
-          if (hm) {
-            const uint32_t p = __ffs(hm) - 1;
-            const uint32_t pm0 = __shfl_sync(kFull, lv_mask, p);
-            const uint32_t pm = (p + dd < nq) ? pm0 : 0u;
-            uint32_t k, dmask = 0, rmid = 0, rend = 0;
-            if (pm) {
-              k = min((uint32_t)__popc(pm), (uint32_t)min(h, 32ull));
-              uint32_t t = pm;  // donate the k highest pending bits
-              for (uint32_t r = __popc(pm); r > k; --r) t &= t - 1;
-              dmask = t;
-            } else {
-              uint32_t ppos = __shfl_sync(kFull, lv_pos, p), pend = __shfl_sync(kFull, lv_end, p);
-              rmid = ppos + (((pend - ppos) / 2 + 31) & ~31u);
-              rend = pend;
-              k = 1;
-            }
-            unsigned long long s0 = 0;
-            uint32_t okr = 0;
-            const unsigned long long rmask = P.job_ring - 1;
-            if (lane == 0) {
-              // k <= waiting warps, so positions stay within one warp's worth
-              // of reservations per donor of pop_cnt: the slot of position p
-              // was last used by position p - ring, consumed long ago; wait
-              // (bounded) until its consumer has released it
-              atomicAdd(&P.sc->outstanding.v, (unsigned long long)k);
-              s0 = atomicAdd(&P.sc->push_cnt.v, (unsigned long long)k);
-              atomicAdd(&P.sc->donations, (unsigned long long)k);
-              okr = 1;
-              long long tw = clock64();
-              for (uint32_t r = 0; r < k && okr; ++r)
-                while (ld_volatile(P.job_seq[(s0 + r) & rmask]) != s0 + r) {
-                  if (clock64() - tw > P.timeout_cycles) {
-                    atomicOr(&P.sc->error, kErrTimeout);
-                    okr = 0;
-                    break;
-                  }
-                  __nanosleep(64);
-                }
-            }
-            okr = __shfl_sync(kFull, okr, 0);
-            s0 = __shfl_sync(kFull, s0, 0);
-            if (okr) {
-              // level p's pivot run 
-              const uint32_t pbase = pivot_base(p);
-              const uint32_t pchunk = __shfl_sync(kFull, lv_chunk, p);
-              const uint32_t fsrc = __shfl_sync(kFull, my_f, (lane - 8) & 31);
-              uint32_t bits = dmask;
-              for (uint32_t r = 0; r < k; ++r) {
-                uint32_t word = 0;
-                uint32_t cw = 0, jdepth, jlo = 0, jhi = 0;
-                if (pm) {
-                  uint32_t b = __ffs(bits) - 1;
-                  bits &= bits - 1;
-                  cw = P.g.arena[(uint64_t)pbase * 4 + pchunk + b];
-                  jdepth = p + 1;
-                } else {
-                  jdepth = p;
-                  jlo = rmid;
-                  jhi = rend;
-                }
-                if (lane == 0) word = upd;
-                else if (lane == 1) word = qo;
-                else if (lane == 2) word = jdepth;
-                else if (lane == 3) word = jlo;
-                else if (lane == 4) word = jhi;
-                else if (lane >= 8 && lane < 24) {
-                  uint32_t fi = lane - 8;
-                  word = fi < p ? fsrc : (fi == p && pm ? cw : 0u);
-                }
-                uint32_t *rec = reinterpret_cast<uint32_t *>(P.jobs + ((s0 + r) & rmask));
-                __stcg(rec + lane, word);
-              }
-              __threadfence();
-              __syncwarp();
-              if (lane < k) atomicExch(&P.job_seq[(s0 + lane) & rmask], s0 + lane + 1);
-              if (lane == p) {
-                if (pm) lv_mask &= ~dmask;
-                else lv_end = rmid;
-              }
-              if (p == L) {  // the donated piece came from the current level
-                if (pm) cur_mask &= ~dmask;
-                else cur_end = rmid;
-              }
-            }
-          }
-        }
-      }
-      continue;
-    }
-    // descend into the lowest pending candidate of level L
-    const uint32_t b = __ffs(cur_mask) - 1;
-    const uint32_t w = P.g.arena[(uint64_t)cur_base * 4 + cur_chunk + b];
-    cur_mask &= cur_mask - 1;
-    if (lane == L) {
-      lv_pos = cur_pos;
-      lv_end = cur_end;
-      lv_mask = cur_mask;
-      lv_chunk = cur_chunk;
-      my_f = w;
-      uint2 a = P.g.adj[w];
-      my_off = a.x;
-      my_deg = a.y;
-    }
-    ++L;
-    setup_level(L, 0, 0);
-  }
-  flush();
-}
-
 
 // phantom = 1 adds one outstanding task that nothing finishes (a test of the
 // bounded waits: the launch then ends only through their timeouts).
@@ -986,10 +743,8 @@ __global__ void k_sched_init(Sched *sc, const BatchHdr *hdr, unsigned long long 
   }
 }
 
-// kLM: label-major runs with slot offsets (the engine's graph); otherwise
-// plain id-sorted runs.
 template <bool kLM>
-__global__ void __launch_bounds__(256, kLM ? 4 : 5) k_match(MatchArgs P) {
+__global__ void __launch_bounds__(256, 4) k_match(MatchArgs P) {
   extern __shared__ __align__(16) uint32_t smem[];
   const uint32_t lane = threadIdx.x & 31;
   if (*P.abort_flag & kErrArena) return;  // the batch was refused before its insert
@@ -1034,10 +789,7 @@ __global__ void __launch_bounds__(256, kLM ? 4 : 5) k_match(MatchArgs P) {
       hi = __shfl_sync(kFull, word, 4);
       fval = __shfl_sync(kFull, word, (lane + 8) & 31);
     }
-    if constexpr (kLM)
-      run_task(P, bt, nupd, upd, qo, depth, lo, hi, fval, smem + (threadIdx.x >> 5) * warp_words(P.W));
-    else
-      run_task_plain(P, nupd, upd, qo, depth, lo, hi, fval);
+    run_task<kLM>(P, bt, nupd, upd, qo, depth, lo, hi, fval, smem + (threadIdx.x >> 5) * warp_words<kLM>(P.W));
     finish_task(P);
   }
 }
@@ -1063,25 +815,26 @@ void launch_sched_init(Sched *sc, const BatchHdr *hdr, unsigned long long *job_s
   k_sched_init<<<(job_ring + 255) / 256, 256, 0, s>>>(sc, hdr, job_seq, job_ring, phantom);
 }
 
+namespace {
+
+// Shared memory of a block, with the kernel's limit raised to it.
+template <bool kLM>
+int match_smem(uint32_t W) {
+  const int bytes = 8 * 4 * (int)warp_words<kLM>(W);
+  cudaFuncSetAttribute(k_match<kLM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return bytes;
+}
+
+}  // namespace
+
 void launch_match(const MatchArgs &a, int blocks, cudaStream_t s) {
-  if (!a.g.loff) {
-    k_match<false><<<blocks, 256, 0, s>>>(a);
-    return;
-  }
-  const int smem = 8 * 4 * (int)warp_words(a.W);
-  cudaFuncSetAttribute(k_match<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  k_match<true><<<blocks, 256, smem, s>>>(a);
+  if (a.g.loff) k_match<true><<<blocks, 256, match_smem<true>(a.W), s>>>(a);
+  else k_match<false><<<blocks, 256, match_smem<false>(a.W), s>>>(a);
 }
 
 int match_max_blocks_per_sm(uint32_t width) {
   int n = 0;
-  if (!width) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_match<false>, 256, 0);
-    return n;
-  }
-  const int smem = 8 * 4 * (int)warp_words(width);
-  cudaFuncSetAttribute(k_match<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_match<true>, 256, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_match<true>, 256, match_smem<true>(width));
   return n;
 }
 

@@ -51,24 +51,35 @@ constexpr size_t kScratchBytes = align256(kOffHdr + sizeof(BatchHdr) + 16);
 
 static __device__ __align__(256) unsigned char g_na_scratch[kScratchBytes];
 
-// Device address of g_na_scratch per device.  In host code the array's name
-// is only a host-side stand-in, so the address comes from
-// cudaGetSymbolAddress, once per device, with that device current.
+// Device address of g_na_scratch per device, with the device's SM count and
+// clock rate (asking the driver for the latter takes about a millisecond).  In
+// host code the array's name is only a host-side stand-in, so the address
+// comes from cudaGetSymbolAddress, once per device, with that device current.
+struct NaDevice {
+  unsigned char *scratch;
+  int sms, clock_khz;
+};
 std::mutex g_na_mu;
-unsigned char *g_na_addr[256] = {};
+NaDevice g_na_dev[256] = {};
 
-int scratch_of(int device, unsigned char **out) {
+int device_of(int device, NaDevice *out) {
   std::lock_guard<std::mutex> lk(g_na_mu);
   if (device < 0 || device >= 256) return DSM_ERR_ARG;
-  if (!g_na_addr[device]) {
+  NaDevice &d = g_na_dev[device];
+  if (!d.scratch) {
     void *p = nullptr;
     if (cudaGetSymbolAddress(&p, g_na_scratch) != cudaSuccess || !p) {
       cudaGetLastError();
       return DSM_ERR_CUDA;
     }
-    g_na_addr[device] = (unsigned char *)p;
+    int sms = 0, clk_khz = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaDeviceGetAttribute(&clk_khz, cudaDevAttrClockRate, device);
+    d.sms = std::max(sms, 1);
+    d.clock_khz = clk_khz > 0 ? clk_khz : 1965000;
+    d.scratch = (unsigned char *)p;
   }
-  *out = g_na_addr[device];
+  *out = d;
   return DSM_OK;
 }
 
@@ -111,8 +122,9 @@ extern "C" int dsm_count_edge_embeddings_noalloc(int device, uint32_t nv, const 
     cudaGetLastError();
     return done(DSM_ERR_CUDA);
   };
-  unsigned char *base = nullptr;
-  if ((rc = scratch_of(device, &base))) return done(rc);
+  NaDevice dev;
+  if ((rc = device_of(device, &dev))) return done(rc);
+  unsigned char *base = dev.scratch;
 
   // query descriptor, orders and the (label, label) -> ordered edge table
   QDev qd;
@@ -166,10 +178,7 @@ extern "C" int dsm_count_edge_embeddings_noalloc(int device, uint32_t nv, const 
   SeedArgs sa{g, dh, reinterpret_cast<const uint4 *>(d_updates), vtp, (const uint32_t *)(base + kOffPairOff),
               (const uint32_t *)(base + kOffPairEnt), (const QDev *)(base + kOffQd),
               (const OrderRec *)(base + kOffOrders), (uint4 *)(base + kOffSeeds), sc, kAllSlots, 0u, 0u, 0u};
-  int sms = 0, clk_khz = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  cudaDeviceGetAttribute(&clk_khz, cudaDevAttrClockRate, device);
-  launch_seeds(sa, std::max(sms, 1) * 4, s);
+  launch_seeds(sa, dev.sms * 4, s);
   launch_sched_init(sc, dh, seq, kNaRing, s);
 
   MatchArgs ma;
@@ -190,10 +199,11 @@ extern "C" int dsm_count_edge_embeddings_noalloc(int device, uint32_t nv, const 
   ma.cap = 0;
   ma.seg_count = (unsigned long long *)d_counts;
   ma.list = 0;
+  ma.pack_max = 1;  // partial embeddings in batches
   ma.donate = 1;
-  ma.timeout_cycles = 5000ll * (long long)(clk_khz > 0 ? clk_khz : 1965000);
-  int per_sm = std::max(1, std::min(match_max_blocks_per_sm(0), 4));
-  launch_match(ma, std::max(sms, 1) * per_sm, s);
+  ma.timeout_cycles = 5000ll * (long long)dev.clock_khz;
+  int per_sm = std::max(1, std::min(match_max_blocks_per_sm(nq), 4));
+  launch_match(ma, dev.sms * per_sm, s);
   if (cudaGetLastError() != cudaSuccess) return cuda_failed();
 
   unsigned int error = 0;

@@ -202,3 +202,38 @@ def test_without_room_for_the_edge_filter():
         for i in range(len(ups)):
             assert np.array_equal(r.tuples_of(qid, i), want[2][i])
         e.close()
+
+
+@pytest.mark.parametrize("m,r", [(1, 1), (31, 1), (33, 2), (64, 1), (65, 3), (900, 12), (3, 4000)])
+def test_plain_runs_count_alike(m, r):
+    """The allocation-free entry point on plain id-sorted runs: the same levels
+    around a batch, counted on the graph that has the edge."""
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    nv, labels, edges, ups = _layers(m, r, m * 100 + r)
+    both = np.concatenate([edges, edges[:, ::-1], ups[:1, 1:3], ups[:1, 2:0:-1]])
+    both = np.unique(both, axis=0)  # sorted by vertex, then neighbour
+    deg = np.bincount(both[:, 0], minlength=nv)
+    start = np.concatenate([[0], np.cumsum((deg + 3) // 4)])
+    arena = np.full(4 * int(start[-1]), 0xFFFFFFFF, np.uint32)
+    first = np.concatenate([[0], np.cumsum(deg)])
+    for v in range(nv):
+        arena[4 * start[v]:4 * start[v] + deg[v]] = both[first[v]:first[v + 1], 1]
+    dev = lambda x: torch.from_numpy(np.ascontiguousarray(x.astype(np.uint32)).view(np.int32)).cuda()
+    t_adj, t_arena = dev(np.stack([start[:-1], deg], 1)), dev(arena)
+    t_lab, t_ups = dev(labels), dev(ups[:1])
+    total = 0
+    for q in (PATH, CLOSED, TWO):
+        want = int(oracle_stream(nv, labels, edges, q).apply(ups[:1], listed=False)[1][0])
+        cnt = torch.full((1,), -1, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        rc = d.lib.dsm_count_edge_embeddings_noalloc(
+            C.c_int(0), C.c_uint32(nv), C.c_void_p(t_adj.data_ptr()), C.c_void_p(t_arena.data_ptr()),
+            C.c_void_p(t_lab.data_ptr()), C.c_void_p(q.offsets.ctypes.data), C.c_void_p(q.nbrs.ctypes.data),
+            C.c_void_p(q.labels.ctypes.data), C.c_uint32(q.nv), C.c_void_p(t_ups.data_ptr()), C.c_uint32(1),
+            C.c_void_p(cnt.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0
+        assert int(cnt[0]) == want
+        total += want
+    assert total > 0
