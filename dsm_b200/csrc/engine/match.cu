@@ -190,7 +190,9 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   unsigned long long task_cnt = 0, work = 0;  // warp-uniform
   uint32_t alg = 0;                           // bytes, this lane's share
   // what the segment had left of its work limit when this task last looked
-  // (at most 2^32 - 1): a task that alone exceeds it publishes at once
+  // (at most 2^32 - 1): a task that alone exceeds it publishes at once, but for
+  // a query with a listing budget, which the tuples listed until the heartbeat
+  // count towards
   uint32_t work_left = 0xFFFFFFFFu;
 
   // Listing reserves slots in the result table; a query past its listing
@@ -518,7 +520,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
         if (ok) put(t, cnt + __popc(m & lanemask_lt()), make_uint2(w, k));
         cnt += ns;
       }
-      if (P.work_limit && work >= work_left) {
+      if (P.work_limit && work >= work_left && (!P.qlimit || cnt_only)) {
         if (publish_work()) break;
       }
       if (hb >= 64) {
