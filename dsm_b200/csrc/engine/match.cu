@@ -132,7 +132,7 @@ __device__ void finish_task(const MatchArgs &P) {
 // each, where a search of a run takes 8 to 14 dependent ones, and most entries
 // are turned away (on a 2^24-edge power-law graph 27 of 32): those that pass
 // are gathered, and 32 of them searched together.  Three queries x 4096
-// updates on that graph 44 -> 31 ms, 256 queries x 1021 updates 34 -> 27 ms;
+// updates on that graph 44 -> 26 ms, 256 queries x 1021 updates 34 -> 24 ms;
 // where most entries pass (a hub-heavy graph with 8 labels) it neither gains
 // nor costs (15 ms).
 //
@@ -457,7 +457,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
           const uint32_t m = __ballot_sync(kFull, ok);
           if (ok) cand[nc + __popc(m & lanemask_lt())] = make_uint2(pos, w | (k << kIdBits));
           nc += __popc(m);
-          test = nc >= 32 || c >= e;
+          test = nc >= 32 || (c >= e && nc);
           __syncwarp();
         }
       }
@@ -471,55 +471,56 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
         k = ok ? x.y >> kIdBits : 0u;
         nc -= n;
       }
-      const uint32_t en = kLM ? (t_lab << kIdBits) | w : w;
-      ok = ok && test;
-      if (!kLM || t_lab >= 31)  // plain runs hold every label, slot 31 every label >= 31
-        ok = ok && ((P.g.lab[w] & kLabelMask) == t_lab);
-      // injectivity: only earlier positions with the same label can hold w
-      for (uint32_t same = t_same; same; same &= same - 1) ok = ok && w != F[__ffs(same) - 1][k];
-      if (bitmap) {
-        const uint32_t qv = (__shfl_sync(kFull, q_word, t) >> 21) & 15u;
-        ok = ok && ((bitmap[(size_t)qv * Q.col_len + (w >> 5)] >> (w & 31)) & 1u);
-      }
-      uint32_t r = 0;
-      for (uint32_t bits = t_bn; bits; bits &= bits - 1, ++r) {
-        if (!ok) continue;
-        const uint32_t j = __ffs(bits) - 1;
-        uint4 row;
-        if (r < kRows) {
-          row = rows[r][k];
-        } else {
-          const uint32_t x = F[j][k];
-          if constexpr (kLM) {
-            const uint32_t *o = P.g.loff + (size_t)x * (P.g.nlt + 1) + t_lab;
-            row = make_uint4(P.g.adj[x].x, o[0], o[1], P.g.lab[x] >> 31);
+      if (test) {
+        const uint32_t en = kLM ? (t_lab << kIdBits) | w : w;
+        if (!kLM || t_lab >= 31)  // plain runs hold every label, slot 31 every label >= 31
+          ok = ok && ((P.g.lab[w] & kLabelMask) == t_lab);
+        // injectivity: only earlier positions with the same label can hold w
+        for (uint32_t same = t_same; same; same &= same - 1) ok = ok && w != F[__ffs(same) - 1][k];
+        if (bitmap) {
+          const uint32_t qv = (__shfl_sync(kFull, q_word, t) >> 21) & 15u;
+          ok = ok && ((bitmap[(size_t)qv * Q.col_len + (w >> 5)] >> (w & 31)) & 1u);
+        }
+        uint32_t r = 0;
+        for (uint32_t bits = t_bn; bits; bits &= bits - 1, ++r) {
+          if (!ok) continue;
+          const uint32_t j = __ffs(bits) - 1;
+          uint4 row;
+          if (r < kRows) {
+            row = rows[r][k];
           } else {
-            const uint2 a = P.g.adj[x];
-            row = make_uint4(a.x, 0, a.y, 0);
+            const uint32_t x = F[j][k];
+            if constexpr (kLM) {
+              const uint32_t *o = P.g.loff + (size_t)x * (P.g.nlt + 1) + t_lab;
+              row = make_uint4(P.g.adj[x].x, o[0], o[1], P.g.lab[x] >> 31);
+            } else {
+              const uint2 a = P.g.adj[x];
+              row = make_uint4(a.x, 0, a.y, 0);
+            }
+          }
+          if (r != piv[k].z) {
+            ok = run_has(P.g.arena + (uint64_t)row.x * 4 + row.y, row.z - row.y, en);
+            alg += 4;
+          }
+          // liveness: only edges of a touched vertex can have changed, and of
+          // those the filter turns away all that the batch does not change
+          if (kLM && ok && row.w) {
+            const uint32_t x = F[j][k];
+            if (may_change(bt, x, w)) ok = edge_live(bt, x, w, tp);
           }
         }
-        if (r != piv[k].z) {
-          ok = run_has(P.g.arena + (uint64_t)row.x * 4 + row.y, row.z - row.y, en);
-          alg += 4;
-        }
-        // liveness: only edges of a touched vertex can have changed, and of
-        // those the filter turns away all that the batch does not change
-        if (kLM && ok && row.w) {
-          const uint32_t x = F[j][k];
-          if (may_change(bt, x, w)) ok = edge_live(bt, x, w, tp);
+        const uint32_t m = __ballot_sync(kFull, ok);
+        const uint32_t ns = __popc(m);
+        work += ns;
+        if (t == nq - 1) {
+          emit(m, w, t, k);
+        } else if (m && !(P.bfs_stop == t + 1 && write_rows(m, w, k))) {
+          if (ok) put(t, cnt + __popc(m & lanemask_lt()), make_uint2(w, k));
+          cnt += ns;
         }
       }
-      const uint32_t m = __ballot_sync(kFull, ok);
-      const uint32_t ns = __popc(m);
-      work += ns;
       ++hb;
       ++dticks;
-      if (t == nq - 1) {
-        emit(m, w, t, k);
-      } else if (m && !(P.bfs_stop == t + 1 && write_rows(m, w, k))) {
-        if (ok) put(t, cnt + __popc(m & lanemask_lt()), make_uint2(w, k));
-        cnt += ns;
-      }
       if (P.work_limit && work >= work_left && (!P.qlimit || cnt_only)) {
         if (publish_work()) break;
       }
