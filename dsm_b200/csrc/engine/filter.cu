@@ -227,43 +227,68 @@ __device__ __forceinline__ unsigned long long range_entry(const BlockRanges &R, 
 
 // Full runs: one op over every current candidate of its core vertex.
 //
-// Bound by the gathers and marks of the receivers.  Only neighbours of the
-// labels the leaf rule can change are visited (leaf_slots: one contiguous
-// range each of the label-major run).  A block takes 256 vertices, one a
-// thread, lays the candidates' ranges of one label end to end (a block scan of
-// their lengths) and gives each thread one entry in turn, its owner found by
-// eight steps through the scan: a hub's range is then shared by the block,
-// where one warp walked the hub's whole run before and the launch waited for
-// it.  2^20 vertices, 2^24 edges (R-MAT), one op: 635 -> 46 us.
+// Bound by the latency of the steps (candidates, offsets, scan, entries,
+// receivers): few vertices are candidates.  Only neighbours of the labels the
+// leaf rule can change are visited (leaf_slots: one contiguous range each of
+// the label-major run).  A block looks through 1024 vertices at a time and
+// gathers the candidates; 256 of them, or the last, a thread each, have their
+// ranges of one label laid end to end (a block scan of their lengths), and each
+// thread takes one entry in turn, its owner found by eight steps through the
+// scan: a hub's range is then shared by the block, where one warp walked the
+// hub's whole run before and the launch waited for it.  2^20 vertices, 2^24
+// edges (R-MAT), one op: 635 us; 46 us with the ranges of every 256 vertices
+// laid out, most of them no candidates; 33 us so.
+constexpr uint32_t kOpTile = 1024;
 __global__ void __launch_bounds__(256) k_filter_op(DevGraph g, const FilterDevice *F, uint32_t k) {
   const FilterDevice f = F[blockIdx.y];
   if (k >= f.nops || !f.desc->full_now) return;
   __shared__ BlockRanges R;
+  __shared__ uint32_t s_cand[256 + kOpTile];
+  __shared__ uint32_t s_n;
   const DevFilterOp &op = f.ops[k];
-  const uint32_t t = threadIdx.x, cu = op.core_u, words = f.words;
-  for (uint32_t base = blockIdx.x * 256; base < g.nv; base += gridDim.x * 256) {
-    const uint32_t v = base + t;
-    const bool isc = v < g.nv && ((f.valid[v] >> cu) & 1u);
-    if (!__syncthreads_or(isc)) continue;
-    uint32_t off = 0;
-    if (isc) {
-      core_rule(op, v, f.valid, f.enc, words);
-      off = g.adj[v].x;
+  const uint32_t t = threadIdx.x, lane = t & 31, cu = op.core_u, words = f.words;
+  if (t == 0) s_n = 0;
+  __syncthreads();
+  for (uint32_t base = blockIdx.x * kOpTile; base < g.nv; base += gridDim.x * kOpTile) {
+    const bool last = base + gridDim.x * kOpTile >= g.nv || base + gridDim.x * kOpTile < base;
+#pragma unroll
+    for (uint32_t i = 0; i < kOpTile; i += 256) {
+      const uint32_t v = base + i + t;
+      const bool isc = v < g.nv && ((f.valid[v] >> cu) & 1u);
+      const uint32_t m = __ballot_sync(kFull, isc);
+      uint32_t at = 0;
+      if (m && lane == 0) at = atomicAdd(&s_n, (uint32_t)__popc(m));
+      at = __shfl_sync(kFull, at, 0);
+      if (isc) s_cand[at + __popc(m & lanemask_lt())] = v;
     }
-    for (uint32_t sm = op.leaf_slots; sm; sm &= sm - 1) {
-      const uint32_t sl = __ffs(sm) - 1;
-      if (sl >= g.nlt) break;  // no vertex has a label of this slot or a later one
-      uint32_t a = 0, len = 0;
+    __syncthreads();
+    for (uint32_t n = s_n; n >= 256 || (last && n); ) {
+      const uint32_t take = min(n, 256u);
+      n -= take;
+      const bool isc = t < take;
+      const uint32_t v = isc ? s_cand[n + t] : 0u;
+      uint32_t off = 0;
       if (isc) {
-        const uint32_t *lo = g.loff + (size_t)v * (g.nlt + 1) + sl;
-        a = lo[0];
-        len = lo[1] - a;
+        core_rule(op, v, f.valid, f.enc, words);
+        off = g.adj[v].x;
       }
-      const uint32_t total = lay_ranges(R, (unsigned long long)off * 4 + a, len);
-      for (uint32_t e = t; e < total; e += 256)
-        leaf_rule(op, g.arena[range_entry(R, e)] & kIdMask, f.vcand, f.enc, words);
-      __syncthreads();
+      for (uint32_t sm = op.leaf_slots; sm; sm &= sm - 1) {
+        const uint32_t sl = __ffs(sm) - 1;
+        if (sl >= g.nlt) break;  // no vertex has a label of this slot or a later one
+        uint32_t a = 0, len = 0;
+        if (isc) {
+          const uint32_t *lo = g.loff + (size_t)v * (g.nlt + 1) + sl;
+          a = lo[0];
+          len = lo[1] - a;
+        }
+        const uint32_t total = lay_ranges(R, (unsigned long long)off * 4 + a, len);
+        for (uint32_t e = t; e < total; e += 256)
+          leaf_rule(op, g.arena[range_entry(R, e)] & kIdMask, f.vcand, f.enc, words);
+        __syncthreads();
+      }
+      if (t == 0) s_n = n;
     }
+    __syncthreads();
   }
 }
 
@@ -391,16 +416,18 @@ __global__ void k_region_seed(DevGraph g, RegionDevice rg, const uint32_t *hdr_n
 __global__ void k_region_close(RegionInfo *I, uint32_t hop) { I->bound[hop] = min(I->total, I->cap); }
 
 // Hop `hop`: every neighbour of the vertices first reached at hop - 1.  A
-// block shares the runs of 256 of them (a warp per run left the launch waiting
-// for the warps that had drawn the hubs).
+// block shares the runs of up to 256 of them, fewer while there are blocks
+// without any (a warp per run left the launch waiting for the warps that had
+// drawn the hubs, and one block for the first hop's 256 vertices for that block).
 __global__ void __launch_bounds__(256) k_region_expand(DevGraph g, RegionDevice rg, uint32_t hop) {
   __shared__ BlockRanges R;
   const RegionInfo &I = *rg.info;
   if (I.ov_round < 64) return;  // the list is full: queries that far out run in full
   const uint32_t lo = hop >= 2 ? I.bound[hop - 2] : 0u, hi = I.bound[hop - 1];
   const uint32_t t = threadIdx.x, epoch = I.epoch;
-  for (uint32_t base = lo + blockIdx.x * 256; base < hi; base += gridDim.x * 256) {
-    const uint2 av = base + t < hi ? g.adj[rg.list[base + t]] : make_uint2(0, 0);
+  const uint32_t tile = min((hi - lo + gridDim.x - 1) / gridDim.x, 256u);
+  for (uint32_t base = lo + blockIdx.x * tile; base < hi; base += gridDim.x * tile) {
+    const uint2 av = t < tile && base + t < hi ? g.adj[rg.list[base + t]] : make_uint2(0, 0);
     const uint32_t total = lay_ranges(R, (unsigned long long)av.x * 4, av.y);
     for (uint32_t e = t; e < total; e += 256) {
       claim(rg, epoch, g.arena[range_entry(R, e)] & kIdMask, hop);
