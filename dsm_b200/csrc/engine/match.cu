@@ -32,6 +32,14 @@ __device__ __forceinline__ T ld_volatile(const T &x) {
 }
 
 constexpr unsigned long long kSeqDone = 1ull << 63;
+// Partial embeddings between heartbeats when tuples count towards a listing
+// budget: those listed before a search is found over its limit count, so a
+// later stop lists fewer queries, an earlier one more.  Against one partial at
+// a time (a heartbeat every 64 chunks) over 156 batches, queries listed more /
+// fewer: chunks alone 55 / 684, 640 252 / 442, 576 304 / 398, 400 717 / 187,
+// 256 1383 / 37; two runs of one build differ by 110 / 106.  One listed request
+// on 2^24 edges: 7.3 -> 6.7 ms; a count keeps 64 chunks.
+constexpr uint32_t kListBeat = 576;
 
 // Lane 0 only.  Returns 1 (seed `slot`), 2 (job of ticket `slot`; the caller
 // releases the ring slot after reading it) or 0 (no more work).
@@ -424,6 +432,9 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
     c = e;
   }
   uint32_t hb = 0;     // chunks since the last heartbeat
+  // tuples count towards a listing budget until the search is found over its
+  // limit: heartbeats by partial embeddings too
+  const bool beat = P.work_limit && P.qlimit && P.list;
   int32_t dticks = 0;  // chunks since the last donation check (below zero: none for a while)
   uint32_t nc = 0;  // candidates that passed the edge filter
   while (true) {
@@ -524,7 +535,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
       if (P.work_limit && work >= work_left && (!P.qlimit || cnt_only)) {
         if (publish_work()) break;
       }
-      if (hb >= 64) {
+      if (hb >= 64 || (beat && work >= kListBeat)) {
         hb = 0;
         unsigned int err = 0;
         if (lane == 0) {
