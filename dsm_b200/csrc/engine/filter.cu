@@ -422,7 +422,9 @@ __global__ void k_region_close(RegionInfo *I, uint32_t hop) { I->bound[hop] = mi
 __global__ void __launch_bounds__(256) k_region_expand(DevGraph g, RegionDevice rg, uint32_t hop) {
   __shared__ BlockRanges R;
   const RegionInfo &I = *rg.info;
-  if (I.ov_round < 64) return;  // the list is full: queries that far out run in full
+  // The list is full: queries that far out run in full.  Other blocks of this
+  // launch may lower the word meanwhile, so the block decides as one.
+  if (__syncthreads_or(*(volatile const uint32_t *)&rg.info->ov_round < 64)) return;
   const uint32_t lo = hop >= 2 ? I.bound[hop - 2] : 0u, hi = I.bound[hop - 1];
   const uint32_t t = threadIdx.x, epoch = I.epoch;
   const uint32_t tile = min((hi - lo + gridDim.x - 1) / gridDim.x, 256u);

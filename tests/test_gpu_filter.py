@@ -205,3 +205,38 @@ def test_filter_at_the_edges_of_its_tiles(nv, labels_to):
         ql = np.minimum(labels[rng.integers(0, nv, nq)], 31)
         qs.append(d.Query.from_edges(ql, sorted(tree)))
     _filter_case(nv, labels, np.array(sorted(edges), np.uint32), qs)
+
+
+@pytest.mark.parametrize("first,fan", [(64_000, 4), (65_530, 4), (65_537, 1), (70_000, 1), (30_000, 3)])
+def test_region_list_fills_within_a_hop(first, fan):
+    """The region's list (65,536 vertices here) fills while a hop is being
+    expanded: by the hub's own neighbours, or by theirs with the list nearly
+    full before; the last case fits.  The state equals a full recompute."""
+    rng = np.random.default_rng(first + fan)
+    nv = 100_000
+    labels = rng.integers(0, 3, nv).astype(np.uint32)
+    labels[0] = 0
+    near = 1 + rng.permutation(nv - 1)[:first]
+    rest = np.setdiff1d(np.arange(1, nv), near)
+    out = np.repeat(near, fan)
+    edges = np.concatenate([np.stack([np.zeros_like(near), near], 1),
+                            np.stack([out, rest[rng.integers(0, len(rest), len(out))]], 1)]).astype(np.uint32)
+    qs = [d.Query.from_edges([0, 1, 2, 1, 2], [(0, 1), (1, 2), (2, 3), (0, 4), (0, 2)]),
+          d.Query.from_edges([1, 0, 2], [(0, 1), (1, 2)])]
+
+    class W:
+        pass
+
+    w = W()
+    w.nv, w.labels, w.edges = nv, labels, edges
+    inc, full = _inc_pair(w, qs)
+    for e, _ in (inc, full):
+        e.set_option(d.OPT_LIST, 0)
+        e.set_option(d.OPT_WORK_LIMIT, 1000)
+    for k in range(4):
+        b = np.array([[k & 1, 0, near[0], 0], [1, 0, rest[k], 0]], np.uint32)
+        for e, _ in (inc, full):
+            e.run_batch(b)
+        _same_state(inc, full, qs, nv, f"batch {k}")
+    for e, _ in (inc, full):
+        e.close()
