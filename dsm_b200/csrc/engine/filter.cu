@@ -262,7 +262,9 @@ __global__ void __launch_bounds__(256) k_filter_op(DevGraph g, const FilterDevic
       if (isc) s_cand[at + __popc(m & lanemask_lt())] = v;
     }
     __syncthreads();
-    for (uint32_t n = s_n; n >= 256 || (last && n); ) {
+    uint32_t n = s_n;
+    __syncthreads();  // every thread has it: below, an op without leaf ranges meets no barrier before it changes
+    while (n >= 256 || (last && n)) {
       const uint32_t take = min(n, 256u);
       n -= take;
       const bool isc = t < take;

@@ -240,3 +240,43 @@ def test_region_list_fills_within_a_hop(first, fan):
         _same_state(inc, full, qs, nv, f"batch {k}")
     for e, _ in (inc, full):
         e.close()
+
+
+@pytest.mark.parametrize("tiles,extra", [(1, 0), (1, 1), (1, 1025), (2, 300)])
+def test_filter_ops_carry_candidates_from_tile_to_tile(tiles, extra):
+    """16 queries leave an SM's worth of blocks for each, so a block looks
+    through several tiles of 1024 vertices and carries fewer than 256
+    candidates from one to the next: tiles of 0 to 1024 candidates, around 256
+    of them in sum, against the oracle."""
+    torch = pytest.importorskip("torch")
+    stride = 1024 * torch.cuda.get_device_properties(0).multi_processor_count
+    nv = tiles * stride + extra
+    rng = np.random.default_rng(nv)
+    per_tile = np.array([0, 1, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1024])
+    v = np.arange(nv)
+    core = v % 1024 < per_tile[(v // 1024 + v // stride * 5) % len(per_tile)]
+    labels = np.where(core, 0, 1 + rng.integers(0, 2, nv)).astype(np.uint32)
+    of = [np.nonzero(labels == k)[0] for k in range(3)]
+    ends = lambda a, k: np.stack([a, of[k][rng.integers(0, len(of[k]), len(a))]], 1)
+    keep = rng.random(len(of[0])) < 0.9  # the others are no candidates of a vertex with both neighbours
+    edges = np.concatenate([ends(of[0], 1), ends(of[0][keep], 2), ends(of[1], 2), ends(of[0][::3], 0)])
+    edges = edges[edges[:, 0] != edges[:, 1]].astype(np.uint32)
+    shapes = [(3, [(0, 1), (0, 2)]), (4, [(0, 1), (0, 2), (1, 3)]), (4, [(0, 1), (1, 2), (2, 3), (0, 3)]),
+              (5, [(0, 1), (0, 2), (1, 3), (2, 4)])]
+    qs = [d.Query.from_edges([0, 1, 2, 0, 1][:n] if k % 4 == 0 else rng.permutation([0, 0, 1, 1, 2])[:n], es)
+          for k in range(4) for n, es in shapes]
+    e = d.Engine(0)
+    e.set_option(d.OPT_FILTER, 2)
+    e.set_option(d.OPT_LIST, 0)
+    e.set_option(d.OPT_WORK_LIMIT, 100)
+    e.load_graph_edges(nv, labels, edges)
+    qids = [e.register(q) for q in qs]
+    e.run_batch(np.array([[1, *edges[0], 0]], np.uint32))  # there already: the filter's graph is the one loaded
+    off, nb = e.export_graph()
+    for qid, q in zip(qids, qs):
+        bm, vc, (full, _) = e.filter_state(qid, q.nv, nv)
+        obm, ovc, _, _ = orc.cluster_filter(q.labels, q.offsets, q.nbrs, nv, labels, off, nb)
+        assert full and np.array_equal(vc, ovc)
+        assert np.array_equal(bm, obm), f"query {qid}: bitmaps differ at u {np.nonzero((bm != obm).any(1))[0]}"
+    assert any(b.any() for b in obm)
+    e.close()
