@@ -678,6 +678,7 @@ int Engine::finish_device(Staged &S) {
     std::string key;
     key_append(key, au);
     key_append(key, pk);
+    key_append(key, d_upd.ptr);  // grows with the updates; what au holds, with those that are no self loops
     key_append(key, blocks);
     if (int rc = run_segment(1, key, seg_b)) return rc;
   } else if (int rc = seg_b()) {

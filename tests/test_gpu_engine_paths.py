@@ -288,3 +288,24 @@ def test_breadth_first_rows_agree(cfg, scale, nqs, form):
     assert np.array_equal(got[~fe], c[~fo])
     for i in range(len(bb)):
         assert np.array_equal(r.tuples_of(qids[0], i), t[i] if not fo[i] else t[i][:0]), f"update {i}"
+
+
+def test_graph_replay_when_only_the_updates_outgrow_their_buffer():
+    """Self loops count as updates and not as keys: with them the update array
+    alone grows, and both captured segments are captured anew."""
+    rng = np.random.default_rng(5)
+    nv = 60
+    edges = np.array([(a, b) for a in range(nv) for b in range(a) if rng.random() < 0.2], np.uint32)
+    labels = rng.integers(0, 2, nv).astype(np.uint32)
+    q = d.Query.from_edges([0, 1, 0], [(0, 1), (1, 2)])
+    e, (qid,) = _fresh(nv, labels, edges, [q], OPT_GRAPH=1)
+    st = oracle_stream(nv, labels, edges, q)
+    captures = []
+    for loops in (0, 1, 9, 60, 9):  # 48 keys each; 49 updates no longer fit the 768 bytes of 48
+        a = rng.integers(0, nv, 48 + loops)
+        b = np.where(np.arange(48 + loops) < 48, (a + 1 + rng.integers(0, nv - 1, 48 + loops)) % nv, a)
+        ups = np.stack([rng.integers(0, 2, 48 + loops), a, b, 0 * a], 1).astype(np.uint32)
+        run_stream(e, [qid], [st], [rng.permutation(ups)], check_graph_every=1)
+        captures.append(e.stats()["graph_captures"])
+    assert captures[0] == 2 and captures[1] == 4
+    e.close()
