@@ -22,6 +22,7 @@ constexpr uint32_t kIdBits = 27;
 constexpr uint32_t kIdMask = (1u << kIdBits) - 1;
 constexpr uint32_t kMaxVertices = 1u << kIdBits;
 constexpr uint32_t kSlots = 32;
+constexpr uint32_t kMaxWidth = 16;  // query vertices
 __host__ __device__ __forceinline__ uint32_t label_slot(uint32_t label) { return label < 31 ? label : 31; }
 __host__ __device__ __forceinline__ uint32_t pack_entry(uint32_t label, uint32_t v) {
   return (label_slot(label) << kIdBits) | v;

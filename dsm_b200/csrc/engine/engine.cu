@@ -158,6 +158,8 @@ int Engine::init(int dev, size_t mem_budget) {
   list_limit_bytes = std::min<uint64_t>(list_limit_bytes, budget / 4);
   ev_pool.resize(8, nullptr);
   for (auto &ev : ev_pool) CK(cudaEventCreate(&ev));
+  CK(match_prepare());
+  CK(list_prepare());
   int per_sm = match_max_blocks_per_sm(4);
   match_blocks_per_sm = std::max(1, std::min(per_sm, 8));
   // small fixed buffers

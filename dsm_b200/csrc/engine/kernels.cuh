@@ -177,6 +177,12 @@ struct MatchArgs {
 // finishes: a test hook), every ring slot free for its first position.
 void launch_sched_init(Sched *sc, const BatchHdr *hdr, unsigned long long *job_seq, uint32_t job_ring,
                        cudaStream_t s, uint32_t phantom = 0);
+// Raises the matcher's shared-memory limit on the current device to what the
+// widest query takes.  The limit belongs to the kernel and the device, not to a
+// caller: set to one value by all of them, before their first launch, nobody
+// lowers it for another (a limit set to each launch's own bytes let an engine
+// of narrow queries fail the launch of one with wide ones in another thread).
+cudaError_t match_prepare();
 void launch_match(const MatchArgs &a, int blocks, cudaStream_t s);
 // Between the two launches of a breadth-first plan: the scheduler restarts
 // with the rows written so far as its tasks (counters of work done, the
@@ -186,6 +192,7 @@ void launch_rows_arm(Sched *sc, const unsigned long long *rows_cnt, unsigned lon
 int match_max_blocks_per_sm(uint32_t width);
 
 // Listed results in canonical order on the device (list.cu).
+cudaError_t list_prepare();  // as match_prepare, for the sort
 constexpr uint32_t kListBlocks = 256;
 struct ListArgs {
   const BatchHdr *hdr;              // n, nseg

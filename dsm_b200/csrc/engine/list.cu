@@ -309,7 +309,14 @@ __global__ void __launch_bounds__(256) k_list_merge(ListArgs A, const uint32_t *
   }
 }
 
+// Shared memory of a sort block for tuples of up to W words.
+constexpr int sort_smem(uint32_t W) { return (int)(kChunk * 2 + kChunk * (W | 1) * 4); }
+
 }  // namespace
+
+cudaError_t list_prepare() {
+  return cudaFuncSetAttribute(k_list_sort_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_smem(kMaxWidth));
+}
 
 int launch_list_scan(const ListArgs &a, size_t nseg, cudaStream_t s) {
   if (nseg && nseg <= 2048) {  // eight rounds of one block: no longer than the launch it saves (4 us)
@@ -336,9 +343,7 @@ int launch_list_sort(const ListArgs &a, uint32_t W, unsigned long long nseg, uns
   int passes = 0;
   for (unsigned long long run = kChunk; run < most; run *= 2) ++passes;
   // the last pass ends in `out`
-  const size_t smem = kChunk * 2 + (size_t)kChunk * (W | 1) * 4;
-  cudaFuncSetAttribute(k_list_sort_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_list_sort_chunks<<<(unsigned)chunks, 256, smem, s>>>(a, out, passes & 1 ? scratch : out);
+  k_list_sort_chunks<<<(unsigned)chunks, 256, sort_smem(W), s>>>(a, out, passes & 1 ? scratch : out);
   ++launched;
   uint32_t *src = passes & 1 ? scratch : out, *dst = passes & 1 ? out : scratch;
   unsigned long long run = kChunk;

@@ -831,15 +831,21 @@ void launch_sched_init(Sched *sc, const BatchHdr *hdr, unsigned long long *job_s
 
 namespace {
 
-// Shared memory of a block, with the kernel's limit raised to it.
+// Shared memory of a block for queries of up to W vertices.
 template <bool kLM>
-int match_smem(uint32_t W) {
-  const int bytes = 8 * 4 * (int)warp_words<kLM>(W);
-  cudaFuncSetAttribute(k_match<kLM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  return bytes;
+constexpr int match_smem(uint32_t W) {
+  return 8 * 4 * (int)warp_words<kLM>(W);
 }
 
 }  // namespace
+
+cudaError_t match_prepare() {
+  const cudaError_t e = cudaFuncSetAttribute(k_match<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             match_smem<true>(kMaxWidth));
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_match<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              match_smem<false>(kMaxWidth));
+}
 
 void launch_match(const MatchArgs &a, int blocks, cudaStream_t s) {
   if (a.g.loff) k_match<true><<<blocks, 256, match_smem<true>(a.W), s>>>(a);

@@ -68,7 +68,7 @@ int device_of(int device, NaDevice *out) {
   NaDevice &d = g_na_dev[device];
   if (!d.scratch) {
     void *p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_na_scratch) != cudaSuccess || !p) {
+    if (cudaGetSymbolAddress(&p, g_na_scratch) != cudaSuccess || !p || match_prepare() != cudaSuccess) {
       cudaGetLastError();
       return DSM_ERR_CUDA;
     }
