@@ -477,6 +477,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
         const uint2 x = cand[lane], y = cand[32 + lane];
         __syncwarp();
         if (32 + lane < nc) cand[lane] = y;
+        __syncwarp();  // the descent reads the first of the rest, the next chunk writes behind them
         ok = lane < n;
         w = x.y & kIdMask;
         k = ok ? x.y >> kIdBits : 0u;
