@@ -153,6 +153,11 @@ __device__ void finish_task(const MatchArgs &P) {
 // per partial, 64 candidates (position in the ranges, id | owner << 27), and a
 // buffer of 64 survivors per level (id | parent << 27; plain runs, whose ids may
 // take all 32 bits, keep the parents behind the ids).
+//
+// Entries of a batch are counted in 32 bits: 32 ranges of an engine's graph hold
+// fewer than 2^32 (its ids have 27 bits); of plain runs' partials those are
+// taken whose ranges do.
+constexpr uint32_t kPast = 0xFFFFFFFFu;  // no run is as long: a vertex has fewer neighbours than there are ids
 constexpr uint32_t kRows = 3;  // backward neighbours with stored ranges; further ones are read when needed
 template <bool kLM>
 __host__ __device__ constexpr uint32_t warp_words(uint32_t W) {
@@ -281,6 +286,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   const uint32_t most = P.pack_max ? 32u : 1u;  // partials expanded together
 
   // The ranges of E(l)'s partials (F holds the batch); returns their total.
+  // Plain runs: may make the batch smaller, so that the total fits.
   auto setup = [&]() -> uint32_t {
     const uint32_t tw = __shfl_sync(kFull, q_word, l + 1);
     t_bn = tw & 0xFFFFu;
@@ -317,7 +323,15 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
 #pragma unroll
     for (uint32_t d = 1; d < 32; d <<= 1) {
       const uint32_t x = __shfl_up_sync(kFull, incl, d);
-      if (lane >= d) incl += x;
+      if (lane >= d) incl = kLM || incl + x >= x ? incl + x : kPast;
+    }
+    if constexpr (!kLM) {  // the partials from which on the sum does not fit stay in the buffer (the first fits)
+      const uint32_t fit = __popc(__ballot_sync(kFull, incl != kPast));
+      if (fit < nb) {
+        nb = fit;
+        incl = min(incl, __shfl_sync(kFull, incl, nb - 1));
+        if (lane >= nb) len = 0;
+      }
     }
     const uint64_t start = (uint64_t)poff * 4 + pa - (incl - len);  // entry i of the scan is arena[start + i]
     piv[lane] = make_uint4((uint32_t)start, (uint32_t)(start >> 32), pr, pa);
@@ -445,7 +459,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
       uint32_t k = 0, w = 0;
       if (!two || (nc < 32 && c < e)) {  // a chunk of the ranges
         const uint32_t pos = c + lane;
-        ok = pos < e;
+        ok = lane < e - c;
 #pragma unroll
         for (uint32_t d = 16; d; d >>= 1) {  // the owner: the first lane with incl > pos
           const uint32_t v = __shfl_sync(kFull, incl, k + d - 1);
@@ -457,7 +471,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
           if constexpr (kLM) w &= kIdMask;
           alg += 4;
         }
-        c = min(c + 32, e);
+        c = e - c > 32 ? c + 32 : e;
         if (two) {
           uint32_t r = 0;
           for (uint32_t bits = t_bn; bits; bits &= bits - 1, ++r)
@@ -566,7 +580,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
           const uint32_t wait = ((lv_n >> 8) & 0xFFu) - (lane < l ? above : 0u);
           const bool has = lane + 1 >= depth && lane <= l &&
                            ((wait && lane + 1 + dd < nq) ||
-                            ((lv_n >> 16) && lane + dd < nq) || lv_e >= lv_c + split_min);
+                            ((lv_n >> 16) && lane + dd < nq) || lv_e - lv_c >= split_min);
           const uint32_t hm = __ballot_sync(kFull, has);
           if (hm) {
             __syncwarp();  // the survivors in the buffers are visible to every lane
@@ -605,7 +619,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
                 }
                 ecut = __shfl_sync(kFull, excl, __ffs(um) - 1);
                 todo -= jobs;
-              } else if (ei >= ci + split_min) {
+              } else if (ei - ci >= split_min) {
                 // half of what is left, a job for each partial it reaches into
                 // (the last ones, when fewer warps wait)
                 uint32_t mid = ci + (((ei - ci) / 2 + 31) & ~31u);

@@ -237,3 +237,42 @@ def test_plain_runs_count_alike(m, r):
         assert int(cnt[0]) == want
         total += want
     assert total > 0
+
+
+@pytest.mark.parametrize("fill", [(1 << 27) - 200, (1 << 27) + 5])
+def test_plain_runs_of_more_entries_than_32_bits_count(fill):
+    """A hub whose run, 32 times over, holds just under and just over 2^32
+    entries: 40 partials at the hub, each with the hub's run as its pivot.
+    The fillers' label is in no query, so the count is that of the graph
+    without them."""
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    q = d.Query.from_edges([0, 5, 1, 2], [(0, 1), (0, 2), (0, 3)])
+    small = np.array([0, 5] + [1] * 40 + [2] * 40, np.uint32)
+    spokes = np.array([(0, k) for k in range(2, 82)], np.uint32)
+    want = int(oracle_stream(82, small, spokes, q).apply(np.array([[1, 0, 1, 0]], np.uint32), listed=False)[1][0])
+    assert want == 1600
+    # ids: fillers, 40 + 40 + 1 neighbours that count, the hub; runs: the hub's, then {hub}, which all others share
+    nv = fill + 82
+    hub, deg = nv - 1, nv - 1
+    i32 = dict(dtype=torch.int32, device="cuda")
+    t_lab = torch.full((nv,), 3, **i32)
+    t_lab[fill:] = torch.tensor([1] * 40 + [2] * 40 + [5, 0], **i32)
+    unit = (deg + 3) // 4
+    t_arena = torch.zeros(4 * unit + 4, **i32)
+    t_arena[:deg] = torch.arange(deg, **i32)
+    t_arena[4 * unit] = hub
+    t_adj = torch.empty((nv, 2), **i32)
+    t_adj[:, 0], t_adj[:, 1] = unit, 1
+    t_adj[hub, 0], t_adj[hub, 1] = 0, deg
+    t_ups = torch.tensor([[1, hub, nv - 2, 0]], **i32)
+    cnt = torch.full((1,), -1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    rc = d.lib.dsm_count_edge_embeddings_noalloc(
+        C.c_int(0), C.c_uint32(nv), C.c_void_p(t_adj.data_ptr()), C.c_void_p(t_arena.data_ptr()),
+        C.c_void_p(t_lab.data_ptr()), C.c_void_p(q.offsets.ctypes.data), C.c_void_p(q.nbrs.ctypes.data),
+        C.c_void_p(q.labels.ctypes.data), C.c_uint32(q.nv), C.c_void_p(t_ups.data_ptr()), C.c_uint32(1),
+        C.c_void_p(cnt.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    assert int(cnt[0]) == want
