@@ -194,8 +194,14 @@ __device__ __forceinline__ void leaf_rule(const DevFilterOp &op, uint32_t n, con
 }
 
 // The ranges of a block's 256 vertices (thread t: len entries from arena word
-// `first`) laid end to end: s_incl is the inclusive scan of the lengths, entry
-// e of the total lies at arena word s_start[o] + e for its owner o.
+// `first`) laid end to end: incl is the inclusive scan of the lengths, entry
+// e of the total lies at arena word start[o] + e for its owner o.  Longer ranges
+// are laid in rounds of kSpan entries a vertex, so that 256 of them count in 32
+// bits (a vertex has up to 2^27 neighbours).
+#ifndef DSM_RANGE_SPAN  // tests build with a small one
+#define DSM_RANGE_SPAN (1u << 23)
+#endif
+constexpr uint32_t kSpan = DSM_RANGE_SPAN;
 struct BlockRanges {
   unsigned long long start[256];
   uint32_t incl[256];
@@ -283,10 +289,13 @@ __global__ void __launch_bounds__(256) k_filter_op(DevGraph g, const FilterDevic
           a = lo[0];
           len = lo[1] - a;
         }
-        const uint32_t total = lay_ranges(R, (unsigned long long)off * 4 + a, len);
-        for (uint32_t e = t; e < total; e += 256)
-          leaf_rule(op, g.arena[range_entry(R, e)] & kIdMask, f.vcand, f.enc, words);
-        __syncthreads();
+        for (uint32_t from = 0;; from += kSpan) {
+          const uint32_t rest = len > from ? len - from : 0u;
+          const uint32_t total = lay_ranges(R, (unsigned long long)off * 4 + a + from, min(rest, kSpan));
+          for (uint32_t e = t; e < total; e += 256)
+            leaf_rule(op, g.arena[range_entry(R, e)] & kIdMask, f.vcand, f.enc, words);
+          if (!__syncthreads_or(rest > kSpan)) break;
+        }
       }
       if (t == 0) s_n = n;
     }
@@ -432,12 +441,16 @@ __global__ void __launch_bounds__(256) k_region_expand(DevGraph g, RegionDevice 
   const uint32_t tile = min((hi - lo + gridDim.x - 1) / gridDim.x, 256u);
   for (uint32_t base = lo + blockIdx.x * tile; base < hi; base += gridDim.x * tile) {
     const uint2 av = t < tile && base + t < hi ? g.adj[rg.list[base + t]] : make_uint2(0, 0);
-    const uint32_t total = lay_ranges(R, (unsigned long long)av.x * 4, av.y);
-    for (uint32_t e = t; e < total; e += 256) {
-      claim(rg, epoch, g.arena[range_entry(R, e)] & kIdMask, hop);
-      if ((e >> 8) % 8 == 7 && *(volatile const uint32_t *)&rg.info->ov_round < 64) break;
+    for (uint32_t from = 0;; from += kSpan) {
+      const uint32_t rest = av.y > from ? av.y - from : 0u;
+      const uint32_t total = lay_ranges(R, (unsigned long long)av.x * 4 + from, min(rest, kSpan));
+      for (uint32_t e = t; e < total; e += 256) {
+        claim(rg, epoch, g.arena[range_entry(R, e)] & kIdMask, hop);
+        if ((e >> 8) % 8 == 7 && *(volatile const uint32_t *)&rg.info->ov_round < 64) break;
+      }
+      if (__syncthreads_or(*(volatile const uint32_t *)&rg.info->ov_round < 64)) return;
+      if (!__syncthreads_or(rest > kSpan)) break;
     }
-    if (__syncthreads_or(*(volatile const uint32_t *)&rg.info->ov_round < 64)) return;
   }
 }
 

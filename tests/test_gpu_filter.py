@@ -280,3 +280,36 @@ def test_filter_ops_carry_candidates_from_tile_to_tile(tiles, extra):
         assert np.array_equal(bm, obm), f"query {qid}: bitmaps differ at u {np.nonzero((bm != obm).any(1))[0]}"
     assert any(b.any() for b in obm)
     e.close()
+
+
+def test_ranges_laid_in_several_rounds(tmp_path):
+    """The filter's block-wide ranges with rounds of 5 entries a vertex, in a
+    library built for the purpose: bitmaps, masks and regions as ever."""
+    import os
+    import shutil
+    import subprocess
+    import sys
+
+    from dsm_b200 import build as b
+    b.build()
+    pkg = tmp_path / "dsm_b200"
+    pkg.mkdir()
+    shutil.copy(os.path.join(b.HERE, "__init__.py"), pkg)
+    src = "engine/filter.cu"
+    objs = [os.path.join(b.BUILD, x.replace("/", "_") + ".o") for x in b.LIB_SOURCES if x != src]
+    subprocess.run([b.NVCC, *b.CU_FLAGS, "-DDSM_RANGE_SPAN=5", "-c", os.path.join(b.CSRC, src), "-o",
+                    str(tmp_path / "filter.o")], check=True)
+    subprocess.run([b.NVCC, *b.ARCH, "-shared", "-o", str(pkg / "libdsm.so"), str(tmp_path / "filter.o"), *objs,
+                    "-lcudart"], check=True)
+    script = """
+import dsm_b200, tests.test_gpu_filter as t
+assert dsm_b200.__file__.startswith({tmp!r})
+for nv, labels in ((257, 32), (700, 3)):
+    t.test_filter_at_the_edges_of_its_tiles(nv, labels)
+t.test_region_list_fills_within_a_hop(30_000, 3)
+t.test_region_list_fills_within_a_hop(65_530, 4)
+t.test_incremental_filter_equals_full(1, 0, 1, 32, 10)
+""".format(tmp=str(tmp_path))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([str(tmp_path), b.ROOT]))
+    r = subprocess.run([sys.executable, "-c", script], env=env, cwd=str(tmp_path), capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
