@@ -241,8 +241,10 @@ int Engine::launch_front(Staged &S) {
   }
   // the edge filter anew once it holds as many deleted edges as words, or has
   // outgrown them (a pass over the runs per as many updates)
-  if (flt_words && (flt_removed > flt_words || flt_added > 2 * flt_words))
-    if ((rc = build_edge_filter(flt_edges + flt_added))) return rc;
+  if (flt_words && (flt_removed > flt_words || flt_added > 2 * flt_words)) {
+    uint64_t edges = 0;
+    if ((rc = count_edges(&edges)) || (rc = build_edge_filter(edges))) return rc;
+  }
   flt_added += S.inserts;
   flt_removed += m - S.inserts;
   // what allocates, synchronises or copies pageable memory runs before the

@@ -259,16 +259,35 @@ int Engine::load_graph(uint32_t nv_, const uint32_t *labels, std::vector<uint64_
   return build_edge_filter(keys.size());
 }
 
-// The matcher's edge filter from the graph on the device (`edges`: at least as
-// many as it has): a word per one to two edges (a power of two, 2^27 at most).
-// Without room for it the matcher searches every run.
+// Edges of the graph on the device (once per rebuild of the filter: host counts
+// of the updates do not tell those that changed nothing).
+int Engine::count_edges(uint64_t *edges) {
+  unsigned long long *sum = (unsigned long long *)d_arena_top.ptr + 1, entries = 0;
+  CK(cudaMemsetAsync(sum, 0, 8, stream));
+  launch_entry_count(dev_graph(), sum, num_sms * 4, stream);
+  ++stats.kernel_launches;
+  CK(cudaMemcpyAsync(&entries, sum, 8, cudaMemcpyDeviceToHost, stream));
+  CK(cudaStreamSynchronize(stream));
+  *edges = entries / 2;
+  return DSM_OK;
+}
+
+// The matcher's edge filter from the graph on the device, which has `edges`: a
+// word per one to two of them (a power of two, 2^27 at most).  Without room for
+// a larger one it stays as large as it is, up to eight edges a word (above, half
+// of all edges pass it); without room for any the matcher searches every run.
 int Engine::build_edge_filter(uint64_t edges) {
   uint64_t words = 1024;
   while (words * 2 < edges && words < (1ull << 27)) words *= 2;
   flt_words = 0;
-  if (dalloc(d_flt, words * 4)) return DSM_OK;
+  if (dalloc(d_flt, words * 4)) {
+    while (words * 4 > d_flt.bytes) words /= 2;
+    if (!words || words * 8 < edges) {
+      dfree(d_flt);
+      return DSM_OK;
+    }
+  }
   flt_words = words;
-  flt_edges = edges;
   flt_added = flt_removed = 0;
   CK(cudaMemsetAsync(d_flt.ptr, 0, words * 4, stream));
   launch_edge_filter(dev_graph(), num_sms * 8, stream);

@@ -233,10 +233,11 @@ struct Engine {
   uint32_t nlt = 0;  // label slots in use (slot offsets per vertex: nlt + 1)
   std::vector<uint32_t> label_host;
   DevBuf d_lab, d_adj, d_cap, d_arena, d_arena_top, d_loff;
-  // edge filter of the matcher: words in use (0: none), edges it was built
-  // with, inserts and deletes since
+  // edge filter of the matcher: words in use (0: none), inserts and deletes
+  // since it was built
   DevBuf d_flt;
-  uint64_t flt_words = 0, flt_edges = 0, flt_added = 0, flt_removed = 0;
+  uint64_t flt_words = 0, flt_added = 0, flt_removed = 0;
+  int count_edges(uint64_t *edges);
   int build_edge_filter(uint64_t edges);
   // incremental filter region (filter.cuh RegionInfo)
   DevBuf d_rinfo, d_rmark, d_rlist, d_rprev;

@@ -409,6 +409,15 @@ __global__ void k_edge_filter(DevGraph g) {
   }
 }
 
+// Bound by the degrees' bytes; launched once per rebuild of the edge filter.
+__global__ void k_entry_count(DevGraph g, unsigned long long *sum) {
+  unsigned long long n = 0;
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < g.nv; v += gridDim.x * blockDim.x) n += g.adj[v].y;
+#pragma unroll
+  for (uint32_t d = 16; d; d >>= 1) n += __shfl_xor_sync(kFull, n, d);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(sum, n);
+}
+
 __global__ void k_batch_clear(ClearArgs A) {
   const BatchHdr h = *reinterpret_cast<const BatchHdr *>(A.stage);
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -504,6 +513,10 @@ void launch_arena_move(DevGraph g, const uint2 *nadj, uint32_t *narena, int bloc
 }
 
 void launch_edge_filter(DevGraph g, int blocks, cudaStream_t s) { k_edge_filter<<<blocks, 256, 0, s>>>(g); }
+
+void launch_entry_count(DevGraph g, unsigned long long *sum, int blocks, cudaStream_t s) {
+  k_entry_count<<<blocks, 256, 0, s>>>(g, sum);
+}
 
 void launch_adj_insert(const AdjUpdateArgs &a, int blocks, cudaStream_t s) {
   k_adj_insert<<<blocks, 256, 0, s>>>(a);

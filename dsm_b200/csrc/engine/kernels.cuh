@@ -91,6 +91,8 @@ void launch_adj_insert(const AdjUpdateArgs &a, int blocks, cudaStream_t s);
 void launch_arena_move(DevGraph g, const uint2 *nadj, uint32_t *narena, int blocks, cudaStream_t s);
 // The graph's edge filter (g.flt, cleared before) from its runs.
 void launch_edge_filter(DevGraph g, int blocks, cudaStream_t s);
+// Adds the entries of all runs to *sum.
+void launch_entry_count(DevGraph g, unsigned long long *sum, int blocks, cudaStream_t s);
 void launch_adj_delete(const AdjUpdateArgs &a, int blocks, cudaStream_t s);
 // Ends a batch: the endpoints' marks go and, with hdr->pack, what the host
 // downloads of it is laid out in one piece: 64 bytes of the error block, the

@@ -276,3 +276,24 @@ def test_plain_runs_of_more_entries_than_32_bits_count(fill):
         C.c_void_p(cnt.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream))
     assert rc == 0
     assert int(cnt[0]) == want
+
+
+def test_edge_filter_keeps_to_the_graph_size():
+    """Edges deleted and inserted again and again, and inserts of edges that
+    are there: the graph stays the size it is, and so does the memory in use."""
+    rng, edges, labels = _dense(300, 4000, 6)
+    q = d.Query.from_edges(labels[:4], [(0, 1), (1, 2), (2, 3), (0, 3), (0, 2)])
+    e = d.Engine(0)
+    e.set_option(d.OPT_LIST, 0)
+    e.load_graph_edges(300, labels, edges)
+    e.register(q)
+    st = oracle_stream(300, labels, edges, q)
+    used = []
+    for k in range(24):
+        pick = edges[rng.permutation(len(edges))[:3000]]
+        ups = np.concatenate([np.full((3000, 1), k & 1), pick, np.zeros((3000, 1))], 1).astype(np.uint32)
+        r = e.run_batch(ups)
+        assert np.array_equal(r.counts[0], st.apply(ups, listed=False)[1])
+        used.append(e.stats()["device_bytes_in_use"])
+    assert used[-1] == used[0], used
+    e.close()
