@@ -124,8 +124,11 @@ int dsm_engine_set_option(dsm_engine *e, int option, int64_t value) {
       E.query_list_limit = (unsigned long long)value;
       return DSM_OK;
     case DSM_OPT_MEM_BUDGET:
-      if (value <= 0 || (uint64_t)value < E.bytes_in_use)
+      if (value <= 0 || (uint64_t)value < E.bytes_in_use - E.spare_bytes())
         return E.fail(DSM_ERR_ARG, "budget must cover the bytes in use");
+      while ((uint64_t)value < E.bytes_in_use && E.release_spare()) {
+      }
+      E.budget_counts_spare = E.graph_loaded;
       E.budget = (size_t)value;
       E.admit_pending();
       return DSM_OK;

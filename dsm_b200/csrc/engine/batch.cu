@@ -198,6 +198,7 @@ int Engine::read_sched(uint32_t nq) {
 }
 
 int Engine::launch_front(Staged &S) {
+  listing = false;
   if (int rc = sync_queries()) return rc;
   HostOut &H = hout[S.slot];
   const uint32_t n = S.n, m = S.m;
@@ -235,9 +236,6 @@ int Engine::launch_front(Staged &S) {
   if (list_mode && S.match) {
     const size_t cap = std::max<uint64_t>(result_cap, 1024);
     if ((rc = dalloc(d_out_seg, cap * 4)) || (rc = dalloc(d_out_tup, cap * S.W * 4))) return rc;
-    // without room for these the table itself crosses to the host
-    S.placed = !dalloc(d_segoff, (S.nseg + 1) * 8) && !dalloc(d_segcur, S.nseg * 4) &&
-               !dalloc(d_segchunk, (S.nseg + 1) * 4) && !dalloc(d_listsum, 3 * kListBlocks * 8);
   }
   // the edge filter anew once it holds as many deleted edges as words, or has
   // outgrown them (a pass over the runs per as many updates)
@@ -254,6 +252,11 @@ int Engine::launch_front(Staged &S) {
   if (qd_dirty)
     if ((rc = upload_qd())) return rc;
   if (S.match && (rc = prepare_filters())) return rc;
+  // last, so that no other allocation of the batch makes them go: without room
+  // for these the table itself crosses to the host
+  S.placed = list_mode && S.match && spare_alloc(d_segoff, (S.nseg + 1) * 8) && spare_alloc(d_segcur, S.nseg * 4) &&
+             spare_alloc(d_segchunk, (S.nseg + 1) * 4) && spare_alloc(d_listsum, 3 * kListBlocks * 8);
+  listing = S.placed;
   // what the host reads of the batch: error block, counts, view times
   const size_t counted = (size_t)S.nq_live * n * 8;
   S.pack = counted + (size_t)n * 4 <= kPackBytes;
@@ -503,7 +506,7 @@ int Engine::place_results(Staged &S) {
   const size_t used = S.cnt * (size_t)S.W;
   if (used + S.words <= d_out_tup.bytes / 4) {
     S.out = table + used;
-  } else if (dalloc(d_list, S.words * 4) == DSM_OK) {
+  } else if (spare_alloc(d_list, S.words * 4)) {
     S.out = (uint32_t *)d_list.ptr;
   } else {
     S.placed = false;
@@ -541,6 +544,7 @@ int Engine::finish_device(Staged &S) {
     // nothing was written to the arena; the marks still go
     launch_clear_touch(g, dh, (const uint4 *)d_upd.ptr, pk, blocks, stream);
     CK(cudaStreamSynchronize(stream));
+    listing = false;  // the batch starts anew
     if (int rc = compact_arena(arena_need16 * 4)) return rc;
     return kRetryArena;
   }
@@ -599,7 +603,7 @@ int Engine::finish_device(Staged &S) {
       launch_sched_init((Sched *)d_sched.ptr, dh, (unsigned long long *)d_job_seq.ptr, job_ring, stream, stall_test);
       ++stats.kernel_launches;
       std::memset(&ma, 0, sizeof(ma));
-      ma.g = g;
+      ma.g = dev_graph();  // the edge filter may have made room for the table
       ma.bt = DevBatchEdges{(const unsigned long long *)d_bkey.ptr, (const uint32_t *)d_binfo.ptr,
                         (const uint32_t *)d_bloom.ptr, (const uint32_t *)d_etable.ptr,
                         (const unsigned long long *)d_dkey.ptr, 0, 0};
@@ -625,7 +629,7 @@ int Engine::finish_device(Staged &S) {
       ma.split_min = split_min;
       ma.donate_depth = donate_depth;
       ma.pack_max = pack_max;
-          ma.out_seg = (uint32_t *)d_out_seg.ptr;
+      ma.out_seg = (uint32_t *)d_out_seg.ptr;
       ma.out_tup = (uint32_t *)d_out_tup.ptr;
       ma.cap = std::min<unsigned long long>(d_out_seg.bytes / 4, d_out_tup.bytes / 4 / S.W);
       const int mblocks = num_sms * (warps_per_sm ? std::max(1, warps_per_sm / 8) : default_blocks_per_sm());
@@ -663,6 +667,7 @@ int Engine::finish_device(Staged &S) {
                                                    S.sc.out_count.v, d_out_seg.bytes / 4)
                                              : 0;
   if (int rc = place_results(S)) return rc;
+  listing = false;
   if (S.cnt && !S.placed) {
     if (int rc = halloc(H.out_seg, S.cnt * 4)) return rc;
     if (int rc = halloc(H.out_tup, S.cnt * S.W * 4)) return rc;

@@ -60,14 +60,17 @@ int Engine::cuda_fail(cudaError_t e, const char *where) {
     if (_e != cudaSuccess) return cuda_fail(_e, #call); \
   } while (0)
 
-int Engine::dalloc(DevBuf &b, size_t bytes) {
+// Room for a buffer (its contents go when it grows): DSM_OK, or why not.
+int Engine::try_alloc(DevBuf &b, size_t bytes, std::string *why) {
   if (b.bytes >= bytes && b.ptr) return DSM_OK;
   size_t grow = std::max(bytes, b.bytes + b.bytes / 2);
   grow = (grow + 255) & ~(size_t)255;
   if (bytes_in_use - b.bytes + grow > budget) {
     grow = bytes;
-    if (bytes_in_use - b.bytes + grow > budget)
-      return fail(DSM_ERR_OOM, "device memory budget exhausted (" + std::to_string(bytes) + " bytes requested)");
+    if (bytes_in_use - b.bytes + grow > budget) {
+      *why = "device memory budget exhausted (" + std::to_string(bytes) + " bytes requested)";
+      return DSM_ERR_OOM;
+    }
   }
   if (b.ptr) {
     cudaFree(b.ptr);
@@ -78,11 +81,60 @@ int Engine::dalloc(DevBuf &b, size_t bytes) {
   cudaError_t e = cudaMalloc(&b.ptr, grow);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    return fail(DSM_ERR_OOM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    b.ptr = nullptr;
+    *why = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+    return DSM_ERR_OOM;
   }
   b.bytes = grow;
   bytes_in_use += grow;
   return DSM_OK;
+}
+
+// A buffer that a batch needs: what batches can do without makes room for it.
+int Engine::dalloc(DevBuf &b, size_t bytes) {
+  std::string why;
+  while (try_alloc(b, bytes, &why))
+    if (bytes_in_use - b.bytes - spare_bytes() + bytes > budget || !release_spare()) return fail(DSM_ERR_OOM, why);
+  return DSM_OK;
+}
+
+// A buffer that batches can do without: only where there is room.
+bool Engine::spare_alloc(DevBuf &b, size_t bytes) {
+  std::string why;
+  return try_alloc(b, bytes, &why) == DSM_OK;
+}
+
+// Device memory given back before an allocation, a registration or a smaller
+// budget is refused: the tuples' place behind a full table and the listing's
+// scans (results are then placed on the host), and the edge filter (the
+// matcher searches every run, until the next load).  The scans of a batch that
+// is between its matcher and its listing stay.  Registrations leave scans and
+// filter alone under a budget that was set while they were there: it was set
+// against the bytes in use, which count them.
+std::vector<DevBuf *> Engine::spare_bufs(bool registering) {
+  std::vector<DevBuf *> v = {&d_list};
+  if (registering && budget_counts_spare) return v;
+  if (!listing) v.insert(v.end(), {&d_segoff, &d_segcur, &d_segchunk, &d_listsum});
+  v.push_back(&d_flt);
+  return v;
+}
+
+size_t Engine::spare_bytes(bool registering) {
+  size_t n = 0;
+  for (DevBuf *b : spare_bufs(registering)) n += b->bytes;
+  return n;
+}
+
+bool Engine::release_spare(bool registering) {
+  for (DevBuf *b : spare_bufs(registering))
+    if (b->ptr) {
+      cudaStreamSynchronize(stream);  // what was launched may still read it
+      dfree(*b);
+      if (b == &d_flt) flt_words = 0;
+      ++query_gen;  // captured graphs hold it
+      return true;
+    }
+  return false;
 }
 
 void Engine::dfree(DevBuf &b) {
@@ -256,6 +308,7 @@ int Engine::load_graph(uint32_t nv_, const uint32_t *labels, std::vector<uint64_
   label_host.assign(labels, labels + nv_);
   for (auto &q : slots) q.filter_dirty = true;
   if (int r = region_init()) return r;
+  budget_counts_spare = false;
   return build_edge_filter(keys.size());
 }
 
@@ -280,7 +333,7 @@ int Engine::build_edge_filter(uint64_t edges) {
   uint64_t words = 1024;
   while (words * 2 < edges && words < (1ull << 27)) words *= 2;
   flt_words = 0;
-  if (dalloc(d_flt, words * 4)) {
+  if (!spare_alloc(d_flt, words * 4)) {
     while (words * 4 > d_flt.bytes) words /= 2;
     if (!words || words * 8 < edges) {
       dfree(d_flt);
@@ -414,11 +467,11 @@ int Engine::admit(QueryPlan &plan, uint32_t *qid, bool *fits_later, int64_t want
   size_t charged = 0;
   for (const Slot &q : slots)
     if (q.live) charged += q.foot;
-  if (base + charged + foot > budget && d_list.ptr) {  // scratch a listing batch can do without
-    dfree(d_list);
-    base = bytes_in_use - std::min(bytes_in_use, query_bytes_allocated());
-  }
-  if (fits_later) *fits_later = base + foot <= budget;
+  const size_t spare = spare_bytes(true);
+  if (fits_later) *fits_later = base - spare + foot <= budget;
+  if (base - spare + charged + foot <= budget)
+    while (base + charged + foot > budget && release_spare(true))
+      base = bytes_in_use - std::min(bytes_in_use, query_bytes_allocated());
   if (base + charged + foot > budget)
     return fail(DSM_ERR_OOM, "query admission: footprint " + std::to_string(foot) + " bytes exceeds the budget");
   uint32_t id = (uint32_t)slots.size();

@@ -260,6 +260,7 @@ struct Engine {
   static constexpr size_t kMiscBytes = 256;
   HostBuf h_sched;    // Sched, the error block and the listing counters, read after the matcher
   HostBuf h_qlisted;  // view of the last
+  bool listing = false;  // a batch is between its matcher and its listing: d_segoff and the like are in use
   HostOut hout[2];
   int next_slot = 0;
   uint64_t compactions = 0;
@@ -275,7 +276,13 @@ struct Engine {
   int init(int device, size_t budget);
   int fail(int code, const std::string &msg);
   int cuda_fail(cudaError_t e, const char *where);
+  int try_alloc(DevBuf &b, size_t bytes, std::string *why);
   int dalloc(DevBuf &b, size_t bytes);
+  bool spare_alloc(DevBuf &b, size_t bytes);
+  std::vector<DevBuf *> spare_bufs(bool registering = false);
+  size_t spare_bytes(bool registering = false);
+  bool release_spare(bool registering = false);
+  bool budget_counts_spare = false;  // the budget was set after the graph was loaded
   void dfree(DevBuf &b);
   int halloc(HostBuf &b, size_t bytes);
   std::vector<DevBuf *> all_dev_bufs();

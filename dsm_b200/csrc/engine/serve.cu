@@ -151,7 +151,7 @@ Outcome Engine::handle_control(Request &r) {
   bool later = true;
   o.rc = behind ? DSM_ERR_OOM : admit(r.plan, &o.qid, &later);
   if (behind) later = query_footprint(r.plan) + (bytes_in_use - std::min(bytes_in_use, query_bytes_allocated())) <=
-                      budget;
+                      budget + spare_bytes(true);
   if (o.rc == DSM_ERR_OOM && later) {
     std::lock_guard<std::mutex> q(srv.qmu);
     srv.pending.push_back(std::move(r));

@@ -297,3 +297,91 @@ def test_edge_filter_keeps_to_the_graph_size():
         used.append(e.stats()["device_bytes_in_use"])
     assert used[-1] == used[0], used
     e.close()
+
+
+def _budgeted(**opts):
+    """An engine on a graph whose edge filter takes 512 KiB, the memory in use
+    without that filter, and one query's footprint."""
+    rng, edges, labels = _dense(2000, 200_000, 7)
+    q = d.Query.from_edges(labels[:4], [(0, 1), (1, 2), (2, 3), (0, 3), (0, 2)])
+    e = d.Engine(0)
+    for k, v in opts.items():
+        e.set_option(getattr(d, k), v)
+    e.load_graph_edges(2000, labels, edges)
+    full = e.stats()["device_bytes_in_use"]
+    lean = d.Engine(0, full - 1)
+    lean.load_graph_edges(2000, labels, edges)
+    bare = lean.stats()["device_bytes_in_use"]
+    lean.register(q)
+    foot = lean.stats()["query_bytes"]
+    lean.close()
+    assert full - bare == 512 << 10 and foot < 100_000
+    return e, q, rng, edges, labels, bare, foot
+
+
+def _toggles(rng, edges, n):
+    pick = edges[rng.permutation(len(edges))[:n]]
+    return np.concatenate([rng.integers(0, 2, (n, 1)), pick, np.zeros((n, 1))], 1).astype(np.uint32)
+
+
+@pytest.mark.parametrize("queries", [3, 30])
+@pytest.mark.parametrize("when", ["created", "loaded"])
+def test_the_edge_filter_makes_room_for_queries(queries, when):
+    """A budget for the graph and some queries, less than the filter takes or
+    more, given at creation or (less) after loading: as many are admitted as if
+    there were no filter, and not one more."""
+    e, q, rng, edges, labels, bare, foot = _budgeted()
+    budget = bare + queries * foot
+    if when == "created":
+        e.close()
+        e = d.Engine(0, budget)
+        e.load_graph_edges(2000, labels, edges)
+        assert e.stats()["device_bytes_in_use"] == bare + (512 << 10) * (queries == 30)
+    elif queries == 30:  # set against the bytes in use, which count the filter
+        budget += 512 << 10
+        e.set_option(d.OPT_MEM_BUDGET, budget)
+    else:
+        e.set_option(d.OPT_MEM_BUDGET, budget)
+    ids = [e.register(q) for _ in range(queries)]
+    with pytest.raises(d.DSMError) as x:
+        e.register(q)
+    assert x.value.code == 2  # DSM_ERR_OOM
+    e.set_option(d.OPT_MEM_BUDGET, 8 << 30)
+    ups = _toggles(rng, edges, 40)
+    want = oracle_stream(2000, labels, edges, q).apply(ups, listed=False)[1]
+    r = e.run_batch(ups)
+    for qid in ids:
+        assert np.array_equal(r.counts[r.query_index(qid)], want)
+    e.close()
+
+
+def test_the_edge_filter_stays_while_queries_fit():
+    e, q, rng, edges, labels, bare, foot = _budgeted()
+    full = e.stats()["device_bytes_in_use"]
+    e.set_option(d.OPT_MEM_BUDGET, full + 2 * foot)
+    e.register(q)
+    e.register(q)
+    assert e.stats()["device_bytes_in_use"] == full
+    e.close()
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+@pytest.mark.parametrize("n,cap", [(600, 1 << 20), (40, 1200)])
+def test_the_edge_filter_makes_room_for_a_batch(n, cap, graph):
+    """A batch that needs more scratch, and one whose result table has to grow,
+    with the budget at the bytes in use: the filter's go to them."""
+    e, q, rng, edges, labels, bare, foot = _budgeted(OPT_RESULT_CAP=cap, OPT_GRAPH=graph)
+    e.register(q)
+    st = oracle_stream(2000, labels, edges, q)
+    none = np.array([[1, *edges[0], 0]] * 40, np.uint32)  # there already
+    e.run_batch(none)
+    e.set_option(d.OPT_MEM_BUDGET, e.stats()["device_bytes_in_use"])
+    st.apply(none, listed=False)
+    for _ in range(2):
+        ups = _toggles(rng, edges, n)
+        r = e.run_batch(ups)
+        _, c, t = st.apply(ups)
+        assert r.listed and np.array_equal(r.counts[0], c)
+        assert np.array_equal(r.tuples.reshape(-1, 4), np.concatenate(t))
+    assert e.stats()["result_regrows"] == (cap == 1200) or n == 600
+    e.close()
