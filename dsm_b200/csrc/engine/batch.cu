@@ -218,8 +218,7 @@ int Engine::launch_front(Staged &S) {
   if ((rc = dalloc(d_upd, nn * 16)) || (rc = dalloc(d_bkey, mm * 8)) || (rc = dalloc(d_bidx, mm * 4)) ||
       (rc = dalloc(d_binfo, mm * 4)) || (rc = dalloc(d_gflag, mm)) || (rc = dalloc(d_vtp, nn * 4)) ||
       (rc = dalloc(d_dkey, dd * 8)) || (rc = dalloc(d_dhead, (dd + 1) * 4)) || (rc = dalloc(d_dsel, dd * 4)) ||
-      (rc = dalloc(d_segcnt, S.nseg * 8)) || (rc = sched_block(S.nq_live)) || (rc = dalloc(d_stage, S.stage_bytes)) ||
-      (rc = dalloc(d_pack, 64 + kPackBytes)))
+      (rc = dalloc(d_segcnt, S.nseg * 8)) || (rc = sched_block(S.nq_live)))
     return rc;
   size_t bloom_words = 64;
   while (bloom_words < 4ull * m) bloom_words *= 2;
@@ -233,6 +232,12 @@ int Engine::launch_front(Staged &S) {
     if ((rc = dalloc(d_jobs, (size_t)job_ring * sizeof(JobRec))) || (rc = dalloc(d_job_seq, (size_t)job_ring * 8)))
       return rc;
   }
+  // The upload and the packed download lie in the donation ring, which is idle
+  // before and after the matcher (an upload of more than its 64 MiB, beyond a
+  // million updates, has a buffer of its own): copies of their own would count
+  // towards the budget, 40 to 52 bytes an update and 256 KiB.
+  if (S.stage_bytes > d_jobs.bytes && (rc = dalloc(d_stage, S.stage_bytes))) return rc;
+  unsigned char *const stage = (unsigned char *)(S.stage_bytes > d_jobs.bytes ? d_stage.ptr : d_jobs.ptr);
   if (list_mode && S.match) {
     const size_t cap = std::max<uint64_t>(result_cap, 1024);
     if ((rc = dalloc(d_out_seg, cap * 4)) || (rc = dalloc(d_out_tup, cap * S.W * 4))) return rc;
@@ -284,13 +289,13 @@ int Engine::launch_front(Staged &S) {
 
   // one upload from the slot's pinned staging
   CK(cudaEventRecord(H.ev0, stream));
-  CK(cudaMemcpyAsync(d_stage.ptr, H.stage.ptr, S.stage_bytes, cudaMemcpyHostToDevice, stream));
+  CK(cudaMemcpyAsync(stage, H.stage.ptr, S.stage_bytes, cudaMemcpyHostToDevice, stream));
 
   DevGraph g = dev_graph();
   const BatchHdr *dh = (const BatchHdr *)d_hdr.ptr;
   unsigned int *d_err = (unsigned int *)d_misc.ptr;
   unsigned long long *segwork = S.work_limit ? (unsigned long long *)d_segwork.ptr : nullptr;
-  ClearArgs ca{(const unsigned char *)d_stage.ptr, (BatchHdr *)d_hdr.ptr, (uint4 *)d_upd.ptr,
+  ClearArgs ca{stage, (BatchHdr *)d_hdr.ptr, (uint4 *)d_upd.ptr,
                (unsigned long long *)d_bkey.ptr, (unsigned long long *)d_dkey.ptr, (uint32_t *)d_bidx.ptr,
                (uint32_t *)d_dhead.ptr, (unsigned long long *)d_job_seq.ptr, S.match && !S.plain ? job_ring : 0ull,
                (uint32_t *)d_vtp.ptr, (unsigned long long *)d_segcnt.ptr, segwork,
@@ -538,7 +543,7 @@ int Engine::finish_device(Staged &S) {
                    (unsigned int *)d_misc.ptr, (unsigned long long *)((char *)d_misc.ptr + 8),
                    (unsigned long long *)((char *)d_misc.ptr + 16)};
   const int blocks = num_sms * 4;
-  const PackArgs pk{(unsigned char *)d_pack.ptr, (const uint32_t *)d_misc.ptr,
+  const PackArgs pk{(unsigned char *)d_jobs.ptr, (const uint32_t *)d_misc.ptr,
                     (const unsigned long long *)d_segcnt.ptr, (const uint32_t *)d_vtp.ptr};
   if (arena_short) {
     // nothing was written to the arena; the marks still go
@@ -701,7 +706,7 @@ int Engine::finish_device(Staged &S) {
   }
   char *back = (char *)H.back.ptr;
   if (S.pack) {
-    CK(cudaMemcpyAsync(back, d_pack.ptr, 64 + counted + (size_t)S.n * 4, cudaMemcpyDeviceToHost, stream));
+    CK(cudaMemcpyAsync(back, d_jobs.ptr, 64 + counted + (size_t)S.n * 4, cudaMemcpyDeviceToHost, stream));
   } else {
     CK(cudaMemcpyAsync(back, d_misc.ptr, 64, cudaMemcpyDeviceToHost, stream));
     if (counted) CK(cudaMemcpyAsync(back + 64, d_segcnt.ptr, counted, cudaMemcpyDeviceToHost, stream));

@@ -223,7 +223,8 @@ struct Engine {
   uint64_t query_gen = 0;                    // bumped whenever the live queries or filters change
   bool filter_timed = false;  // the filter events of this batch were recorded
   uint64_t result_cap = 1 << 20;
-  uint32_t job_ring = 1 << 19;  // job slots of the matcher's donation ring
+  // job slots of the matcher's donation ring (64 MiB; more than a packed download takes)
+  static constexpr uint32_t job_ring = 1 << 19;
   uint64_t list_limit_bytes = 8ull << 30;  // beyond this a batch returns counts only
 
   // graph
@@ -254,7 +255,7 @@ struct Engine {
 
   // batch scratch
   DevBuf d_upd, d_bkey, d_bidx, d_binfo, d_gflag, d_vtp, d_dkey, d_dhead, d_dsel, d_seeds, d_sched, d_jobs,
-      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_stage, d_pack, d_bloom, d_etable, d_fdev,
+      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_stage, d_bloom, d_etable, d_fdev,
       d_widths, d_segoff, d_segcur, d_segchunk, d_listsum, d_list;
   std::vector<FilterDevice> fdev_host;  // what d_fdev holds
   static constexpr size_t kMiscBytes = 256;

@@ -385,3 +385,21 @@ def test_the_edge_filter_makes_room_for_a_batch(n, cap, graph):
         assert np.array_equal(r.tuples.reshape(-1, 4), np.concatenate(t))
     assert e.stats()["result_regrows"] == (cap == 1200) or n == 600
     e.close()
+
+
+def test_a_batch_takes_little_beside_the_ring():
+    """The upload and the packed download lie in the donation ring (64 MiB of
+    records, 4 MiB of slots): a batch of one update takes 64 KiB more at most,
+    one of 4,096 up to 256 bytes an update."""
+    rng, edges, labels = _dense(2000, 200_000, 7)
+    e = d.Engine(0)
+    e.set_option(d.OPT_LIST, 0)
+    e.load_graph_edges(2000, labels, edges)
+    e.register(d.Query.from_edges([0, 1, 2], [(0, 1), (1, 2)]))
+    before = e.stats()["device_bytes_in_use"]
+    e.run_batch(_toggles(rng, edges, 1))
+    one = e.stats()["device_bytes_in_use"] - before
+    assert one <= (68 << 20) + (64 << 10)
+    e.run_batch(_toggles(rng, edges, 4096))
+    assert e.stats()["device_bytes_in_use"] - before - one <= 256 * 4096
+    e.close()
