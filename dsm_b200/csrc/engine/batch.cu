@@ -228,10 +228,8 @@ int Engine::launch_front(Staged &S) {
   if (S.match && (rc = dalloc(d_seeds, S.seed_cap * 16))) return rc;
   if (S.match && (bfs_levels || (tune_next && !S.plain)) && (rc = dalloc(d_rows, bfs_rows * sizeof(JobRec))))
     return rc;
-  if (!d_jobs.ptr) {
-    if ((rc = dalloc(d_jobs, (size_t)job_ring * sizeof(JobRec))) || (rc = dalloc(d_job_seq, (size_t)job_ring * 8)))
-      return rc;
-  }
+  if ((rc = dalloc(d_jobs, (size_t)job_ring * sizeof(JobRec))) || (rc = dalloc(d_job_seq, (size_t)job_ring * 8)))
+    return rc;
   // The upload and the packed download lie in the donation ring, which is idle
   // before and after the matcher (an upload of more than its 64 MiB, beyond a
   // million updates, has a buffer of its own): copies of their own would count

@@ -403,3 +403,23 @@ def test_a_batch_takes_little_beside_the_ring():
     e.run_batch(_toggles(rng, edges, 4096))
     assert e.stats()["device_bytes_in_use"] - before - one <= 256 * 4096
     e.close()
+
+
+def test_a_ring_refused_by_halves():
+    """A budget with room for the ring's records and not for its slots: the
+    batch is refused; with room it runs, and equals the oracle."""
+    rng, edges, labels = _dense(2000, 200_000, 7)
+    q = d.Query.from_edges([0, 1, 2], [(0, 1), (1, 2)])
+    e = d.Engine(0)
+    e.set_option(d.OPT_LIST, 0)
+    e.load_graph_edges(2000, labels, edges)
+    qid = e.register(q)
+    ups = _toggles(rng, edges, 20)
+    e.set_option(d.OPT_MEM_BUDGET, e.stats()["device_bytes_in_use"] + (66 << 20))
+    with pytest.raises(d.DSMError) as x:
+        e.run_batch(ups)
+    assert x.value.code == 2  # DSM_ERR_OOM
+    e.set_option(d.OPT_MEM_BUDGET, 8 << 30)
+    r = e.run_batch(ups)
+    assert np.array_equal(r.counts[0], oracle_stream(2000, labels, edges, q).apply(ups, listed=False)[1])
+    e.close()
