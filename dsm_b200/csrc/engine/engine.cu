@@ -307,6 +307,7 @@ int Engine::load_graph(uint32_t nv_, const uint32_t *labels, std::vector<uint64_
   graph_loaded = true;
   label_host.assign(labels, labels + nv_);
   for (auto &q : slots) q.filter_dirty = true;
+  queries_dirty = true;  // the device's query table holds the bitmaps' row length
   if (int r = region_init()) return r;
   budget_counts_spare = false;
   return build_edge_filter(keys.size());

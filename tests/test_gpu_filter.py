@@ -313,3 +313,27 @@ t.test_incremental_filter_equals_full(1, 0, 1, 32, 10)
     env = dict(os.environ, PYTHONPATH=os.pathsep.join([str(tmp_path), b.ROOT]))
     r = subprocess.run([sys.executable, "-c", script], env=env, cwd=str(tmp_path), capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("first,second", [(40, 3000), (3000, 40)])
+def test_another_graph_under_registered_queries(first, second):
+    """A graph of another size loaded while queries stay registered and
+    filtered: the bitmaps' rows are the new graph's."""
+    rng = np.random.default_rng(first)
+    q = d.Query.from_edges([0, 1, 2, 1], [(0, 1), (1, 2), (2, 3)])
+    e = d.Engine(0)
+    e.set_option(d.OPT_FILTER, 2)
+    qid = None
+    for nv in (first, second, first):
+        labels = rng.integers(0, 3, nv).astype(np.uint32)
+        edges = rng.integers(0, nv, (8 * nv, 2)).astype(np.uint32)
+        edges = edges[edges[:, 0] != edges[:, 1]]
+        e.load_graph_edges(nv, labels, edges)
+        if qid is None:
+            qid = e.register(q)
+        st = oracle_stream(nv, labels, edges, q)
+        a = rng.integers(0, nv, 24)
+        ups = np.stack([rng.integers(0, 2, 24), a, (a + 1 + rng.integers(0, nv - 1, 24)) % nv, 0 * a], 1).astype(np.uint32)
+        total, _ = run_stream(e, [qid], [st], [ups, ups[::-1].copy()], check_graph_every=1)
+        assert total > 0
+    e.close()
