@@ -284,10 +284,13 @@ int Engine::load_graph(uint32_t nv_, const uint32_t *labels, std::vector<uint64_
     }
   });
   int rc;
+  const std::vector<void *> held = {d_lab.ptr, d_adj.ptr, d_cap.ptr, d_loff.ptr, d_arena.ptr};
   if ((rc = dalloc(d_lab, (size_t)nv_ * 4)) || (rc = dalloc(d_adj, (size_t)nv_ * 8)) ||
       (rc = dalloc(d_cap, (size_t)nv_ * 4)) || (rc = dalloc(d_loff, loff.size() * 4)) ||
       (rc = dalloc(d_arena, arena_words * 4))) {
     cudaFreeHost(stage.ptr);
+    // a buffer that was replaced took its part of the graph at hand with it
+    if (held != std::vector<void *>{d_lab.ptr, d_adj.ptr, d_cap.ptr, d_loff.ptr, d_arena.ptr}) graph_loaded = false;
     return rc;
   }
   CK(cudaMemcpyAsync(d_loff.ptr, loff.data(), loff.size() * 4, cudaMemcpyHostToDevice, stream));
@@ -360,8 +363,10 @@ int Engine::region_init() {
   const uint32_t prev_cap = 1u << 18;
   int rc;
   if ((rc = dalloc(d_rinfo, sizeof(RegionInfo))) || (rc = dalloc(d_rmark, (size_t)std::max<uint32_t>(nv, 1) * 4)) ||
-      (rc = dalloc(d_rlist, (size_t)std::max<uint32_t>(cap, 1) * 4)) || (rc = dalloc(d_rprev, (size_t)prev_cap * 4)))
+      (rc = dalloc(d_rlist, (size_t)std::max<uint32_t>(cap, 1) * 4)) || (rc = dalloc(d_rprev, (size_t)prev_cap * 4))) {
+    dfree(d_rinfo);  // no region: every filter run is full
     return rc;
+  }
   RegionInfo I;
   std::memset(&I, 0, sizeof(I));
   I.stale = 1;

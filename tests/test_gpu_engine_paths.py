@@ -309,3 +309,32 @@ def test_graph_replay_when_only_the_updates_outgrow_their_buffer():
         captures.append(e.stats()["graph_captures"])
     assert captures[0] == 2 and captures[1] == 4
     e.close()
+
+
+def test_a_refused_load_leaves_no_half_graph():
+    """A second graph that fits the budget only in part is refused: the engine
+    then has the first graph whole or none, and takes the second with room."""
+    w = workload(1)
+    q = d.Query.from_edges([0, 1, 2], [(0, 1), (1, 2)])
+    rng = np.random.default_rng(2)
+    nv = 6 * w.nv
+    labels = rng.integers(0, 3, nv).astype(np.uint32)
+    edges = rng.integers(0, nv, (400_000, 2)).astype(np.uint32)
+    edges = edges[edges[:, 0] != edges[:, 1]]
+    ups = np.array([[1, 0, k, 0] for k in range(1, 9)], np.uint32)
+    want = oracle_stream(nv, labels, edges, q).apply(ups, listed=False)[1]
+    none = oracle_stream(w.nv, w.labels, w.edges, q).apply(ups, listed=False)[1]
+    for room in (0, nv * 4, nv * 12, nv * 30, 4 << 20):
+        e, (qid,) = _fresh(w.nv, w.labels, w.edges, [q], OPT_LIST=0, OPT_FILTER=2)
+        e.set_option(d.OPT_MEM_BUDGET, e.stats()["device_bytes_in_use"] + room)
+        with pytest.raises(d.DSMError) as x:
+            e.load_graph_edges(nv, labels, edges)
+        assert x.value.code == OOM
+        e.set_option(d.OPT_MEM_BUDGET, 8 << 30)
+        try:
+            assert np.array_equal(e.run_batch(ups).counts[0], none)
+        except d.DSMError as x:
+            assert x.code == 8  # DSM_ERR_STATE: no graph
+        e.load_graph_edges(nv, labels, edges)
+        assert np.array_equal(e.run_batch(ups).counts[0], want)
+        e.close()
