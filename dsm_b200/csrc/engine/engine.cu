@@ -183,7 +183,7 @@ std::vector<DevBuf *> Engine::all_dev_bufs() {
                              &d_pair_off, &d_pair_ent, &d_upd, &d_bkey, &d_bidx, &d_binfo, &d_gflag,
                              &d_vtp, &d_dkey, &d_dhead, &d_dsel, &d_seeds, &d_sched, &d_jobs,
                              &d_job_seq, &d_out_seg, &d_out_tup, &d_segcnt, &d_hdr, &d_segwork, &d_stage,
-                             &d_rinfo, &d_rmark, &d_rlist, &d_rprev, &d_rows, &d_bloom, &d_etable, &d_fdev,
+                             &d_rinfo, &d_rmark, &d_rlist, &d_rprev, &d_rows, &d_bloom, &d_etable, &batch_filters.dev, &one_filter.dev,
                              &d_widths, &d_segoff, &d_segcur, &d_segchunk, &d_listsum, &d_list};
   for (auto &q : slots) v.push_back(&q.bitmap);
   for (auto &q : slots) v.push_back(&q.filter_scratch);
@@ -867,29 +867,31 @@ FilterDevice Engine::filter_device(uint32_t id) const {
   return f;
 }
 
-// The device array of the filters that the next launch runs; uploaded when
-// it differs from the last one (the upload waits: the array is pageable).
-int Engine::set_filters(const std::vector<uint32_t> &ids) {
+// A device array of filters; uploaded when it differs from what it holds (the
+// upload waits: the array is pageable).  The batches' array and that of
+// query_filter are apart, so that a call of the latter between batches changes
+// nothing that captured graphs hold.
+int Engine::set_filters(FilterSet &fs, const std::vector<uint32_t> &ids) {
   std::vector<FilterDevice> f;
   f.reserve(ids.size());
   for (uint32_t id : ids) f.push_back(filter_device(id));
-  if (f.size() == fdev_host.size() &&
-      (f.empty() || std::memcmp(f.data(), fdev_host.data(), f.size() * sizeof(FilterDevice)) == 0))
+  if (f.size() == fs.host.size() &&
+      (f.empty() || std::memcmp(f.data(), fs.host.data(), f.size() * sizeof(FilterDevice)) == 0))
     return DSM_OK;
-  fdev_host.clear();
-  if (int rc = dalloc(d_fdev, std::max<size_t>(f.size(), 1) * sizeof(FilterDevice))) return rc;
-  CK(cudaMemcpyAsync(d_fdev.ptr, f.data(), f.size() * sizeof(FilterDevice), cudaMemcpyHostToDevice, stream));
+  fs.host.clear();
+  if (int rc = dalloc(fs.dev, std::max<size_t>(f.size(), 1) * sizeof(FilterDevice))) return rc;
+  CK(cudaMemcpyAsync(fs.dev.ptr, f.data(), f.size() * sizeof(FilterDevice), cudaMemcpyHostToDevice, stream));
   CK(cudaStreamSynchronize(stream));
-  fdev_host = std::move(f);
-  ++query_gen;
+  fs.host = std::move(f);
+  if (&fs == &batch_filters) ++query_gen;
   return DSM_OK;
 }
 
-int Engine::run_filters(int mode, int force_full) {
+int Engine::run_filters(const FilterSet &fs, int mode, int force_full) {
   uint32_t max_ops = 0;
-  for (const FilterDevice &f : fdev_host) max_ops = std::max(max_ops, f.nops);
+  for (const FilterDevice &f : fs.host) max_ops = std::max(max_ops, f.nops);
   stats.kernel_launches +=
-      launch_query_filters(dev_graph(), (const FilterDevice *)d_fdev.ptr, (uint32_t)fdev_host.size(), max_ops, mode,
+      launch_query_filters(dev_graph(), (const FilterDevice *)fs.dev.ptr, (uint32_t)fs.host.size(), max_ops, mode,
                            num_sms, stream, region_dev(), force_full || !filter_incremental);
   return DSM_OK;
 }
@@ -923,7 +925,7 @@ int Engine::prepare_filters() {
     if (int rc = upload_qd()) return rc;
   if (changed) CK(cudaStreamSynchronize(stream));  // qd_host is pageable
   if (filter_mode > 0)
-    if (int rc = set_filters(live_ids)) return rc;
+    if (int rc = set_filters(batch_filters, live_ids)) return rc;
   return DSM_OK;
 }
 
@@ -940,7 +942,7 @@ int Engine::launch_filters() {
     launch_region_build(dev_graph(), region_dev(), hdr_n, (const uint4 *)d_upd.ptr, hops, num_sms, stream);
     stats.kernel_launches += 3 + 2 * hops;
   }
-  if (int rc = run_filters(filter_mode, 0)) return rc;
+  if (int rc = run_filters(batch_filters, filter_mode, 0)) return rc;
   if (region) {
     launch_region_save(region_dev(), hdr_n, (const uint4 *)d_upd.ptr, stream);
     ++stats.kernel_launches;
@@ -971,8 +973,8 @@ int Engine::query_filter(uint32_t qid, uint32_t *bitmaps, uint32_t *v_cand_us) {
   if (qid >= slots.size() || !slots[qid].live) return fail(DSM_ERR_NOT_FOUND, "no such query");
   CK(cudaSetDevice(device));
   if (int rc = prepare_filter(qid)) return rc;
-  if (int rc = set_filters({qid})) return rc;
-  if (int rc = run_filters(2, 1)) return rc;
+  if (int rc = set_filters(one_filter, {qid})) return rc;
+  if (int rc = run_filters(one_filter, 2, 1)) return rc;
   CK(cudaGetLastError());
   const Slot &s = slots[qid];
   if (bitmaps)

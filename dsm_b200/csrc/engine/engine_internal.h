@@ -255,9 +255,13 @@ struct Engine {
 
   // batch scratch
   DevBuf d_upd, d_bkey, d_bidx, d_binfo, d_gflag, d_vtp, d_dkey, d_dhead, d_dsel, d_seeds, d_sched, d_jobs,
-      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_stage, d_bloom, d_etable, d_fdev,
+      d_job_seq, d_out_seg, d_out_tup, d_segcnt, d_misc, d_hdr, d_qlisted, d_segwork, d_stage, d_bloom, d_etable,
       d_widths, d_segoff, d_segcur, d_segchunk, d_listsum, d_list;
-  std::vector<FilterDevice> fdev_host;  // what d_fdev holds
+  struct FilterSet {
+    DevBuf dev;
+    std::vector<FilterDevice> host;  // what dev holds
+  };
+  FilterSet batch_filters, one_filter;
   static constexpr size_t kMiscBytes = 256;
   HostBuf h_sched;    // Sched, the error block and the listing counters, read after the matcher
   HostBuf h_qlisted;  // view of the last
@@ -312,8 +316,8 @@ struct Engine {
   bool capturing = false;
   int prepare_filter(uint32_t id);
   FilterDevice filter_device(uint32_t id) const;
-  int set_filters(const std::vector<uint32_t> &ids);
-  int run_filters(int mode, int force_full);
+  int set_filters(FilterSet &fs, const std::vector<uint32_t> &ids);
+  int run_filters(const FilterSet &fs, int mode, int force_full);
   int launch_match_seq(const MatchArgs &ma, int blocks, uint32_t levels);
   RegionDevice region_dev();
   int region_init();

@@ -337,3 +337,25 @@ def test_another_graph_under_registered_queries(first, second):
         total, _ = run_stream(e, [qid], [st], [ups, ups[::-1].copy()], check_graph_every=1)
         assert total > 0
     e.close()
+
+
+def test_a_query_s_filter_between_captured_batches():
+    """dsm_query_filter between filtered batches: bitmaps as the oracle's, the
+    batches' captured segments replayed, not captured again."""
+    w = workload(2, scale_log2=-4, num_batches=1)
+    ups, qs = next(w.batches()), w.queries[:3]
+    inc, full = _inc_pair(w, qs, OPT_GRAPH=1)
+    captures = []
+    for k in range(8):
+        b = ups[k * 16:(k + 1) * 16]
+        ri, rf = inc[0].run_batch(b), full[0].run_batch(b)
+        assert np.array_equal(ri.counts, rf.counts)
+        _same_state(inc, full, qs, w.nv, f"batch {k}")
+        q = qs[k % 3]
+        bm, vc = inc[0].filter(inc[1][k % 3], q.nv, w.nv)
+        obm, ovc, _, _ = orc.cluster_filter(q.labels, q.offsets, q.nbrs, w.nv, w.labels, *inc[0].export_graph())
+        assert np.array_equal(vc, ovc) and np.array_equal(bm, obm)
+        captures.append(inc[0].stats()["graph_captures"])
+    assert captures[-1] == captures[2], captures
+    for e, _ in (inc, full):
+        e.close()
