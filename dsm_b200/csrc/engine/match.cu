@@ -201,7 +201,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   const uint32_t *bitmap = Q.bitmap;
   const uint32_t seg = Q.local * nupd + upd;
   unsigned long long task_cnt = 0, work = 0;  // warp-uniform
-  uint32_t alg = 0;                           // bytes, this lane's share
+  uint32_t alg = 0;                           // bytes, this lane's share since they were last added up
   // what the segment had left of its work limit when this task last looked
   // (at most 2^32 - 1): a task that alone exceeds it publishes at once, but for
   // a query with a listing budget, which the tuples listed until the heartbeat
@@ -252,16 +252,18 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
     return work_left == 0;
   };
 
+  auto add_bytes = [&]() {
+    const uint32_t a0 = __reduce_add_sync(kFull, alg & 0xFFFFu), a1 = __reduce_add_sync(kFull, alg >> 16);
+    if (lane == 0) atomicAdd(&P.sc->alg_bytes, ((unsigned long long)a1 << 16) + a0);
+    alg = 0;
+  };
   auto flush = [&]() {
     if (P.work_limit && work) publish_work();
-    const uint32_t a0 = __reduce_add_sync(kFull, alg & 0xFFFFu), a1 = __reduce_add_sync(kFull, alg >> 16);
-    if (lane == 0) {
-      if (task_cnt) {
-        atomicAdd(&P.seg_count[seg], task_cnt);
-        atomicAdd(&P.sc->matches, task_cnt);
-      }
-      atomicAdd(&P.sc->alg_bytes, ((unsigned long long)a1 << 16) + a0);
+    if (lane == 0 && task_cnt) {
+      atomicAdd(&P.seg_count[seg], task_cnt);
+      atomicAdd(&P.sc->matches, task_cnt);
     }
+    add_bytes();
   };
 
   __syncwarp();  // the last task's reads of the warp's shared memory are done
@@ -558,6 +560,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
           err = ld_volatile(P.sc->error);
         }
         if (__shfl_sync(kFull, err, 0)) break;
+        if (__any_sync(kFull, alg >> 31)) add_bytes();  // a lane reads far less than 2^31 bytes in 64 chunks
         if (P.work_limit && publish_work()) break;
         if (P.qlimit && !cnt_only) cnt_only = !bitmap && counts_only();
       }
