@@ -350,8 +350,6 @@ def run_serve(args, rank=0, world=1):
     e.set_option(d.OPT_FILTER, args.filter)
     if args.pack >= 0:
         e.set_option(d.OPT_PACK_MAX, args.pack)
-    if args.merge >= 0:
-        e.set_option(d.OPT_MERGE_MAX, args.merge)
     e.set_option(d.OPT_WORK_LIMIT, args.work_limit)
     e.set_option(d.OPT_QUERY_LIST_LIMIT, args.query_list_limit)
     t0 = time.time()
@@ -407,7 +405,7 @@ def run_serve(args, rank=0, world=1):
             assert again == ids, "the initial queries came back with other ids"
     clocks = sampler.stop()
     tuned = {k: e.get_option(getattr(d, "OPT_" + k.upper()))
-             for k in ("warps_per_sm", "split_min", "donate_depth", "pack_max", "merge_max", "bfs_levels")}
+             for k in ("warps_per_sm", "split_min", "donate_depth", "pack_max", "bfs_levels")}
 
     # the forms must agree request by request
     ref = runs["batched"]
@@ -657,8 +655,6 @@ def run_step(args, rank, world):
     e.set_option(d.OPT_FILTER, args.filter)
     if args.pack >= 0:
         e.set_option(d.OPT_PACK_MAX, args.pack)
-    if args.merge >= 0:
-        e.set_option(d.OPT_MERGE_MAX, args.merge)
     if args.autotune and args.warmup > 0:
         e.set_option(d.OPT_AUTOTUNE, 1)
     e.load_graph_edges(w.nv, w.labels, w.edges)
@@ -717,7 +713,7 @@ def run_step(args, rank, world):
                        "l2": "256 MiB buffer written between timed batches",
                        "filter": args.filter,
                        "tuned": {k: e.get_option(getattr(d, "OPT_" + k.upper()))
-                                 for k in ("warps_per_sm", "split_min", "donate_depth", "pack_max", "merge_max", "bfs_levels")}},
+                                 for k in ("warps_per_sm", "split_min", "donate_depth", "pack_max", "bfs_levels")}},
             "updates_per_sec": upd / (dev_ms / 1e3), "matches": matches,
             "latency_ms": {"p50": float(np.percentile(R[:, 1], 50)), "p99": float(np.percentile(R[:, 1], 99))},
             "e2e": {"value": matches / (wall_ms / 1e3), "unit": "matches/s",
@@ -756,7 +752,7 @@ def main():
     ap.add_argument("--autotune", type=int, default=1)
     ap.add_argument("--filter", type=int, default=0, help="DSM_OPT_FILTER (0 labels only, 1 LDF+NLF, 2 cluster encoding)")
     ap.add_argument("--pack", type=int, default=-1, help="DSM_OPT_PACK_MAX before tuning (-1: engine default)")
-    ap.add_argument("--merge", type=int, default=-1, help="DSM_OPT_MERGE_MAX before tuning (-1: engine default)")
+    ap.add_argument("--merge", type=int, default=-1, help="accepted, without effect (the matcher has no merges)")
     ap.add_argument("--cpu-s", type=float, default=15.0, help="seconds of CPU matching for cpu_baseline")
     ap.add_argument("--ref-s", type=float, default=60.0, help="reference arm: seconds of CPU matching")
     ap.add_argument("--ref-host-s", type=float, default=60.0, help="reference arm: seconds of updateHostGraph")

@@ -108,7 +108,7 @@ int dsm_engine_set_option(dsm_engine *e, int option, int64_t value) {
       E.merge_max = (uint32_t)value;
       return DSM_OK;
     case DSM_OPT_PACK_MAX:
-      if (value < 0 || value > (1 << 20)) return E.fail(DSM_ERR_ARG, "intersection tile 0..2^20 entries");
+      if (value < 0 || value > (1 << 20)) return E.fail(DSM_ERR_ARG, "matcher batches 0..2^20");
       E.pack_max = (uint32_t)value;
       return DSM_OK;
     case DSM_OPT_AUTOTUNE: E.tune_next = value != 0; return DSM_OK;

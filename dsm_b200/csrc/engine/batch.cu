@@ -945,7 +945,7 @@ int Engine::autotune(MatchArgs &ma, const Staged &S, int &blocks) {
   const unsigned long long nseeds = hs->nseeds;
   struct Cand {
     int bps;
-    uint32_t split, dd, pack, merge, bfs;
+    uint32_t split, dd, pack, bfs;
   };
   auto rearm = [&]() -> int {
     std::memset(hs, 0, sizeof(Sched));
@@ -995,11 +995,10 @@ int Engine::autotune(MatchArgs &ma, const Staged &S, int &blocks) {
     }
     return DSM_OK;
   };
-  const Cand cur{blocks / std::max(num_sms, 1), ma.split_min, ma.donate_depth, ma.pack_max, merge_max,
-                 bfs_levels};
+  const Cand cur{blocks / std::max(num_sms, 1), ma.split_min, ma.donate_depth, ma.pack_max, bfs_levels};
   // stage 0: depth-first or breadth-first rows for the first 1 or 2 levels
   std::vector<Cand> c0;
-  for (uint32_t bl : {0u, 1u, 2u}) c0.push_back({cur.bps, cur.split, cur.dd, cur.pack, cur.merge, bl});
+  for (uint32_t bl : {0u, 1u, 2u}) c0.push_back({cur.bps, cur.split, cur.dd, cur.pack, bl});
   float best0 = 1e30f, best1 = 1e30f, best2 = 1e30f;
   Cand b0 = cur;
   if (d_rows.ptr)
@@ -1007,15 +1006,15 @@ int Engine::autotune(MatchArgs &ma, const Staged &S, int &blocks) {
   // stage 1: one partial embedding at a time or 32, at the current launch shape
   std::vector<Cand> c1;
   for (uint32_t pk : {0u, cur.pack ? cur.pack : 1024u})
-    c1.push_back({cur.bps, cur.split, cur.dd, pk, cur.merge, b0.bfs});
+    c1.push_back({cur.bps, cur.split, cur.dd, pk, b0.bfs});
   Cand b1 = b0, bc = b0;
   if (!stop)
     if (int rc = sweep(c1, !d_rows.ptr, b1, best1)) return rc;
-  // stage 2: blocks per SM x split threshold x donation depth, at that tile
+  // stage 2: blocks per SM x split threshold x donation depth, at that plan and batch
   std::vector<Cand> c2;
   for (int bps = std::max(1, match_blocks_per_sm - 2); bps <= match_blocks_per_sm; ++bps)
     for (uint32_t split : {64u, 128u, 512u})
-      for (uint32_t dd : {1u, 2u}) c2.push_back({bps, split, dd, b1.pack, b1.merge, b1.bfs});
+      for (uint32_t dd : {1u, 2u}) c2.push_back({bps, split, dd, b1.pack, b1.bfs});
   bc = b1;
   if (!stop)
     if (int rc = sweep(c2, false, bc, best2)) return rc;
@@ -1024,7 +1023,6 @@ int Engine::autotune(MatchArgs &ma, const Staged &S, int &blocks) {
     split_min = bc.split;
     donate_depth = bc.dd;
     pack_max = bc.pack;
-    merge_max = bc.merge;
     bfs_levels = bc.bfs;
     stats.tune_best_ms = best2;
   }
