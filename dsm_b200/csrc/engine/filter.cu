@@ -250,12 +250,15 @@ __global__ void __launch_bounds__(256) k_filter_op(DevGraph g, const FilterDevic
   if (k >= f.nops || !f.desc->full_now) return;
   __shared__ BlockRanges R;
   __shared__ uint32_t s_cand[256 + kOpTile];
-  __shared__ uint32_t s_n;
+  // candidates gathered, of even and odd tiles: what a tile leaves goes to the
+  // other one's, so that no thread still reads what is written
+  __shared__ uint32_t s_n[2];
   const DevFilterOp &op = f.ops[k];
   const uint32_t t = threadIdx.x, lane = t & 31, cu = op.core_u, words = f.words;
-  if (t == 0) s_n = 0;
+  if (t < 2) s_n[t] = 0;
   __syncthreads();
-  for (uint32_t base = blockIdx.x * kOpTile; base < g.nv; base += gridDim.x * kOpTile) {
+  uint32_t odd = 0;
+  for (uint32_t base = blockIdx.x * kOpTile; base < g.nv; base += gridDim.x * kOpTile, odd ^= 1) {
     const bool last = base + gridDim.x * kOpTile >= g.nv || base + gridDim.x * kOpTile < base;
 #pragma unroll
     for (uint32_t i = 0; i < kOpTile; i += 256) {
@@ -263,13 +266,12 @@ __global__ void __launch_bounds__(256) k_filter_op(DevGraph g, const FilterDevic
       const bool isc = v < g.nv && ((f.valid[v] >> cu) & 1u);
       const uint32_t m = __ballot_sync(kFull, isc);
       uint32_t at = 0;
-      if (m && lane == 0) at = atomicAdd(&s_n, (uint32_t)__popc(m));
+      if (m && lane == 0) at = atomicAdd(&s_n[odd], (uint32_t)__popc(m));
       at = __shfl_sync(kFull, at, 0);
       if (isc) s_cand[at + __popc(m & lanemask_lt())] = v;
     }
     __syncthreads();
-    uint32_t n = s_n;
-    __syncthreads();  // every thread has it: below, an op without leaf ranges meets no barrier before it changes
+    uint32_t n = s_n[odd];
     while (n >= 256 || (last && n)) {
       const uint32_t take = min(n, 256u);
       n -= take;
@@ -289,16 +291,18 @@ __global__ void __launch_bounds__(256) k_filter_op(DevGraph g, const FilterDevic
           a = lo[0];
           len = lo[1] - a;
         }
-        for (uint32_t from = 0;; from += kSpan) {
-          const uint32_t rest = len > from ? len - from : 0u;
-          const uint32_t total = lay_ranges(R, (unsigned long long)off * 4 + a + from, min(rest, kSpan));
+        uint32_t total;
+        do {
+          total = lay_ranges(R, (unsigned long long)off * 4 + a, min(len, kSpan));
           for (uint32_t e = t; e < total; e += 256)
             leaf_rule(op, g.arena[range_entry(R, e)] & kIdMask, f.vcand, f.enc, words);
-          if (!__syncthreads_or(rest > kSpan)) break;
-        }
+          __syncthreads();
+          a += kSpan;
+          len -= min(len, kSpan);
+        } while (total >= kSpan);  // below it no vertex has more
       }
-      if (t == 0) s_n = n;
     }
+    if (t == 0) s_n[odd ^ 1] = n;
     __syncthreads();
   }
 }
@@ -441,16 +445,18 @@ __global__ void __launch_bounds__(256) k_region_expand(DevGraph g, RegionDevice 
   const uint32_t tile = min((hi - lo + gridDim.x - 1) / gridDim.x, 256u);
   for (uint32_t base = lo + blockIdx.x * tile; base < hi; base += gridDim.x * tile) {
     const uint2 av = t < tile && base + t < hi ? g.adj[rg.list[base + t]] : make_uint2(0, 0);
-    for (uint32_t from = 0;; from += kSpan) {
-      const uint32_t rest = av.y > from ? av.y - from : 0u;
-      const uint32_t total = lay_ranges(R, (unsigned long long)av.x * 4 + from, min(rest, kSpan));
+    unsigned long long first = (unsigned long long)av.x * 4;
+    uint32_t len = av.y, total;
+    do {
+      total = lay_ranges(R, first, min(len, kSpan));
       for (uint32_t e = t; e < total; e += 256) {
         claim(rg, epoch, g.arena[range_entry(R, e)] & kIdMask, hop);
         if ((e >> 8) % 8 == 7 && *(volatile const uint32_t *)&rg.info->ov_round < 64) break;
       }
       if (__syncthreads_or(*(volatile const uint32_t *)&rg.info->ov_round < 64)) return;
-      if (!__syncthreads_or(rest > kSpan)) break;
-    }
+      first += kSpan;
+      len -= min(len, kSpan);
+    } while (total >= kSpan);  // below it no vertex has more
   }
 }
 
