@@ -146,7 +146,10 @@ __device__ __forceinline__ bool edge_live(const DevBatchEdges &t, uint32_t x, ui
 // Entries of x's run with label slot `slot` whose edge is not live after the
 // first `tp` updates: of the batch's edges at x, those it changes (the run
 // holds the union graph, so each is in it) and that are not live then.
-__device__ __forceinline__ uint32_t dead_entries(const DevBatchEdges &t, uint32_t x, uint32_t slot, uint32_t tp) {
+// A hub may have a million of them, three dependent loads each: `progress` is
+// counted up as it goes, for the warps whose bounded waits look at it.
+__device__ __forceinline__ uint32_t dead_entries(const DevBatchEdges &t, uint32_t x, uint32_t slot, uint32_t tp,
+                                                 unsigned long long *progress) {
   const unsigned long long first = ((unsigned long long)x << 32) | ((unsigned long long)slot << kIdBits);
   uint32_t lo = 0, hi = 2 * t.n;
   while (lo < hi) {
@@ -157,6 +160,7 @@ __device__ __forceinline__ uint32_t dead_entries(const DevBatchEdges &t, uint32_
   for (unsigned long long prev = ~0ull; lo < 2 * t.n; ++lo) {
     const unsigned long long k = t.dkey[lo];
     if ((k >> kIdBits) != (first >> kIdBits)) break;
+    if ((lo & 255) == 255) atomicAdd(progress, 1ull);
     if (k != prev) dead += !edge_live(t, x, (uint32_t)k & kIdMask, tp);
     prev = k;
   }

@@ -381,7 +381,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
     const uint4 row = rows[0][lane];
     const uint32_t x = F[j][lane];
     uint32_t gone = 0;
-    if (len && row.w && may_change(bt, x, slot_key(t_lab))) gone = dead_entries(bt, x, t_lab, tp);
+    if (len && row.w && may_change(bt, x, slot_key(t_lab))) gone = dead_entries(bt, x, t_lab, tp, &P.sc->progress.v);
     for (uint32_t same = t_same & ~(1u << j); same; same &= same - 1) {
       const uint32_t i = __ffs(same) - 1, i_bn = __shfl_sync(kFull, q_word, i) & 0xFFFFu;
       if (((j_bn >> i) | (i_bn >> j)) & 1u) {

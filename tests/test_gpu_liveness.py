@@ -63,3 +63,37 @@ def test_views_of_toggled_edges_equal_oracle(n, pack):
             for i in range(n):
                 assert np.array_equal(r.tuples_of(qid, i), t[i])
     e.close()
+
+
+@pytest.mark.parametrize("timeout", [10, 40])
+def test_a_hub_with_many_changed_edges_keeps_the_waits_going(timeout):
+    """200,000 edges of one hub deleted and inserted in a batch that counts
+    leaves on that hub: the search through the changed edges takes longer than
+    the matcher's bounded waits and counts as progress."""
+    n, m = 200_000, 8
+    hub, first = 0, 1 + m
+    nv = first + n
+    labels = np.zeros(nv, np.uint32)
+    labels[1:first] = 2
+    labels[first:] = 1
+    spokes = np.stack([np.zeros(nv - 1, np.int64), np.arange(1, nv)], 1).astype(np.uint32)
+    half = np.arange(first, nv)[::2]
+    flip = lambda op: np.stack([np.full(len(half), op), np.zeros(len(half), np.int64), half, 0 * half], 1)
+    ends = lambda: np.array([[op, hub, 1 + k, 0] for k in range(m) for op in (0, 1)])
+    # the hub with its leaves, half of them, all of them again: seen by the
+    # updates of its edges to the m ends
+    ups = np.concatenate([ends(), flip(0), ends(), flip(1), ends()]).astype(np.uint32)
+    q = d.Query.from_edges([2, 0, 1], [(0, 1), (1, 2)])
+    e = d.Engine(0)
+    e.set_option(d.OPT_LIST, 0)
+    e.set_option(d.OPT_TIMEOUT_MS, timeout)
+    e.load_graph_edges(nv, labels, spokes)
+    qid = e.register(q)
+    r = e.run_batch(ups)
+    got = r.counts[r.query_index(qid)]
+    a, b = 2 * m, 2 * m + len(half)
+    assert (got[:a] == n).all()
+    assert (got[b:b + a] == n - len(half)).all()
+    assert (got[b + a + len(half):] == n).all()
+    assert (got[a:b] == m).all() and (got[b + a:b + a + len(half)] == m).all()
+    e.close()
