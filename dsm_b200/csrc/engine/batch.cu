@@ -933,7 +933,7 @@ int Engine::compact_arena(uint64_t extra_words) {
 // The matcher's result does not depend on its launch shape or on how work is
 // donated, so the batch's own matcher launch is repeated on the same union
 // graph (counts only) for each candidate -- first the plan (breadth-first
-// levels), then the batch (one partial embedding or 32), then resident blocks
+// levels), then the batch (four partial embeddings or 32), then resident blocks
 // per SM x range-split threshold x donation depth -- timed with events, and the fastest
 // becomes the engine's setting.  The first candidate runs twice and its first
 // run is not counted (it warms L2 for all).
@@ -1003,7 +1003,7 @@ int Engine::autotune(MatchArgs &ma, const Staged &S, int &blocks) {
   Cand b0 = cur;
   if (d_rows.ptr)
     if (int rc = sweep(c0, true, b0, best0)) return rc;
-  // stage 1: one partial embedding at a time or 32, at the current launch shape
+  // stage 1: four partial embeddings together or 32, at the current launch shape
   std::vector<Cand> c1;
   for (uint32_t pk : {0u, cur.pack ? cur.pack : 1024u})
     c1.push_back({cur.bps, cur.split, cur.dd, pk, b0.bfs});

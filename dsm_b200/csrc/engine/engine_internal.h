@@ -206,7 +206,7 @@ struct Engine {
   int label_quirk = 0;
   int sort_results = 1;
   uint32_t split_min = 0, donate_depth = 0;  // donation granularity (0 = kernel default)
-  uint32_t pack_max = 1024;                  // 0: partial embeddings one at a time; else in batches
+  uint32_t pack_max = 1024;                  // 0: batches of four partial embeddings; else of 32
   uint32_t merge_max = 64;                   // DSM_OPT_MERGE_MAX as set: read back, nothing else
   uint32_t bfs_levels = 0;                   // breadth-first rows: levels beyond the seed (0: depth-first)
   uint64_t bfs_rows = 1u << 20;              // row table capacity

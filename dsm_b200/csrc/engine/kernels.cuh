@@ -162,7 +162,7 @@ struct MatchArgs {
   // donated when at least donate_depth levels lie below them (1..4)
   uint32_t split_min;
   uint32_t donate_depth;
-  // 0: partial embeddings expanded one at a time; else 32 together
+  // 0: up to four partial embeddings expanded together; else 32
   uint32_t pack_max;
   // breadth-first rows: in a launch with bfs_stop > 0, a task that finds
   // candidates completing bfs_stop positions (with at least two positions

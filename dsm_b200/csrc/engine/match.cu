@@ -158,6 +158,12 @@ __device__ void finish_task(const MatchArgs &P) {
 // fewer than 2^32 (its ids have 27 bits); of plain runs' partials those are
 // taken whose ranges do.
 constexpr uint32_t kPast = 0xFFFFFFFFu;  // no run is as long: a vertex has fewer neighbours than there are ids
+// Partials together where the caller asks for small batches (DSM_OPT_PACK_MAX 0),
+// which deal a search of few partials out sooner.  One at a time took longer on
+// 256 queries x 1021 updates than the matcher without batches did (275 against
+// 218 ms a batch and its undoing; two 167, four 108, eight 75, 32 49); four are
+// no slower than it anywhere (three screened queries 1.9 -> 1.5 ms).
+constexpr uint32_t kFew = 4;
 constexpr uint32_t kRows = 3;  // backward neighbours with stored ranges; further ones are read when needed
 template <bool kLM>
 __host__ __device__ constexpr uint32_t warp_words(uint32_t W) {
@@ -285,7 +291,7 @@ __device__ void run_task(const MatchArgs &P, const DevBatchEdges &bt, uint32_t n
   // E(lane), parked while deeper ones run: lv_n = nb | cnt << 8 | partials
   // whose range is not begun << 16
   uint32_t lv_c = 0, lv_e = 0, lv_n = 0;
-  const uint32_t most = P.pack_max ? 32u : 1u;  // partials expanded together
+  const uint32_t most = P.pack_max ? 32u : kFew;  // partials expanded together
 
   // The ranges of E(l)'s partials (F holds the batch); returns their total.
   // Plain runs: may make the batch smaller, so that the total fits.

@@ -133,10 +133,9 @@ const char *dsm_last_error(dsm_engine *e);
                                    depend on it; DSM_OPT_AUTOTUNE tries 0, 1 and 2. */
 #define DSM_OPT_BFS_ROWS 23      /* row table capacity for DSM_OPT_BFS_LEVELS (default 2^20
                                    rows of 128 bytes) */
-#define DSM_OPT_PACK_MAX 19     /* matcher batches: 0: partial embeddings are expanded one at a
-                                   time; 1..2^20 (default 1024): up to 32 together, their
-                                   candidate ranges laid end to end.  Results do not depend
-                                   on it. */
+#define DSM_OPT_PACK_MAX 19     /* matcher batches: up to 32 partial embeddings (1..2^20, default
+                                   1024) or four (0) are expanded together, their candidate
+                                   ranges laid end to end.  Results do not depend on it. */
 int dsm_engine_set_option(dsm_engine *e, int option, int64_t value);
 int dsm_engine_get_option(dsm_engine *e, int option, int64_t *value);
 
