@@ -84,3 +84,31 @@ def test_batches_around_the_counting_sort(n, nv, nlab):
         for x, y in zip(e.export_graph(), st.export()):
             assert np.array_equal(x, y)
     e.close()
+
+
+@pytest.mark.parametrize("deg", [0, 1, 3, 5, 2047, 2049])
+@pytest.mark.parametrize("where", ["below", "above", "between", "everywhere"])
+def test_many_more_neighbours_than_there_were(deg, where):
+    """A run that moves with 6,000 new entries: all in one gap, or in every."""
+    rng = np.random.default_rng(deg)
+    n = 6000
+    nv = 1 + deg + n
+    there = {"below": np.arange(1 + n, nv), "above": np.arange(1, 1 + deg),
+             "between": np.concatenate([np.arange(1, 1 + deg // 2), np.arange(1 + deg // 2 + n, nv)]),
+             "everywhere": np.sort(rng.permutation(np.arange(1, nv))[:deg])}[where]
+    new = np.setdiff1d(np.arange(1, nv), there)
+    for nlab in (1, 3):
+        labels = rng.integers(0, nlab, nv).astype(np.uint32)
+        edges = np.stack([np.zeros_like(there), there], 1).astype(np.uint32).reshape(-1, 2)
+        q = d.Query.from_edges([labels[0], nlab - 1], [(0, 1)])
+        e = d.Engine(0)
+        e.set_option(d.OPT_LIST, 0)
+        e.load_graph_edges(nv, labels, edges)
+        qid = e.register(q)
+        st = oracle_stream(nv, labels, edges, q)
+        for b in (_updates(1, rng.permutation(new)), _updates(0, new[::2])):
+            r = e.run_batch(b)
+            assert np.array_equal(r.counts[r.query_index(qid)], st.apply(b, listed=False)[1])
+            for x, y in zip(e.export_graph(), st.export()):
+                assert np.array_equal(x, y)
+        e.close()
