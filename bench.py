@@ -74,14 +74,15 @@ def _peaks():
     return 6650.0, "fallback"
 
 
-# Counters of the matcher measured by ncu (one B200, --clock-control none):
-# config 4 at 1/4 scale, launches 81-83 of `bench.py --scale -2 --steps 1
-# --warmup 1`; config 2 at full size, the timed launch of `bench.py --mode
-# step --steps 1 --warmup 1 --autotune 0` (5 blocks per SM).
-C4_NCU = {"dram_bytes_per_launch": 1.672e8, "l2_bytes_per_launch": 2.385e9, "launch_ms": 1.825,
-          "l2_hit": 0.620, "issue_active": 0.180}
-C2_NCU = {"dram_bytes_per_launch": 4.847e8, "l2_bytes_per_launch": None, "launch_ms": 225.4,
-          "l2_hit": 0.939, "issue_active": 0.395}
+# Counters of the matcher measured by ncu (one B200, --clock-control none;
+# profiles/k_match_bench_workloads.md): config 4 at 1/4 scale, launches 29-31 of
+# `bench.py --scale -2 --steps 1 --warmup 1` (tuned requests of the batched
+# form); config 2 at full size, the timed launch of `bench.py --mode step
+# --steps 1 --warmup 1 --autotune 0` (4 blocks per SM).
+C4_NCU = {"dram_bytes_per_launch": 1.408e10, "l2_bytes_per_launch": 6.593e10, "launch_ms": 10.78,
+          "l2_hit": 0.527, "issue_active": 0.388}
+C2_NCU = {"dram_bytes_per_launch": 5.071e8, "l2_bytes_per_launch": None, "launch_ms": 32.72,
+          "l2_hit": 0.714, "issue_active": 0.461}
 
 
 def l2_figures(ncu):
@@ -487,7 +488,8 @@ def run_serve(args, rank=0, world=1):
                      "l2": l2_figures(C4_NCU),
                      "issue_active": C4_NCU["issue_active"],
                      "note": "algorithmic bytes of the matcher over the served device time of the burst; the "
-                             "matcher waits on dependent L2 loads (issue_active), HBM is not the binding bound"},
+                             "matcher waits on dependent loads (filter words, runs; issue_active), HBM is not "
+                             "the binding bound"},
         "clocks": clocks,
         "gen_seconds": gen_s,
         "load_seconds": load_s,

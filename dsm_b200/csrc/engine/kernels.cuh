@@ -165,7 +165,7 @@ struct MatchArgs {
   // 0: up to four partial embeddings expanded together; else 32
   uint32_t pack_max;
   // breadth-first rows: in a launch with bfs_stop > 0, a task that finds
-  // candidates completing bfs_stop positions (with at least two positions
+  // candidates completing bfs_stop positions (with at least one position
   // left) writes each prefix as a row to rows_out instead of descending,
   // while the table has room (then it descends as usual); a launch with
   // rows_in takes its tasks from those rows instead of the seeds

@@ -68,7 +68,8 @@ const char *dsm_last_error(dsm_engine *e);
 #define DSM_OPT_SORT 8          /* 1: canonically sort each update's tuples (default) */
 #define DSM_OPT_LIST_LIMIT 9    /* bytes of tuples one batch may list; beyond it the batch
                                    returns exact counts only and its view has listed = 0 */
-#define DSM_OPT_MEM_BUDGET 10   /* device memory budget in bytes (>= bytes in use); raising it
+#define DSM_OPT_MEM_BUDGET 10   /* device memory budget in bytes (>= bytes in use, less what
+                                   batches can do without: that is given back); raising it
                                    admits queries that waited for memory */
 #define DSM_OPT_SPLIT_MIN 11    /* work donation: split a remaining pivot range of at least
                                    this many entries (0 = default 128; else >= 64) */
